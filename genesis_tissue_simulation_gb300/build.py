@@ -1,6 +1,6 @@
 """In-tree build of the CUDA library (libgbtissue.so) for sm_103a.
 
-Two translation units are compiled in parallel with nvcc and linked into
+The translation units are compiled in parallel with nvcc and linked into
 ``csrc/_build/libgbtissue.so``.  Flags that matter for results:
 
 * ``-fmad=false``: no implicit multiply-add contraction; the projections contract explicitly
@@ -27,7 +27,7 @@ LIBRARY = BUILD / "libgbtissue.so"
 DEBUG_BUILD = CSRC / "_build_debug"
 DEBUG_LIBRARY = DEBUG_BUILD / "libgbtissue_debug.so"
 SOURCES = ("frame_kernels.cu", "lcs_api.cu", "mesh_build.cu", "batch_api.cu", "adjoint_kernels.cu", "adjoint_api.cu",
-           "surface_kernels.cu", "cut_topology.cu")
+           "surface_kernels.cu", "cut_topology.cu", "brick_plan.cpp", "brick_kernels.cu")
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 
 
@@ -56,7 +56,7 @@ def _stale(library: Path = LIBRARY) -> bool:
     if not library.exists():
         return True
     built = library.stat().st_mtime
-    inputs = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(INCLUDE.glob("*.h"))
+    inputs = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cpp")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(INCLUDE.glob("*.h"))
     return any(p.stat().st_mtime > built for p in inputs)
 
 

@@ -1,0 +1,269 @@
+// The coloured sweep of one brick in one CTA (host side: brick_plan.cpp).
+//
+// What bounds the sweep of a single mesh is the number of times the whole GPU has to agree: a frame
+// kernel that closes every colour with a grid barrier and gathers positions through L2 spent about
+// 1.3 us a colour in the barrier and 2 us in dependent L2 round trips, 37 colours a substep, with the
+// issue slots nearly idle.  Here each CTA keeps the positions of its brick and of a halo in shared
+// memory and runs several colours between two exchanges, projecting the elements near its faces
+// redundantly; a colour then costs one gather from shared memory, the projection and __syncthreads.
+//
+// Exchange: an owner publishes the values its neighbours need as 16-byte records (x, y, z, epoch), one
+// relaxed 128-bit store each, into one of two buffers (by epoch parity), and a reader polls each record
+// it needs until the epoch matches.  Data and flag arrive in one access, so an exchange costs one store
+// and one load through L2 and no fence.  A buffer is written again two epochs later: by then every
+// reader has published its next epoch (the plan makes neighbours read from each other every time).
+#pragma once
+#include "brick_plan.h"
+#include "grid_sync.cuh"
+#include "tissue_device.cuh"
+
+namespace gbt {
+
+constexpr int kBrickThreads = 512;
+constexpr int kBrickFrames = 32;   // instrument frames held in shared memory at a time
+
+struct BrickTables {
+    int bricks, stages, nEdgeColors, nTetColors, maxLocal, maxOwned, nIdle, N;
+    unsigned long long exchangeBefore[2];
+    const BrickDesc* desc; const int* head; const int* localNode; const int* idle;
+    const int2* importList; const int2* exportList;            // (local index, node)
+    int maxImport, maxExport;                                  // of one brick; kept in shared memory when listsShared
+    int listsShared;
+    const unsigned long long* tetWord; const float2* tetAlpha; const unsigned* edgeWord; const float* edgeRest;
+    const int* tetSrc; const int* edgeSrc;                     // colour slots of the mesh's tables
+    float4* mail;                                              // [2 x N] published values
+    float4* mailStart;                                         // [2 x N] published substep-start positions (damped sweeps)
+    unsigned* epoch;                                           // [bricks] exchanges so far, the same in every brick
+};
+
+__device__ __forceinline__ void publish(float4* to, f3 v, unsigned epoch) {
+    const unsigned long long lo = (unsigned long long)__float_as_uint(v.x) | (unsigned long long)__float_as_uint(v.y) << 32;
+    const unsigned long long hi = (unsigned long long)__float_as_uint(v.z) | (unsigned long long)epoch << 32;
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" :: "l"(to), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ void peek(const float4* from, unsigned long long& lo, unsigned long long& hi) {
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}" : "=l"(lo), "=l"(hi) : "l"(from) : "memory");
+}
+
+// One thread's records e[0 .. count) of an exchange, all polled together until each has its epoch.
+constexpr int kTake = 4;
+template <class Put>
+__device__ __forceinline__ bool take(const float4* from, const int2 (&e)[kTake], unsigned waiting, unsigned want, unsigned* status,
+                                     long long budget, Put&& put) {
+    long long start = 0;
+    for (unsigned rounds = 1; waiting != 0u; rounds++) {
+        unsigned long long lo[kTake], hi[kTake];
+#pragma unroll
+        for (int u = 0; u < kTake; u++) if (waiting >> u & 1u) peek(from + e[u].y, lo[u], hi[u]);
+#pragma unroll
+        for (int u = 0; u < kTake; u++)
+            if ((waiting >> u & 1u) && (unsigned)(hi[u] >> 32) == want) {
+                put(e[u].x, mk(__uint_as_float((unsigned)lo[u]), __uint_as_float((unsigned)(lo[u] >> 32)), __uint_as_float((unsigned)hi[u])));
+                waiting &= ~(1u << u);
+            }
+        if ((rounds & 31u) == 0u && waiting != 0u) {
+            if (start == 0) start = clock64();
+            if (*(volatile unsigned*)status != 0u) return false;
+            if (clock64() - start > budget) { atomicOr(status, kSyncTimeout); return false; }
+        }
+    }
+    return true;
+}
+// Publishes the listed values and takes the neighbours'.  A function of values, out of line: the sweep
+// around it keeps its registers, and P and Q stay shared-memory addresses there.
+static __device__ __noinline__ bool exchangeRecords(float4* box, float4* boxStart, float4* P, float4* Q, const int2* exports, int nExports,
+                                                    const int2* imports, int nImports, unsigned epoch, unsigned lag, unsigned* status,
+                                                    long long budget) {
+    const int T = blockDim.x, tid = threadIdx.x;
+    for (int i = tid; i < nExports; i += T) {
+        const int2 e = exports[i];
+        publish(box + e.y, xyz(P[e.x]), epoch);
+        if (boxStart) publish(boxStart + e.y, xyz(Q[e.x]), epoch);
+    }
+    bool bad = false;
+    for (int i = tid; i < nImports; i += kTake * T) {
+        int2 e[kTake];
+        unsigned mine = 0u;
+#pragma unroll
+        for (int u = 0; u < kTake; u++) if (i + u * T < nImports) { e[u] = imports[i + u * T]; mine |= 1u << u; }
+        bad = !take(box, e, mine, epoch + lag, status, budget, [&](int at, f3 v) { float4& p = P[at]; p.x = v.x; p.y = v.y; p.z = v.z; }) || bad;
+        if (boxStart) bad = !take(boxStart, e, mine, epoch + lag, status, budget, [&](int at, f3 v) { Q[at] = make_float4(v.x, v.y, v.z, 0.f); }) || bad;
+    }
+    return __syncthreads_or(bad ? 1 : 0) == 0;
+}
+
+// Where a recorded sweep writes every element's node positions before its projection (by colour slot;
+// the element's owner writes them).
+struct BrickTape { float4* edge; float4* tet; };
+
+struct BrickTet { unsigned long long word; float2 alpha; };
+struct BrickEdge { unsigned word; float rest; };
+
+struct Brick {
+    const BrickTables& bt;
+    BrickDesc d;
+    float4* P;        // [maxLocal] positions (w = inverse mass)
+    float4* Q;        // [maxLocal] damped sweeps, else [maxOwned]: substep-start positions
+    float4* V;        // [maxOwned] velocities
+    float4* A;        // [maxOwned] accelerations
+    ContactFrame* frames;   // [kBrickFrames]
+    float* typeB;     // [6 x 9] rest inverses
+    int* head;        // offsets of this brick (brick_plan.h)
+    const int *edgeOff, *tetOff, *impOff, *expOff;
+    int2 *imports, *exports;   // this brick's lists in shared memory (listsShared)
+    unsigned epoch;   // of the last exchange
+    unsigned* status; // barrier status word: kSyncTimeout once a wait ran out
+    long long budget; unsigned lag;   // lag: epochs awaited beyond the published one (timeout test)
+
+    static __host__ __device__ size_t bytes(const BrickTables& t, bool damped) {
+        const size_t head = (size_t)t.nEdgeColors + t.nTetColors + 2 * t.stages + 4;
+        const size_t all = sizeof(float4) * ((size_t)t.maxLocal + (damped ? t.maxLocal : t.maxOwned) + 2 * (size_t)t.maxOwned) +
+               kBrickFrames * sizeof(ContactFrame) + 54 * sizeof(float) + head * sizeof(int) +
+               (t.listsShared ? sizeof(int2) * ((size_t)t.maxImport + t.maxExport) : 0);
+        return (all + 15) & ~(size_t)15;
+    }
+    // Shared-memory layout, offsets and exchange lists.  Closed by a barrier.
+    __device__ __forceinline__ Brick(const BrickTables& t, const DeviceMesh& m, int b, float4* shared, bool damped, int exchanges, unsigned* statusWord,
+                     long long spinBudget, unsigned lagEpochs)
+        : bt(t), d(t.desc[b]), status(statusWord), budget(spinBudget), lag(lagEpochs) {
+        P = shared;
+        Q = P + t.maxLocal;
+        V = Q + (damped ? t.maxLocal : t.maxOwned);
+        A = V + t.maxOwned;
+        frames = (ContactFrame*)(A + t.maxOwned);
+        imports = (int2*)(frames + kBrickFrames);
+        exports = imports + (t.listsShared ? t.maxImport : 0);
+        typeB = (float*)(exports + (t.listsShared ? t.maxExport : 0));
+        head = (int*)(typeB + 54);
+        edgeOff = head; tetOff = edgeOff + t.nEdgeColors + 1; impOff = tetOff + t.nTetColors + 1; expOff = impOff + t.stages + 1;
+        const int words = t.nEdgeColors + t.nTetColors + 2 * t.stages + 4;
+        for (int i = threadIdx.x; i < words; i += blockDim.x) head[i] = t.head[d.head + i];
+        for (int i = threadIdx.x; i < 54; i += blockDim.x) typeB[i] = m.typeB[i / 9][i % 9];
+        epoch = t.bricks > 1 ? t.epoch[b] : 0u;
+        __syncthreads();
+        if (t.listsShared) {
+            for (int i = threadIdx.x; i < impOff[t.stages] - impOff[0]; i += blockDim.x) imports[i] = t.importList[impOff[0] + i];
+            for (int i = threadIdx.x; i < expOff[t.stages] - expOff[0]; i += blockDim.x) exports[i] = t.exportList[expOff[0] + i];
+            __syncthreads();
+        }
+        if (t.bricks > 1 && threadIdx.x == 0) t.epoch[b] = epoch + (unsigned)exchanges;   // also when a wait runs out
+    }
+
+    // The positions of owned and halo nodes, and the owned nodes' accelerations and velocities.
+    __device__ __forceinline__ void loadState(const float4* pos, const float4* vel, const float4* ext) {
+        for (int i = threadIdx.x; i < d.nLocal; i += blockDim.x) P[i] = pos[bt.localNode[d.nodeBase + i]];
+        for (int i = threadIdx.x; i < d.nOwned; i += blockDim.x) {
+            const int n = bt.localNode[d.nodeBase + i];
+            const float4 F = ext[n];
+            const f3 a = mk(F.x, F.y, F.z) * pos[n].w;
+            A[i] = make_float4(a.x, a.y, a.z, 0.f);
+            V[i] = vel[n];
+        }
+    }
+
+    // The values stage `st` needs: publish this brick's, take the neighbours'.  All threads, after a
+    // barrier; closes with one.  False when a neighbour did not publish within the budget.
+    __device__ __forceinline__ bool exchange(int st, bool withStart) {
+        epoch++;
+        const size_t box = (size_t)(epoch & 1u) * bt.N;
+        const int oe = expOff[st], ne = expOff[st + 1] - oe, oi = impOff[st], ni = impOff[st + 1] - oi;
+        return exchangeRecords(bt.mail + box, withStart ? bt.mailStart + box : nullptr, P, Q,
+                               bt.listsShared ? exports + (oe - expOff[0]) : bt.exportList + oe, ne,
+                               bt.listsShared ? imports + (oi - impOff[0]) : bt.importList + oi, ni, epoch, lag, status, budget);
+    }
+
+    __device__ __forceinline__ bool exchangeAt(int p) const { return (bt.exchangeBefore[p >> 6] >> (p & 63)) & 1ull; }
+    __device__ __forceinline__ BrickTet tetAt(int k) const { return {bt.tetWord[k], bt.tetAlpha[k]}; }
+    __device__ __forceinline__ BrickEdge edgeAt(int e) const { return {bt.edgeWord[e], bt.edgeRest[e]}; }
+
+    template <bool Damped, bool Record>
+    __device__ __forceinline__ void edge(const BrickEdge& w, const FrameCoeffs& fc, int k, const BrickTape& tape) {
+        if (!(w.word & kBrickEdgeLive)) return;
+        const int a = w.word & kBrickNodeMask, b = (w.word >> kBrickNodeBits) & kBrickNodeMask;
+        EdgeRecord r;
+        r.live = 1; r.rest = w.rest;
+        if (Damped) { r.qi = xyz(Q[a]); r.qj = xyz(Q[b]); } else r.qi = r.qj = mk(0.f, 0.f, 0.f);
+        float4 oa, ob;
+        const float4 pa = P[a], pb = P[b];
+        if (Record && (w.word & kBrickEdgeOwner)) {
+            float4* t = tape.edge + 2 * (size_t)bt.edgeSrc[k];
+            t[0] = pa; t[1] = pb;
+        }
+        if (solveEdge(r, fc, pa, pb, oa, ob)) { P[a] = oa; P[b] = ob; }
+    }
+    template <bool Damped, bool Record>
+    __device__ __forceinline__ void tet(const BrickTet& w, const FrameCoeffs& fc, int k, const BrickTape& tape) {
+        if (!(w.word & kBrickTetLive)) return;
+        const unsigned lo = (unsigned)w.word, hi = (unsigned)(w.word >> 28);
+        const int id[4] = {(int)(lo & kBrickNodeMask), (int)((lo >> kBrickNodeBits) & kBrickNodeMask), (int)(hi & kBrickNodeMask),
+                           (int)((hi >> kBrickNodeBits) & kBrickNodeMask)};
+        const float4 p[4] = {P[id[0]], P[id[1]], P[id[2]], P[id[3]]};
+        if (Record && (w.word & kBrickTetOwner)) {
+            float4* t = tape.tet + 4 * (size_t)bt.tetSrc[k];
+            t[0] = p[0]; t[1] = p[1]; t[2] = p[2]; t[3] = p[3];
+        }
+        f3 q[4], o[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) q[c] = Damped ? xyz(Q[id[c]]) : mk(0.f, 0.f, 0.f);
+        if (!solveTet(typeB + 9 * ((hi >> 28) & 7u), p, q, w.alpha, fc, Damped && fc.dampingOverH != 0.f, false, o)) return;
+#pragma unroll
+        for (int c = 0; c < 4; c++) P[id[c]] = make_float4(o[c].x, o[c].y, o[c].z, p[c].w);
+    }
+
+    // One sweep over the colours from the positions in P (owned nodes current, halo by the first
+    // exchange).  A thread always holds the record of its next element, loaded while it projects the one
+    // before, across colours and exchanges.  Opens and closes with a barrier; false on a timeout.
+    // after(edges) is called when a colour is done.
+    template <bool Damped, bool Record = false, class After>
+    __device__ __forceinline__ bool sweep(const FrameCoeffs& fc, After&& after, const BrickTape& tape = BrickTape()) {
+        const int T = blockDim.x, tid = threadIdx.x;
+        const int nE = bt.nEdgeColors, nT = bt.nTetColors;
+        int st = 0;
+        BrickEdge nextEdge;
+        BrickTet nextTet;
+        if (fc.doEdges && nE > 0 && edgeOff[0] + tid < edgeOff[1]) nextEdge = edgeAt(edgeOff[0] + tid);
+        if (fc.doStrain && nT > 0 && tetOff[0] + tid < tetOff[1]) nextTet = tetAt(tetOff[0] + tid);
+        __syncthreads();
+        {   // offsets two colours ahead: none is waited for (all zero when the phase is off)
+            int lo = fc.doEdges ? edgeOff[0] : 0, hi = fc.doEdges ? edgeOff[min(1, nE)] : 0, hi2 = fc.doEdges ? edgeOff[min(2, nE)] : 0;
+            for (int c = 0; c < nE; c++) {
+                const int hi3 = fc.doEdges ? edgeOff[min(c + 3, nE)] : 0;
+                if (exchangeAt(c)) { if (!exchange(st, Damped && st == 0)) return false; st++; }
+                for (int k = lo + tid;;) {
+                    const bool have = k < hi, last = k + T >= hi;
+                    const BrickEdge cur = nextEdge;
+                    const int kn = last ? hi + tid : k + T;
+                    if (kn < (last ? hi2 : hi)) nextEdge = edgeAt(kn);
+                    if (have) edge<Damped, Record>(cur, fc, k, tape);
+                    if (last) break;
+                    k = kn;
+                }
+                lo = hi; hi = hi2; hi2 = hi3;
+                __syncthreads();
+                after(true);
+            }
+        }
+        {   // offsets two colours ahead: none is waited for (all zero when the phase is off)
+            int lo = fc.doStrain ? tetOff[0] : 0, hi = fc.doStrain ? tetOff[min(1, nT)] : 0, hi2 = fc.doStrain ? tetOff[min(2, nT)] : 0;
+            for (int c = 0; c < nT; c++) {
+                const int hi3 = fc.doStrain ? tetOff[min(c + 3, nT)] : 0;
+                if (exchangeAt(nE + c)) { if (!exchange(st, Damped && st == 0)) return false; st++; }
+                for (int k = lo + tid;;) {
+                    const bool have = k < hi, last = k + T >= hi;
+                    const BrickTet cur = nextTet;
+                    const int kn = last ? hi + tid : k + T;
+                    if (kn < (last ? hi2 : hi)) nextTet = tetAt(kn);
+                    if (have) tet<Damped, Record>(cur, fc, k, tape);
+                    if (last) break;
+                    k = kn;
+                }
+                lo = hi; hi = hi2; hi2 = hi3;
+                __syncthreads();
+                after(false);
+            }
+        }
+        return true;
+    }
+};
+
+}  // namespace gbt

@@ -1,0 +1,214 @@
+// One frame of a single mesh on spatial bricks (brick_frame.cuh), and the upkeep of a plan's tables.
+#include "brick_kernels.h"
+#include "contact_point.cuh"
+
+namespace gbt {
+namespace {
+
+// A node no element touches through its substeps, as the brick's node phases treat its own.
+__device__ void idleNode(const DeviceMesh& m, int n, const FrameCoeffs& fc, const ToolPose& from, const ToolPose& to, const ContactParams& cp) {
+    float4 P = m.pos[n], Q = P;
+    f3 V = xyz(m.vel[n]);
+    if (!(P.w > 0.f)) {
+        m.prev[n] = make_float4(P.x, P.y, P.z, 0.f);
+        m.vel[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
+    }
+    const float4 F = m.ext[n];
+    const f3 a = mk(F.x, F.y, F.z) * P.w;
+    for (int s = 0; s < fc.substeps; s++) {
+        Q = P;
+        V = V + a * fc.h;
+        f3 x = xyz(P) + V * fc.h;
+        if (fc.contact) {
+            const float t = fminf(1.f, (float)(fc.firstSubstep + s + 1) / (float)fc.numSubsteps);
+            x = contactPoint(x, P.w, V, contactFrame(from, to, t, cp, fc.contactAlphaH2), cp);
+        }
+        P = make_float4(x.x, x.y, x.z, P.w);
+        V = ((x - xyz(Q)) * fc.invH) * fc.velScale;
+    }
+    m.pos[n] = P;
+    m.prev[n] = make_float4(Q.x, Q.y, Q.z, 0.f);
+    m.vel[n] = make_float4(V.x, V.y, V.z, 0.f);
+}
+
+template <bool Damped>
+__device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeffs& fc, const ToolPose& from, const ToolPose& to,
+                                           const ContactParams& cp, const BrickTables& bt, unsigned* state) {
+    extern __shared__ float4 shared[];
+    const int tid = threadIdx.x, T = blockDim.x;
+    const int exchanges = bt.bricks > 1 ? fc.substeps * bt.stages : 0;
+    Brick b(bt, m, blockIdx.x, shared, Damped, exchanges, state + 2, fc.spinBudget, fc.syncTestExtra > 0 ? 1u << 30 : 0u);
+    const bool stamp = fc.phaseClock != nullptr && blockIdx.x == 0 && tid == 0;
+    int s = 0, slot = 0;
+    auto mark = [&](unsigned tag) {
+        if (stamp && slot < kPhaseRecordsPerSubstep) {
+            unsigned long long ns;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(ns));
+            fc.phaseClock[(size_t)s * kPhaseRecordsPerSubstep + slot++] = ((unsigned long long)tag << 56) | (ns & 0x00FFFFFFFFFFFFFFull);
+        }
+    };
+    b.loadState(m.pos, m.vel, m.ext);
+    for (; s < fc.substeps; s++) {
+        slot = 0;
+        mark(kPhaseFrameStart);
+        if (fc.contact && s % kBrickFrames == 0) {
+            __syncthreads();
+            if (tid < kBrickFrames && s + tid < fc.substeps) {
+                const float t = fminf(1.f, (float)(fc.firstSubstep + s + tid + 1) / (float)fc.numSubsteps);
+                b.frames[tid] = contactFrame(from, to, t, cp, fc.contactAlphaH2);
+            }
+        }
+        for (int i = tid; i < b.d.nOwned; i += T) {
+            float4 P = b.P[i];
+            b.Q[i] = make_float4(P.x, P.y, P.z, 0.f);
+            if (P.w > 0.f) {
+                const f3 v = xyz(b.V[i]) + xyz(b.A[i]) * fc.h;
+                b.V[i] = make_float4(v.x, v.y, v.z, 0.f);
+                const f3 x = xyz(P) + v * fc.h;
+                b.P[i] = make_float4(x.x, x.y, x.z, P.w);
+            }
+        }
+        mark(kPhasePredict);
+        if (!b.sweep<Damped>(fc, [&](bool edges) { mark(edges ? kPhaseEdges : kPhaseTets); })) return;
+        for (int i = tid; i < b.d.nOwned; i += T) {
+            float4 P = b.P[i];
+            f3 v = mk(0.f, 0.f, 0.f);
+            if (P.w > 0.f) {
+                if (fc.contact) {
+                    const f3 p = contactPoint(xyz(P), P.w, xyz(b.V[i]), b.frames[s % kBrickFrames], cp);
+                    P = make_float4(p.x, p.y, p.z, P.w);
+                    b.P[i] = P;
+                }
+                v = ((xyz(P) - xyz(b.Q[i])) * fc.invH) * fc.velScale;
+            }
+            b.V[i] = make_float4(v.x, v.y, v.z, 0.f);
+        }
+        mark(kPhaseVelocity);
+    }
+    for (int i = tid; i < b.d.nOwned; i += T) {
+        const int n = bt.localNode[b.d.nodeBase + i];
+        m.pos[n] = b.P[i];
+        m.prev[n] = b.Q[i];
+        m.vel[n] = b.V[i];
+    }
+    for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode(m, bt.idle[i], fc, from, to, cp);
+    if (blockIdx.x == 0 && tid == 0) { state[1] = (unsigned)exchanges; state[3] = (unsigned)fc.rotParity; }
+}
+
+__global__ void meshFlagsKernel(DeviceMesh m, int E, int T, int fallback) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < E) refreshEdge(m, i);
+    if (i < T) {
+        refreshTet(m, i);
+        if (fallback && (m.tetMeta[i] & 8))
+            for (int o = 0; o < 3; o++) m.edgeSupport[checkSlot(m, m.tetOwner[3 * i + o], kSiteTetSlot)] = 1;
+    }
+    if (i < m.nNodes) m.pos[i].w = nodeInvMass(m, i);
+}
+
+__global__ void brickLiveKernel(DeviceMesh m, int edges, const int* edgeSrc, unsigned* edgeWord, int tets, const int* tetSrc,
+                                unsigned long long* tetWord, int fallback) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < edges) {
+        const int e = edgeSrc[i];
+        const bool live = m.edgeLive[e] != 0 && !(fallback && m.edgeSupport[checkSlot(m, m.edgeOwner[e], kSiteEdgeSlot)]);
+        edgeWord[i] = (edgeWord[i] & ~kBrickEdgeLive) | (live ? kBrickEdgeLive : 0u);
+    }
+    if (i < tets) tetWord[i] = (tetWord[i] & ~kBrickTetLive) | ((m.tetMeta[tetSrc[i]] & 8) ? kBrickTetLive : 0ull);
+}
+
+__global__ void brickAlphaKernel(int tets, const int* tetSrc, float invH2, const float2* stiff, float2* alpha) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < tets) { const float2 s = stiff[tetSrc[i]]; alpha[i] = make_float2(invH2 / s.x, invH2 / s.y); }
+}
+
+}  // namespace
+
+__global__ void __launch_bounds__(kBrickThreads, 1) brickFrameKernel(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to,
+                                                                     ContactParams cp, BrickTables bt, unsigned* state) {
+    brickFrame<false>(m, fc, from, to, cp, bt, state);
+}
+__global__ void __launch_bounds__(kBrickThreads, 1) brickFrameKernelDamped(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to,
+                                                                           ContactParams cp, BrickTables bt, unsigned* state) {
+    brickFrame<true>(m, fc, from, to, cp, bt, state);
+}
+
+template <class T> cudaError_t BrickBuffers::put(T** to, const T* from, size_t count, cudaStream_t stream) {
+    void* p = nullptr;
+    cudaError_t e = cudaMalloc(&p, (count ? count : 1) * sizeof(T));
+    if (e != cudaSuccess) return e;
+    memory_[held_++] = p;
+    *to = (T*)p;
+    if (!count) return cudaSuccess;
+    return from ? cudaMemcpyAsync(p, from, count * sizeof(T), cudaMemcpyHostToDevice, stream) : cudaMemsetAsync(p, 0, count * sizeof(T), stream);
+}
+
+void BrickBuffers::release() {
+    for (int i = 0; i < held_; i++) cudaFree(memory_[i]);
+    held_ = 0;
+    t = BrickTables{};
+    tets = edges = 0;
+}
+
+cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int maxBytes, cudaStream_t stream) {
+    release();
+    tets = (int)plan.tetWord.size(); edges = (int)plan.edgeWord.size();
+    asked = plan.asked;
+    threads = plan.threads < kBrickThreads ? plan.threads : kBrickThreads;
+    BrickTables q{};
+    q.stages = plan.stages; q.nEdgeColors = plan.nEdgeColors; q.nTetColors = plan.nTetColors;
+    q.maxLocal = plan.maxLocal; q.maxOwned = plan.maxOwned; q.nIdle = (int)plan.idle.size(); q.N = N;
+    q.exchangeBefore[0] = plan.exchangeBefore[0]; q.exchangeBefore[1] = plan.exchangeBefore[1];
+    cudaError_t e = put((BrickDesc**)&q.desc, plan.desc.data(), plan.desc.size(), stream);
+    if (e == cudaSuccess) e = put((int**)&q.head, plan.head.data(), plan.head.size(), stream);
+    if (e == cudaSuccess) e = put((int**)&q.localNode, plan.localNode.data(), plan.localNode.size(), stream);
+    if (e == cudaSuccess) e = put((int**)&q.idle, plan.idle.data(), plan.idle.size(), stream);
+    if (e == cudaSuccess) e = put((int2**)&q.importList, plan.importList.data(), plan.importList.size(), stream);
+    if (e == cudaSuccess) e = put((int2**)&q.exportList, plan.exportList.data(), plan.exportList.size(), stream);
+    if (e == cudaSuccess) e = put((unsigned long long**)&q.tetWord, (const unsigned long long*)plan.tetWord.data(), plan.tetWord.size(), stream);
+    if (e == cudaSuccess) e = put((float2**)&q.tetAlpha, (const float2*)nullptr, plan.tetWord.size(), stream);
+    if (e == cudaSuccess) e = put((unsigned**)&q.edgeWord, plan.edgeWord.data(), plan.edgeWord.size(), stream);
+    if (e == cudaSuccess) e = put((float**)&q.edgeRest, plan.edgeRest.data(), plan.edgeRest.size(), stream);
+    if (e == cudaSuccess) e = put(&tetSrc, plan.tetSrc.data(), plan.tetSrc.size(), stream);
+    if (e == cudaSuccess) e = put(&edgeSrc, plan.edgeSrc.data(), plan.edgeSrc.size(), stream);
+    const size_t mail = plan.bricks > 1 ? 2 * (size_t)N : 0;
+    if (e == cudaSuccess) e = put(&q.mail, (const float4*)nullptr, mail, stream);
+    if (e == cudaSuccess) e = put(&q.mailStart, (const float4*)nullptr, damped ? mail : 0, stream);
+    if (e == cudaSuccess) e = put(&q.epoch, (const unsigned*)nullptr, plan.bricks, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);   // the plan's host tables may go
+    if (e != cudaSuccess) { release(); return e; }
+    q.tetSrc = tetSrc; q.edgeSrc = edgeSrc;
+    q.bricks = plan.bricks;
+    // the exchange lists, next to the node state, when shared memory holds both
+    q.maxImport = plan.maxImport; q.maxExport = plan.maxExport;
+    q.listsShared = 1;
+    if (Brick::bytes(q, damped) > (size_t)maxBytes) q.listsShared = 0;
+    t = q;
+    return cudaSuccess;
+}
+
+cudaError_t BrickBuffers::refresh(const DeviceMesh& m, bool fallback, cudaStream_t stream) {
+    const int n = tets > edges ? tets : edges;
+    if (n) brickLiveKernel<<<(n + 255) / 256, 256, 0, stream>>>(m, edges, edgeSrc, (unsigned*)t.edgeWord, tets, tetSrc,
+                                                               (unsigned long long*)t.tetWord, fallback ? 1 : 0);
+    return cudaGetLastError();
+}
+
+cudaError_t BrickBuffers::compliances(float invH2, const float2* tetStiff, cudaStream_t stream) {
+    if (tets) brickAlphaKernel<<<(tets + 255) / 256, 256, 0, stream>>>(tets, tetSrc, invH2, tetStiff, (float2*)t.tetAlpha);
+    return cudaGetLastError();
+}
+
+cudaError_t refreshMeshFlags(const DeviceMesh& m, int E, int T, bool fallback, cudaStream_t stream) {
+    if (fallback) {
+        const cudaError_t e = cudaMemsetAsync(m.edgeSupport, 0, (size_t)6 * m.nNodes * sizeof(int), stream);
+        if (e != cudaSuccess) return e;
+    }
+    int n = E > T ? E : T;
+    if (m.nNodes > n) n = m.nNodes;
+    meshFlagsKernel<<<(n + 255) / 256, 256, 0, stream>>>(m, E, T, fallback ? 1 : 0);
+    return cudaGetLastError();
+}
+
+}  // namespace gbt

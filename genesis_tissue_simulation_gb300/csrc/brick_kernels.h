@@ -1,0 +1,37 @@
+// Brick frame of a single mesh (brick_kernels.cu) and the device side of a brick plan.
+#pragma once
+#include "brick_frame.cuh"
+
+namespace gbt {
+
+__global__ void brickFrameKernel(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to, ContactParams cp, BrickTables bt,
+                                 unsigned* state);
+__global__ void brickFrameKernelDamped(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to, ContactParams cp, BrickTables bt,
+                                       unsigned* state);
+
+// A plan's tables on the device.
+struct BrickBuffers {
+    BrickTables t{};
+    int tets = 0, edges = 0, threads = kBrickThreads;
+    int asked = 0;   // bricks the plan was asked for
+    int* tetSrc = nullptr; int* edgeSrc = nullptr;
+    // Uploads `plan` (of a mesh of N nodes) on `stream`, for CTAs of at most maxBytes shared memory;
+    // frees what was there.
+    cudaError_t upload(const BrickPlan& plan, int N, bool damped, int maxBytes, cudaStream_t stream);
+    void release();
+    bool ready() const { return t.bricks > 0; }
+    size_t sharedBytes(bool damped) const { return Brick::bytes(t, damped); }
+    // Live bits from the mesh's flags (`flags`: edgeLive, edgeSupport with fallback, tetMeta are current).
+    cudaError_t refresh(const DeviceMesh& m, bool fallback, cudaStream_t stream);
+    // Compliances over h^2 of the bricks' tets from the per-tet stiffnesses.
+    cudaError_t compliances(float invH2, const float2* tetStiff, cudaStream_t stream);
+private:
+    void* memory_[16] = {}; int held_ = 0;
+    template <class T> cudaError_t put(T** to, const T* from, size_t count, cudaStream_t stream);
+};
+
+// Liveness flags of every edge and tet, the edges a live tet carries (with fallback: edgeSupport must
+// be zero), and the nodes' inverse masses, from the current topology.
+cudaError_t refreshMeshFlags(const DeviceMesh& m, int E, int T, bool fallback, cudaStream_t stream);
+
+}  // namespace gbt

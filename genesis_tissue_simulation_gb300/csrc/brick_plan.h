@@ -1,0 +1,54 @@
+// Spatial bricks of a coloured lattice mesh: which elements every CTA of the brick kernel projects,
+// and which node values it takes from its neighbours when (brick_plan.cpp, brick_frame.cuh).
+#pragma once
+#include <cstdint>
+#include <vector>
+#include <cuda_runtime.h>
+
+namespace gbt {
+
+// One brick.  All offsets index the plan's concatenated tables.  `head` is the start of its header
+// words: edgeOff[nEdgeColors + 1], tetOff[nTetColors + 1], importOff[stages + 1], exportOff[stages + 1],
+// each absolute.
+struct BrickDesc {
+    int nodeBase, nOwned, nLocal;   // localNode[nodeBase + l]: node of local index l, owned nodes first
+    int head;
+};
+
+// Element words.  A tet: local nodes in bits 0-13, 14-27, 28-41 and 42-55, Kuhn type 56-58, live 59.
+// An edge: local ends in bits 0-13 and 14-27, live 28.  Bit 60 (tets) and 29 (edges): the brick owns the
+// element's first node, so exactly one brick has it set.
+constexpr int kBrickNodeBits = 14, kBrickMaxLocal = 1 << kBrickNodeBits;
+constexpr unsigned kBrickNodeMask = kBrickMaxLocal - 1;
+constexpr uint64_t kBrickTetLive = 1ull << 59, kBrickTetOwner = 1ull << 60;
+constexpr unsigned kBrickEdgeLive = 1u << 28, kBrickEdgeOwner = 1u << 29;
+
+struct BrickMesh {   // the coloured mesh a plan is made for; nodes on an nx * ny * nz lattice
+    int N, nx, ny, nz;
+    const int* active;                                              // [N]
+    int nEdgeColors, nTetColors;
+    const int* edgeOff; const int2* edgeEnds; const float* edgeRest;   // colour order
+    const int* tetOff; const int4* tetIds; const int* tetMeta;
+};
+
+struct BrickPlan {
+    int bricks = 0, stages = 1, nEdgeColors = 0, nTetColors = 0, maxLocal = 0, maxOwned = 0, maxImport = 0, maxExport = 0;
+    int asked = 0;                         // the brick count the split was chosen for
+    int threads = 32;                      // of a CTA: the widest phase, in whole warps
+    uint64_t exchangeBefore[2] = {0, 0};   // bit p: neighbours' values are taken before phase p (edge colours, then tet colours)
+    double cost = 0.;                      // model time of one substep, microseconds
+    std::vector<BrickDesc> desc;
+    std::vector<int> head, localNode, idle;
+    std::vector<int2> importList, exportList;   // (local index, node)
+    std::vector<uint64_t> tetWord; std::vector<int> tetSrc;
+    std::vector<unsigned> edgeWord; std::vector<float> edgeRest; std::vector<int> edgeSrc;
+    bool ok() const { return bricks > 0; }
+};
+
+// The plan of `mesh` on at most `maxBricks` CTAs that keep at most `maxLocal` nodes each; forced > 0
+// asks for about that many bricks instead of the cheapest count.  wholeHalo: the first exchange takes
+// every halo node (damped sweeps read all of them at the substep's start).  reverse: the sweep runs tet
+// colours and then edge colours from last to first.  Returns a plan without bricks when none fits.
+BrickPlan buildBrickPlan(const BrickMesh& mesh, int maxBricks, int maxLocal, int forced, bool wholeHalo, bool reverse = false);
+
+}  // namespace gbt

@@ -16,6 +16,7 @@
 #include <string>
 #include <vector>
 
+#include "brick_kernels.h"
 #include "frame_kernels.h"
 #include "mesh_build.h"
 #include "session_view.h"
@@ -117,6 +118,11 @@ struct Session {
     DBuf<unsigned> floorSync;               // barrier-floor measurement: counter, status
     DBuf<int> uncovered0; bool fuseEdge0 = false;   // nodes ending no colour-0 edge; colour 0 is a matching
     bool profile = false; std::vector<cudaEvent_t> events; int profiledSteps = 0;
+    // automatic mode, plain frames: the mesh on spatial bricks (brick_frame.cuh).  bricksStale: the
+    // topology may have changed since the live bits were derived
+    BrickBuffers bricks; std::vector<int> brickIdle; unsigned long long planId = 0;
+    std::vector<int2> hostEdgeEnds; std::vector<float> hostEdgeRest; std::vector<int4> hostTetIds; std::vector<int> hostTetMeta, hostActive;
+    bool bricksStale = true, bricksDamped = false; int forcedBricks = 0, maxBrickBytes = 0;
     // section profiler (xpbd_profile_sections, xpbd_solver.cu:30-60): device time per phase kind
     bool sections = false; DBuf<unsigned long long> phaseClock; std::vector<unsigned long long> phaseHost;
     double sectionMs[8] = {}; long long sectionCount[8] = {};
@@ -151,6 +157,7 @@ void freePhysics() {
     S.edgeEnds.release(); S.edgeRest.release(); S.bendIJK.release(); S.bendPairs.release(); S.tetIds.release();
     S.tetAlpha.release(); S.tetStiff.release(); S.state.release(); S.bounds.release(); S.floorSync.release();
     S.uncovered0.release(); S.fuseEdge0 = false;
+    S.bricks.release(); S.bricksStale = true;
     S.lastFrameBlocks = 0;
     S.fiberLambda.release(); S.feasTarget.release(); S.needed.release(); S.incOff.release(); S.incTet.release(); S.guardFlags.release();
     S.rotA.release(); S.rotB.release(); S.rotParity = 0;
@@ -189,6 +196,9 @@ int ensureStream() {
     CK(cudaFuncGetAttributes(&ca, (const void*)frameKernelSessionCluster));
     S.maxClusterBytes = optin - (int)ca.sharedSizeBytes;   // dynamic bytes left beside its static shared memory
     CK(cudaFuncSetAttribute((const void*)frameKernelSessionCluster, cudaFuncAttributeMaxDynamicSharedMemorySize, S.maxClusterBytes));
+    for (const void* k : {(const void*)brickFrameKernel, (const void*)brickFrameKernelDamped})
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
+    S.maxBrickBytes = optin - 1024;
     int khz = 0;
     if (cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, S.device) == cudaSuccess && khz > 0) S.clockKHz = khz;
     S.gridBlocks = std::max(1, perSm) * S.smCount;
@@ -338,6 +348,31 @@ CutParams cutParams() {
 // (*followUp set), so the host flips the parity the kernel leaves in state[3].
 // Launch shapes of a frame: one CTA, the whole GPU, one thread-block cluster.
 constexpr int kShapeBlock = 0, kShapeGrid = 1, kShapeCluster = 2;
+// Automatic mode runs plain frames (no bends, perpendicular damping, guard, friction or blade) on bricks
+// wherever a plan fits.
+bool brickFrames(const FrameCoeffs& fc) {
+    return S.launchMode == 0 && S.bricks.ready() && !fc.doBend && !fc.perpDamp && !fc.guarded && !fc.friction && !fc.cut;
+}
+int launchBricks(const FrameCoeffs& fc, bool* followUp) {
+    DeviceMesh m = deviceMesh();
+    if (S.bricksStale) {
+        CK(refreshMeshFlags(m, S.E, S.T, fc.fallback != 0, S.stream));
+        CK(S.bricks.refresh(m, fc.fallback != 0, S.stream));
+        S.bricksStale = false;
+    }
+    FrameCoeffs f = fc;
+    ToolPose from = S.toolFrom, to = S.tool;
+    ContactParams cp = S.cp;
+    unsigned* state = S.state.p;
+    void* args[] = {&m, &f, &from, &to, &cp, &S.bricks.t, &state};
+    CK(cudaLaunchCooperativeKernel(S.bricksDamped ? (const void*)brickFrameKernelDamped : (const void*)brickFrameKernel, dim3(S.bricks.t.bricks),
+                                   dim3(S.bricks.threads), args, S.bricks.sharedBytes(S.bricksDamped), S.stream));
+    particleRotKernel<<<(S.N + 255) / 256, 256, 0, S.stream>>>(m, nullptr, fc.rotParity);
+    CK(cudaGetLastError());
+    S.lastFrameBlocks = 1;   // the kernel leaves its exchanges in the barrier counter
+    *followUp = true;
+    return 0;
+}
 constexpr int kSessionLogK = 3;   // 8 CTAs, the portable cluster size
 size_t clusterBytes() {
     const size_t perCluster = (size_t)kSessionClusterThreads << kSessionLogK;
@@ -459,6 +494,7 @@ FrameCoeffs frameCoeffs(float h, int N) {
 int launchFrame(const FrameCoeffs& fc, bool* followUp) {
     unsigned* state = S.state.p;
     CK(cudaMemsetAsync(state + 1, 0, 2 * sizeof(unsigned), S.stream));
+    if (brickFrames(fc)) return launchBricks(fc, followUp);
     if (S.brickCount.p) CK(cudaMemsetAsync(S.brickCount.p, 0, sizeof(unsigned), S.stream));
     const Shapes u = usableShapes(fc);
     int shape = requestedShape(u);
@@ -490,6 +526,35 @@ int launchFrame(const FrameCoeffs& fc, bool* followUp) {
                 if (S.autoMs[k] >= 0.f && (S.autoMs[best] < 0.f || S.autoMs[k] < S.autoMs[best])) best = k;
             S.autoShape = best;
         }
+    }
+    return 0;
+}
+
+
+// The session's brick plan: at most one brick per SM, each brick's node state in one CTA's shared
+// memory.  A mesh without a plan keeps the other shapes.
+BrickMesh brickMesh() {
+    return {S.N, S.dx + 1, S.dy + 1, S.dz + 1, S.hostActive.data(), (int)S.edgeColorOff.size() - 1, (int)S.tetColorOff.size() - 1,
+            S.edgeColorOff.data(), S.hostEdgeEnds.data(), S.hostEdgeRest.data(), S.tetColorOff.data(), S.hostTetIds.data(), S.hostTetMeta.data()};
+}
+int planBricks(HostMesh& hm, const int* active) {
+    S.bricks.release();
+    S.bricksStale = true;
+    S.planId++;
+    S.brickIdle.clear();
+    S.bricksDamped = S.strainDamping > 0.f;   // without perpendicular damping (betaS = 0) only the tets are damped
+    S.hostEdgeEnds.swap(hm.edgeEnds); S.hostEdgeRest.swap(hm.edgeRest); S.hostTetIds.swap(hm.tetIds); S.hostTetMeta.swap(hm.tetMeta);
+    S.hostActive.assign(active, active + S.N);
+    const BrickMesh bm = brickMesh();
+    // shared memory: at most four records of 16 B a node, beside the offsets and instrument frames
+    const int perNode = (S.bricksDamped ? 2 : 1) * 16, rest = 8192;
+    for (int room = S.maxBrickBytes - rest, share = 70; share >= 40; share -= 10) {
+        const BrickPlan plan = buildBrickPlan(bm, S.smCount, (int)((long long)room * share / 100) / perNode, S.forcedBricks, S.bricksDamped);
+        if (!plan.ok()) return 0;
+        S.brickIdle = plan.idle;
+        CK(S.bricks.upload(plan, S.N, S.bricksDamped, S.maxBrickBytes, S.stream));
+        if (S.bricks.sharedBytes(S.bricksDamped) <= (size_t)S.maxBrickBytes) return 0;
+        S.bricks.release();
     }
     return 0;
 }
@@ -629,6 +694,8 @@ LCS_API int LCS_InitPhysics(const PhysicsInitDesc* desc, const float* mass, cons
     CK(cudaMemsetAsync(S.bounds.p, 0, 3 * sizeof(unsigned), S.stream));
 #endif
     CK(cudaStreamSynchronize(S.stream));
+    rc = planBricks(hm, active);
+    if (rc) return rc;
     S.generation = ++g_sessionGeneration;
     S.physReady = true;
     return 0;
@@ -842,6 +909,7 @@ LCS_API int LCS_DetectCut() {
     q.lo = v(c.aabbMin); q.hi = v(c.aabbMax); q.ncut = v(c.ncut); q.valid = c.valid;
     detectQuadKernel<<<(n + 255) / 256, 256, 0, S.stream>>>(m, cu, q, S.rotParity ? S.rotB.p : S.rotA.p);
     severKernel<<<(n + 255) / 256, 256, 0, S.stream>>>(m, cu);
+    S.bricksStale = true;
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(S.stream));
     return 0;
@@ -859,6 +927,7 @@ LCS_API int LCS_Step(float dt) {
     if (fc.doStrain && h != S.lastH) {
         tetAlphaKernel<<<(S.T + 255) / 256, 256, 0, S.stream>>>(S.T, fc.invH2, S.tetStiff.p, S.tetAlpha.p);
         CK(cudaGetLastError());
+        if (S.bricks.ready()) CK(S.bricks.compliances(fc.invH2, S.tetStiff.p, S.stream));
         S.lastH = h;
     }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -897,7 +966,7 @@ LCS_API int LCS_Step(float dt) {
             last = ns;
         }
     }
-    if (fc.cut) S.havePrev = true;
+    if (fc.cut) S.havePrev = S.bricksStale = true;
     if (S.toolArmed) S.toolFrom = S.tool;
     if (S.hostState[2] != 0u) return LCS_ERR_DEVICE_TIMEOUT;
     S.rotParity = (int)((S.hostState[3] & 1u) ^ (followUp ? 1u : 0u));
@@ -1089,6 +1158,7 @@ LCS_API int GBT_SetState(const float* pos3N, const float* vel3N, const int* nbr6
     const unsigned never = ~0u;   // liveness: never derived
     CK(cudaMemcpyAsync(S.state.p, &never, sizeof(unsigned), cudaMemcpyHostToDevice, S.stream));
     S.generation = ++g_sessionGeneration;
+    S.bricksStale = true;
     return cudaStatus(cudaStreamSynchronize(S.stream));
 }
 
@@ -1142,6 +1212,20 @@ LCS_API int LCS_ProfileSectionsRead(char* text, int capacity) {
     }
     if (!text || capacity <= (int)out.size()) return (int)out.size() + 1;
     std::memcpy(text, out.c_str(), out.size() + 1);
+    return 0;
+}
+
+// Bricks of the next LCS_InitPhysics's plan: about `count`, or the cheapest by the model (0).
+LCS_API int GBT_SetBrickCount(int count) {
+    if (count < 0) return XPBD_ERR_BAD_ARG;
+    S.forcedBricks = count;
+    return 0;
+}
+// The session's plan: bricks, exchanges a substep, threads a CTA, nodes kept by the largest brick
+// (bricks 0: no plan).
+LCS_API int GBT_BrickInfo(int* out4) {
+    if (!S.physReady || !out4) return XPBD_ERR_NOT_READY;
+    out4[0] = S.bricks.t.bricks; out4[1] = S.bricks.t.bricks > 1 ? S.bricks.t.stages : 0; out4[2] = S.bricks.threads; out4[3] = S.bricks.t.maxLocal;
     return 0;
 }
 
@@ -1221,7 +1305,7 @@ LCS_API int LCS_StepNoAlloc(float dt) {
     unsigned words[2] = {0u, 0u};   // status, current particle-frame buffer
     CK(cudaMemcpyAsync(words, state + 2, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
     CK(cudaStreamSynchronize(S.stream));
-    if (fc.cut) S.havePrev = true;
+    if (fc.cut) S.havePrev = S.bricksStale = true;
     if (S.toolArmed) S.toolFrom = S.tool;
     if (words[0] != 0u) return LCS_ERR_DEVICE_TIMEOUT;
     S.rotParity = (int)((words[1] & 1u) ^ (followUp ? 1u : 0u));
@@ -1348,6 +1432,7 @@ int gbt::sessionView(SessionView* v) {
     v->tetColorOrder = S.tetColorOrder.data();
     v->state = S.state.p;
     v->generation = S.generation;
+    v->bricks = &S.bricks; v->brickMesh = brickMesh(); v->idleNodes = &S.brickIdle; v->planId = S.planId; v->maxBrickBytes = S.maxBrickBytes;
     v->revision = S.cutReady ? S.counters.p : nullptr;
     return 0;
 }

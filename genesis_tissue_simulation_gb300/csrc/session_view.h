@@ -1,6 +1,8 @@
 // What other translation units of the library may read of the LCS session (internal, not exported).
 #pragma once
-#include "tissue_device.cuh"
+#include <vector>
+
+#include "brick_kernels.h"
 
 namespace gbt {
 
@@ -17,6 +19,11 @@ struct SessionView {
     const int* tetColorOrder;          // host [T]: colour slot -> storage index
     unsigned* state;                   // device: [0] liveness revision, [1] barrier counter, [2] status
     unsigned long long generation;     // changes with every new physics session, cut module and restored state
+    const BrickBuffers* bricks;        // the session's brick tables (not ready: no plan)
+    BrickMesh brickMesh;               // host tables the plan was made from
+    const std::vector<int>* idleNodes; // nodes the plan leaves out
+    unsigned long long planId;         // changes with every plan
+    int maxBrickBytes;                 // shared memory of a brick's CTA
     const unsigned* revision;          // device: links severed since the cut module was set up (null without one)
 };
 

@@ -454,13 +454,10 @@ __device__ __forceinline__ TetRecord loadTet(const DeviceMesh& m, int k, const F
 // Unguarded: hydrostatic row J - 1.  Guarded (tissue guard armed): row log J with a linear floor
 // below J = 0.05, its own bulk damping, and a trust region capping every corner's move at 0.15 over
 // the longest row of Dm^-1.
-template <bool Dsm = false>
-__device__ __forceinline__ void applyTet(const DeviceMesh& m, const TetRecord& t, const FrameCoeffs& fc, bool guardedForm = false) {
-    int meta = t.meta;
-    if ((meta & 8) == 0) return;
-    const float* Bm = m.typeB[meta & 7];
-    int id[4] = {t.ids.x, t.ids.y, t.ids.z, t.ids.w};
-    float4 P[4] = {posRef<Dsm>(m, id[0]), posRef<Dsm>(m, id[1]), posRef<Dsm>(m, id[2]), posRef<Dsm>(m, id[3])};
+// From the corner positions P (w = inverse mass), their substep-start positions q (read only when
+// `damped`) and the type's rest inverse Bm: false when nothing moves, else the new positions o.
+__device__ __forceinline__ bool solveTet(const float* Bm, const float4 (&P)[4], const f3 (&sq)[4], float2 alpha, const FrameCoeffs& fc,
+                                         bool damped, bool guardedForm, f3 (&o)[4]) {
     f3 p[4] = {xyz(P[0]), xyz(P[1]), xyz(P[2]), xyz(P[3])};
     f3 br[3] = {mk(Bm[0], Bm[1], Bm[2]), mk(Bm[3], Bm[4], Bm[5]), mk(Bm[6], Bm[7], Bm[8])};
     f3 e1 = p[1] - p[0], e2 = p[2] - p[0], e3 = p[3] - p[0];
@@ -469,7 +466,7 @@ __device__ __forceinline__ void applyTet(const DeviceMesh& m, const TetRecord& t
     for (int c = 0; c < 3; c++) F[c] = fmv(e3, comp(br[2], c), fmv(e2, comp(br[1], c), e1 * comp(br[0], c)));
     float I1 = dotF(F[0], F[0]) + dotF(F[1], F[1]) + dotF(F[2], F[2]);
     f3 cof[3] = {crossF(F[1], F[2]), crossF(F[2], F[0]), crossF(F[0], F[1])};
-    float ad = t.alpha.x, ah = t.alpha.y;
+    float ad = alpha.x, ah = alpha.y;
     float J = dotF(F[0], cof[0]), pJ = fmaxf(J, .05f);
     float iso = powMinusTwoThirds(pJ);
     float q = fmaxf(fmaf(iso, I1, -3.f), 0.f);
@@ -489,7 +486,6 @@ __device__ __forceinline__ void applyTet(const DeviceMesh& m, const TetRecord& t
     gd[0] = (gd[1] + gd[2] + gd[3]) * -1.f;
     gh[0] = (gh[1] + gh[2] + gh[3]) * -1.f;
     // undamped: the velocity terms vd, vh enter multiplied by zero and are not formed
-    const bool damped = tetDamped(fc, guarded);
     float dd = 0.f, dh = 0.f, vd = 0.f, vh = 0.f, w[4];
 #pragma unroll
     for (int c = 0; c < 4; c++) {
@@ -497,7 +493,7 @@ __device__ __forceinline__ void applyTet(const DeviceMesh& m, const TetRecord& t
         dd = fmaf(w[c], dotF(gd[c], gd[c]), dd);
         dh = fmaf(w[c], dotF(gd[c], gh[c]), dh);
         if (damped) {
-            f3 dx = p[c] - t.q[c];
+            f3 dx = p[c] - sq[c];
             vd += dotF(gd[c], dx);
             vh += dotF(gh[c], dx);
         }
@@ -512,9 +508,9 @@ __device__ __forceinline__ void applyTet(const DeviceMesh& m, const TetRecord& t
     for (int c = 0; c < 4; c++) { f3 r = fmv(gd[c], -gamma, gh[c]); schur = fmaf(w[c], dotF(r, r), schur); }
     float rd = damped ? fmaf(-fc.dampingOverH, vd, -CD) * invScale : -CD * invScale;
     float rh = damped ? fmaf(-(bulkScale - 1.f), vh, -CH) * invBulk : -CH * invBulk;
-    if (!(A > 0.f) || !(schur > 0.f)) return;
+    if (!(A > 0.f) || !(schur > 0.f)) return false;
     float dlH = fc.omega * fmaf(-gamma, rd, rh) / schur, dlD = fmaf(-Bc, dlH, fc.omega * rd) * invA;
-    if (!isfinite(dlD) || !isfinite(dlH)) return;
+    if (!isfinite(dlD) || !isfinite(dlH)) return false;
     if (guarded) {
         float largest = 0.f;
 #pragma unroll
@@ -524,10 +520,18 @@ __device__ __forceinline__ void applyTet(const DeviceMesh& m, const TetRecord& t
         dlD *= accepted; dlH *= accepted;
     }
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-        f3 o = fmv(fmv(gd[c], dlD, gh[c] * dlH), w[c], p[c]);
-        posRef<Dsm>(m, id[c]) = make_float4(o.x, o.y, o.z, w[c]);
-    }
+    for (int c = 0; c < 4; c++) o[c] = fmv(fmv(gd[c], dlD, gh[c] * dlH), w[c], p[c]);
+    return true;
+}
+template <bool Dsm = false>
+__device__ __forceinline__ void applyTet(const DeviceMesh& m, const TetRecord& t, const FrameCoeffs& fc, bool guardedForm = false) {
+    if ((t.meta & 8) == 0) return;
+    const int id[4] = {t.ids.x, t.ids.y, t.ids.z, t.ids.w};
+    const float4 P[4] = {posRef<Dsm>(m, id[0]), posRef<Dsm>(m, id[1]), posRef<Dsm>(m, id[2]), posRef<Dsm>(m, id[3])};
+    f3 o[4];
+    if (!solveTet(m.typeB[t.meta & 7], P, t.q, t.alpha, fc, tetDamped(fc, guardedForm), guardedForm, o)) return;
+#pragma unroll
+    for (int c = 0; c < 4; c++) posRef<Dsm>(m, id[c]) = make_float4(o[c].x, o[c].y, o[c].z, P[c].w);
 }
 template <bool Dsm = false, bool Codes = false>
 __device__ __forceinline__ void projectTet(const DeviceMesh& m, int k, const FrameCoeffs& fc, bool guardedForm = false) {

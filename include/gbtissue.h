@@ -203,6 +203,13 @@ LCS_API int LCS_SetBarrierTest(int extraArrivals, float budgetSeconds);
  * closes one phase.  GBT_GridBarrierFloor: microseconds per barrier of `barriers` (1..1e6) back-to-back
  * barriers on the same grid with no work between them, the latency floor of a phase. */
 LCS_API int GBT_FrameBarriers(unsigned* barriers);
+/* Automatic mode runs plain frames (no bends, guard, friction, perpendicular damping or blade) on spatial
+ * bricks, one CTA each, that exchange halo values between groups of colours; results are the same bit for
+ * bit.  GBT_SetBrickCount: about `count` bricks in the next LCS_InitPhysics's plan, 0 = the cheapest.
+ * GBT_BrickInfo: bricks (0: no plan fits), exchanges a substep, threads a CTA, nodes of the largest brick.
+ * After a brick frame GBT_FrameBarriers reports the exchanges it ran. */
+LCS_API int GBT_SetBrickCount(int count);
+LCS_API int GBT_BrickInfo(int* out4);
 LCS_API int GBT_GridBarrierFloor(int barriers, float* usPerBarrier);
 
 /* ---- batched instances (no counterpart in the reference, which has one session per process) ----

@@ -1,0 +1,87 @@
+"""Plain frames on spatial bricks: any brick count, lattice shape, damping and option gives the frame
+of the whole-GPU kernel bit for bit, and the oracle's."""
+import ctypes as ct
+
+import numpy as np
+import pytest
+
+from genesis_tissue_simulation_gb300.grid import build_grid
+from genesis_tissue_simulation_gb300.native_backend import Capsule, PlainTissue, blade_sweep
+
+pytestmark = pytest.mark.gpu
+
+# 2 x 2 x 2 cells, a column, a sheet, odd blocks; bricks from one to one per few nodes
+LATTICES = {(2, 2, 2): (1, 2, 8), (2, 9, 2): (1, 3, 30), (17, 3, 11): (1, 4, 61), (9, 6, 13): (1, 2, 27, 152)}
+
+
+def frames(lib, size, bricks=0, mode=0, damping=0.0, ks=1e6, capsule=True, steps=3, substeps=5, blade_at=None):
+    grid = build_grid(0.2, size=tuple(np.float64(c) * 0.2 - 0.02 for c in size), density=1000.0)
+    dll = ct.CDLL(str(lib))
+    gpu = hasattr(dll, "GBT_SetBrickCount")
+    if gpu:
+        assert dll.GBT_SetBrickCount(bricks) == 0
+    with PlainTissue(grid, dt=1 / 60, substeps=substeps, ks=ks, strain_damping_s=damping, dll_path=lib) as t:
+        info = np.zeros(4, np.int32)
+        try:
+            if gpu:
+                assert dll.LCS_SetLaunchMode(mode) == 0
+                assert dll.GBT_BrickInfo(info.ctypes.data_as(ct.c_void_p)) == 0
+            t.set_gravity(0.0, -981.0, 0.0)
+            top = float(grid.positions[grid.active != 0, 1].max())
+            mid = grid.positions[grid.active != 0].mean(axis=0)
+            for k in range(steps):
+                if capsule:
+                    t.set_capsule(Capsule((mid[0] - 1.0, top + 0.2 - 0.06 * k, mid[2]), (mid[0] + 1.0, top + 0.2 - 0.06 * k, mid[2]), 0.25))
+                detect = blade_at == k
+                if detect:
+                    t.set_blade(blade_sweep((mid[0], top + 1.0, mid[2] - 0.3), (mid[0], mid[1], mid[2] - 0.3),
+                                            (mid[0], top + 1.0, mid[2] + 0.3), (mid[0], mid[1], mid[2] + 0.3)))
+                t.step(detect_cut=detect)
+                if detect:   # the blade is put away: plain frames of a severed lattice follow
+                    t.functions["LCS_SetPressureCutMode"](1)
+            rot = np.zeros((len(grid.positions), 9), np.float32)
+            t.check("GBT_GetParticleRot", rot.ctypes.data_as(ct.c_void_p))
+            return (t.positions(), t.velocities(), t.neighbors(), rot), info
+        finally:
+            if gpu:
+                dll.LCS_SetLaunchMode(0)
+                dll.GBT_SetBrickCount(0)
+
+
+@pytest.mark.parametrize("size,bricks", [(s, b) for s, counts in LATTICES.items() for b in counts])
+@pytest.mark.parametrize("options", [dict(), dict(damping=0.04), dict(damping=0.04, ks=0.0), dict(ks=0.0, capsule=False)],
+                         ids=["plain", "damped", "damped-fallback", "fallback"])
+def test_bricks_match_the_whole_gpu_frame(gpu_lib, size, bricks, options):
+    got, info = frames(gpu_lib, size, bricks, **options)
+    want, _ = frames(gpu_lib, size, mode=1, **options)
+    assert info[0] >= 1 and (bricks == 1) == (info[0] == 1)
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("bricks", [1, 5, 40])
+def test_bricks_match_the_oracle_through_a_cut(gpu_lib, oracle_libs, bricks):
+    """Frames before and after a blade frame: the live bits follow the severed links."""
+    got, _ = frames(gpu_lib, (9, 6, 13), bricks, steps=6, blade_at=2)
+    want, _ = frames(oracle_libs[0], (9, 6, 13), steps=6, blade_at=2)
+    assert (got[2] != want[2]).sum() == 0 and (got[2] < 0).sum() > 0
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
+
+
+def test_a_lost_neighbour_ends_the_frame_with_a_status(gpu_lib):
+    """Exchanges that await an epoch nobody publishes give up within the budget; the next frame is sound."""
+    dll = ct.CDLL(str(gpu_lib))
+    dll.LCS_SetBarrierTest.argtypes = (ct.c_int, ct.c_float)
+    grid = build_grid(0.2, size=(1.78, 1.18, 2.58), density=1000.0)
+    assert dll.GBT_SetBrickCount(8) == 0
+    try:
+        with PlainTissue(grid, dt=1 / 60, substeps=2, ks=1e6, strain_damping_s=0.0, dll_path=gpu_lib) as t:
+            assert dll.LCS_SetBarrierTest(1, 0.05) == 0
+            with pytest.raises(RuntimeError, match="-4002"):
+                t.step()
+            assert dll.LCS_SetBarrierTest(0, 2.0) == 0
+            t.step()
+    finally:
+        dll.LCS_SetBarrierTest(0, 2.0)
+        dll.GBT_SetBrickCount(0)
