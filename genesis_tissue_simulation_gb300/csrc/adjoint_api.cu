@@ -13,7 +13,7 @@
 #include <cstring>
 #include <vector>
 
-#include "adjoint_kernels.h"
+#include "brick_rollout.h"
 #include "session_view.h"
 #include "../../include/gbtissue.h"
 
@@ -44,6 +44,11 @@ struct Diff {
     // last forward
     int frames = 0, blocks = 1; bool grid = false, contact = false; float radius = 0.f;
     DiffCoeffs dc{};
+    // rollouts on bricks (automatic mode, a mesh with a plan): the session's tables with compliances of
+    // the rollout's own, and the reverse sweep's plan.  Made for the session plan `planId`; at session
+    // generation `checked` no idle node was mobile.
+    BrickBuffers reverse; Dev<float2> brickAlpha;
+    bool bricks = false, ranOnBricks = false; unsigned long long planId = 0, checked = ~0ull;
 };
 Diff D;
 
@@ -53,7 +58,8 @@ void releaseAll() {
     for (auto* b : {&D.originPos, &D.originVel, &D.finalPos, &D.finalVel, &D.ckPos, &D.ckVel, &D.tapeQ, &D.tapeV, &D.tapeX, &D.tapeEdge,
                     &D.tapeTet, &D.gx, &D.gv, &D.gq}) b->release();
     for (auto* b : {&D.theta, &D.path, &D.gTheta, &D.gRest, &D.gB, &D.pathPartial}) b->release();
-    D.bake.release(); D.alpha.release(); D.slotStorage.release();
+    D.bake.release(); D.alpha.release(); D.slotStorage.release(); D.brickAlpha.release(); D.reverse.release();
+    D.bricks = D.ranOnBricks = false; D.checked = ~0ull;
     D.ready = false; D.haveForward = false;
 }
 
@@ -80,6 +86,81 @@ DiffBuffers buffers() {
     b.gx = D.gx.p; b.gv = D.gv.p; b.gq = D.gq.p; b.gTheta = D.gTheta.p; b.gRest = D.gRest.p; b.gB = D.gB.p;
     b.pathPartial = D.pathPartial.p;
     return b;
+}
+
+// Shared memory of the backward: both plans' states in one CTA, without the exchange lists if need be.
+size_t backwardBytes(BrickTables& f, BrickTables& r, bool damped, int limit) {
+    for (int lists = 1; lists >= 0; lists--) {
+        f.listsShared = lists && f.listsShared; r.listsShared = lists && r.listsShared;
+        const size_t bytes = Brick::bytes(f, damped) + Brick::bytes(r, damped);
+        if (bytes <= (size_t)limit) return bytes;
+    }
+    return 0;
+}
+bool damped(const SessionView& v) { return v.strainDamping > 0.f; }
+
+// The reverse plan over the session's bricks; leaves D.bricks false when the bricks cannot serve.
+int planReverse(const SessionView& v) {
+    D.bricks = false;
+    if (!(v.launchMode == 0 || v.launchMode == 3) || !v.bricks->ready()) return 0;
+    const BrickTables& t = v.bricks->t;
+    const int perNode = (damped(v) ? 2 : 1) * 16;
+    // the same split: the plan depends on the brick count, and the count on the nodes served
+    const BrickPlan plan = buildBrickPlan(v.brickMesh, v.smCount, v.maxBrickBytes / perNode, t.bricks == 1 ? 1 : v.bricks->asked, false, true);
+    if (!plan.ok() || plan.bricks != t.bricks || plan.maxOwned != t.maxOwned) return 0;
+    CK(D.reverse.upload(plan, v.N, damped(v), v.maxBrickBytes, v.stream));
+    BrickTables f = t, r = D.reverse.t;
+    if (!backwardBytes(f, r, damped(v), v.maxBrickBytes)) { D.reverse.release(); return 0; }
+    CK(D.brickAlpha.ensure(v.bricks->tets));
+    for (const void* k : {(const void*)brickForward, (const void*)brickForwardDamped, (const void*)brickBackward, (const void*)brickBackwardDamped})
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, v.maxBrickBytes));
+    D.planId = v.planId;
+    D.bricks = true;
+    return 0;
+}
+// Whether this rollout runs on bricks: the plan is the session's, and the nodes it leaves out are
+// immobile (looked at again when the session's state was restored).
+int useBricks(const SessionView& v, bool* yes) {
+    *yes = false;
+    if (!D.bricks || v.planId != D.planId) return 0;
+    if (D.checked != v.generation && !v.idleNodes->empty()) {
+        std::vector<int> active(v.N);
+        CK(cudaMemcpyAsync(active.data(), v.mesh.active, (size_t)v.N * sizeof(int), cudaMemcpyDeviceToHost, v.stream));
+        CK(cudaStreamSynchronize(v.stream));
+        for (int n : *v.idleNodes) if (active[n] != 0) return 0;
+    }
+    D.checked = v.generation;
+    *yes = true;
+    return 0;
+}
+int launchBricks(const SessionView& v, bool backward, DeviceMesh m, DiffBuffers b) {
+    BrickTables f = v.bricks->t, r = D.reverse.t;
+    f.tetAlpha = D.brickAlpha.p;
+    ContactParams cp = v.cp;
+    DiffCoeffs dc = D.dc;
+    unsigned* barrier = v.state + 1;
+    long long budget = (long long)((double)v.syncBudgetSeconds * 1e3 * v.clockKHz);
+    const bool d = damped(v);
+    CK(cudaMemsetAsync(barrier, 0, 2 * sizeof(unsigned), v.stream));
+    if (backward) {
+        const size_t bytes = backwardBytes(f, r, d, v.maxBrickBytes);
+        const int threads = std::min(kReverseThreads, std::max(v.bricks->threads, D.reverse.threads));
+        void* args[] = {&m, &dc, &cp, &b, &f, &r, &barrier, &budget};
+        CK(cudaLaunchCooperativeKernel(d ? (const void*)brickBackwardDamped : (const void*)brickBackward, dim3(f.bricks), dim3(threads), args, bytes,
+                                       v.stream));
+    } else {
+        BrickBuffers own = *v.bricks;   // the session's tables, written through with the rollout's compliances
+        own.t.tetAlpha = D.brickAlpha.p;
+        CK(prepareRollout(m, b, D.E, D.T, dc.invH2, own, D.reverse, v.stream));
+        void* args[] = {&m, &dc, &cp, &b, &f, &barrier, &budget};
+        CK(cudaLaunchCooperativeKernel(d ? (const void*)brickForwardDamped : (const void*)brickForward, dim3(f.bricks), dim3(v.bricks->threads),
+                                       args, Brick::bytes(f, d), v.stream));
+    }
+    CK(cudaGetLastError());
+    unsigned status = 0;
+    CK(cudaMemcpyAsync(&status, v.state + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, v.stream));
+    CK(cudaStreamSynchronize(v.stream));
+    return status != 0u ? LCS_ERR_DEVICE_TIMEOUT : 0;
 }
 
 // Launch one of the rollout kernels on the session stream; reads the barrier status back.
@@ -139,7 +220,9 @@ LCS_API int GBT_DiffBegin(float scaleModulus, int checkpointEvery, int maxFrames
     D.grid = useGrid(v);
     D.blocks = D.grid ? blocksFor((const void*)diffBackwardGrid, v) : 1;
     if (D.blocks <= 0) return -(int)cudaErrorInvalidConfiguration;
-    CK(D.pathPartial.ensure(total * D.blocks * 6));
+    rc = planReverse(v);
+    if (rc) return rc;
+    CK(D.pathPartial.ensure(total * std::max(D.blocks, D.bricks ? v.bricks->t.bricks : 0) * 6));
     CK(cudaStreamSynchronize(v.stream));
     D.ready = true;
     return 0;
@@ -175,7 +258,9 @@ LCS_API int GBT_DiffForward(float dt, int frames, const float* logCompliance, co
     DeviceMesh m = v.mesh;
     m.tetAlpha = D.alpha.p;
     D.haveForward = false;
-    rc = launch(v, false, m, buffers());
+    rc = useBricks(v, &D.ranOnBricks);
+    if (rc) return rc;
+    rc = D.ranOnBricks ? launchBricks(v, false, m, buffers()) : launch(v, false, m, buffers());
     if (rc) return rc;
     CK(cudaMemcpyAsync(D.finalPos.p, v.mesh.pos, D.N * sizeof(float4), cudaMemcpyDeviceToDevice, v.stream));
     CK(cudaMemcpyAsync(D.finalVel.p, v.mesh.vel, D.N * sizeof(float4), cudaMemcpyDeviceToDevice, v.stream));
@@ -200,18 +285,20 @@ LCS_API int GBT_DiffBackward(const float* gradPos, float* gradLogCompliance, flo
     CK(cudaMemsetAsync(D.gq.p, 0, D.N * sizeof(float4), s));
     CK(cudaMemsetAsync(D.gTheta.p, 0, std::max(D.T, 1) * sizeof(float), s));
     const size_t total = (size_t)D.frames * D.substeps;
-    if (D.contact) CK(cudaMemsetAsync(D.pathPartial.p, 0, total * D.blocks * 6 * sizeof(float), s));
+    const bool bricks = D.ranOnBricks && v.planId == D.planId;   // the forward's checkpoints serve either path
+    const int blocks = bricks ? v.bricks->t.bricks : D.blocks;
+    if (D.contact) CK(cudaMemsetAsync(D.pathPartial.p, 0, total * blocks * 6 * sizeof(float), s));
     DiffBuffers b = buffers();
     if (gradRestLength) CK(cudaMemsetAsync(D.gRest.p, 0, std::max(D.E, 1) * sizeof(float), s)); else b.gRest = nullptr;
     if (gradRestInverse) CK(cudaMemsetAsync(D.gB.p, 0, 9 * (size_t)std::max(D.T, 1) * sizeof(float), s)); else b.gB = nullptr;
     DeviceMesh m = v.mesh;
     m.tetAlpha = D.alpha.p;
-    rc = launch(v, true, m, b);
+    rc = bricks ? launchBricks(v, true, m, b) : launch(v, true, m, b);
     if (rc) return rc;
     if (D.T) CK(cudaMemcpyAsync(gradLogCompliance, D.gTheta.p, D.T * sizeof(float), cudaMemcpyDeviceToDevice, s));
     if (gradCapsulePath) {
         int n = 6 * (D.frames + 1);
-        if (D.contact) diffPathGradient<<<(n + 127) / 128, 128, 0, s>>>(b, D.blocks, D.substeps, gradCapsulePath);
+        if (D.contact) diffPathGradient<<<(n + 127) / 128, 128, 0, s>>>(b, blocks, D.substeps, gradCapsulePath);
         else CK(cudaMemsetAsync(gradCapsulePath, 0, n * sizeof(float), s));
     }
     if (gradRestLength) {
@@ -233,7 +320,8 @@ LCS_API int GBT_DiffBackward(const float* gradPos, float* gradLogCompliance, flo
 
 LCS_API int GBT_DiffInfo(int* out4) {
     if (!D.ready || !out4) return XPBD_ERR_NOT_READY;
-    out4[0] = D.grid ? 1 : 0; out4[1] = D.blocks; out4[2] = D.every; out4[3] = D.maxFrames;
+    const int bricks = D.bricks ? D.reverse.t.bricks : 0;
+    out4[0] = bricks ? (bricks > 1 ? 1 : 0) : (D.grid ? 1 : 0); out4[1] = bricks ? bricks : D.blocks; out4[2] = D.every; out4[3] = D.maxFrames;
     return 0;
 }
 

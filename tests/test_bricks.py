@@ -85,3 +85,41 @@ def test_a_lost_neighbour_ends_the_frame_with_a_status(gpu_lib):
     finally:
         dll.LCS_SetBarrierTest(0, 2.0)
         dll.GBT_SetBrickCount(0)
+
+
+@pytest.mark.parametrize("size,damping,bricks", [((2, 2, 2), 0.0, 1), ((11, 6, 13), 0.0, 0), ((11, 6, 13), 0.04, 7), ((9, 4, 5), 0.04, 30),
+                                                 ((32, 8, 16), 0.0, 0)])
+def test_rollouts_on_bricks_match_the_whole_gpu_rollout(gpu_lib, size, damping, bricks):
+    """Forward bit for bit; adjoints to the rounding of signed-zero terms and of the path sum's order."""
+    import torch
+
+    from genesis_tissue_simulation_gb300 import diff as D
+    grid = build_grid(0.2, size=tuple(np.float64(c) * 0.2 - 0.02 for c in size), density=1000.0)
+    top = float(grid.positions[grid.active != 0, 1].max())
+    mid = grid.positions[grid.active != 0].mean(axis=0)
+    path = np.array([[mid[0] - 0.5, top + 0.2 - 0.1 * k, mid[2], mid[0] + 0.5, top + 0.2 - 0.1 * k, mid[2]] for k in range(4)], np.float32)
+    dll = ct.CDLL(str(gpu_lib))
+    out = []
+    for mode in (0, 1):
+        assert dll.GBT_SetBrickCount(bricks) == 0
+        try:
+            with D.DifferentiableTissue(grid, dt=1 / 60, substeps=4, ks=1e6, strain_damping_s=damping, gravity=(0.0, -981.0, 0.0),
+                                        checkpoint_every=3, max_frames=3, launch_mode=mode, dll_path=gpu_lib, scale_modulus=1e6) as t:
+                rng = np.random.default_rng(3)
+                theta = torch.tensor(np.log(1e-6) + rng.uniform(-0.5, 0.5, t.tet_count), dtype=torch.float32, device="cuda")
+                g = torch.tensor(rng.standard_normal((t.n_nodes, 3)), dtype=torch.float32, device="cuda")
+                for _ in range(2):   # a second rollout on the same handle starts from the same origin
+                    x = t.forward(theta, torch.tensor(path, device="cuda"))
+                    adj = t.backward(g, rest_shape=True, origin=True)
+                out.append((x.cpu().numpy(), {k: v.cpu().numpy() for k, v in adj.items()}, t.session.velocities(), t.info()))
+        finally:
+            dll.GBT_SetBrickCount(0)
+            dll.LCS_SetLaunchMode(0)
+    (x, adj, v, info), (x1, adj1, v1, _) = out
+    assert bricks == 0 or info["ctas"] == (1 if bricks == 1 else info["ctas"]) and (bricks == 1 or info["ctas"] > 1)
+    assert np.array_equal(x, x1) and np.array_equal(v, v1)
+    for name, a in adj.items():
+        b = adj1[name]
+        assert np.isfinite(a).all()
+        # path: 12 substeps' sums in another order; the rest differs at most by zeros that were added
+        assert np.abs(a - b).max() <= (1e-5 if name == "path" else 1e-6) * max(np.abs(b).max(), 1e-30), name
