@@ -27,7 +27,8 @@ LIBRARY = BUILD / "libgbtissue.so"
 DEBUG_BUILD = CSRC / "_build_debug"
 DEBUG_LIBRARY = DEBUG_BUILD / "libgbtissue_debug.so"
 SOURCES = ("frame_kernels.cu", "lcs_api.cu", "mesh_build.cu", "batch_api.cu", "adjoint_kernels.cu", "adjoint_api.cu",
-           "surface_kernels.cu", "cut_topology.cu", "brick_plan.cpp", "brick_kernels.cu", "brick_rollout.cu")
+           "surface_kernels.cu", "cut_topology.cu", "brick_plan.cpp", "brick_kernels.cu", "brick_rollout.cu",
+           "brick_batch.cu")
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 
 

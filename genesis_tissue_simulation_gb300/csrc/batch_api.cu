@@ -18,7 +18,9 @@
 #include <numeric>
 #include <vector>
 
+#include "brick_batch.h"
 #include "frame_kernels.h"
+#include "host_parallel.h"
 #include "mesh_build.h"
 #include "../../include/gbtissue.h"
 
@@ -61,6 +63,7 @@ struct Batch {
     // per-instance per-type stiffness and compliances; `useCodes` selects them over the explicit tables
     Buf<unsigned> tetCode, edgeCode; Buf<int4> instGeo; Buf<float2> instStiff, instAlpha;
     bool codesAvailable = false, useCodes = false;
+    BatchBricks bricks;                              // mode 0 on bricks (plain frames of a batch that fits)
     Buf<int> mobile;                                 // nodes of positive inverse mass (lockstep node passes)
     Buf<ContactFrame> frames;
     unsigned* hostStatus = nullptr;
@@ -97,6 +100,7 @@ void releaseAll() {
     G.tetCode.release(); G.edgeCode.release(); G.instGeo.release(); G.instStiff.release(); G.instAlpha.release();
     G.codesAvailable = G.useCodes = false;
     G.mobile.release();
+    G.bricks.release();
     if (G.framesHost) cudaFreeHost(G.framesHost);
     G.framesHost = nullptr; G.framesHostCap = 0;
     G.packedXyz.release();
@@ -202,6 +206,12 @@ FrameCoeffs frameCoeffs(float h) {
     return fc;
 }
 
+// Mode 0 runs plain frames on bricks wherever a plan fits; asking for the explicit element tables of a
+// batch that has the implicit ones keeps the lockstep grid.
+bool brickFrames(const FrameCoeffs& fc) {
+    return G.bricks.ready() && !fc.doBend && !fc.perpDamp && (G.useCodes || !G.codesAvailable);
+}
+
 int ensureFramesHost(size_t records) {
     if (records <= G.framesHostCap) return 0;
     if (G.framesHost) cudaFreeHost(G.framesHost);
@@ -242,7 +252,17 @@ void stageFrames(int steps, const ToolPose* tools, float h) {
 int launchFrame(const FrameCoeffs& fc, const ContactFrame* frames) {
     DeviceMesh m = batchMesh();
     m.contactFrames = frames;
-    if (G.mode == 0) {
+    if (G.mode == 0 && brickFrames(fc)) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(G.bricks.ctas); cfg.blockDim = dim3(G.bricks.threads); cfg.dynamicSmemBytes = G.bricks.bytes; cfg.stream = G.stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = 1;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        ContactParams cp = G.cp;
+        CK(cudaLaunchKernelEx(&cfg, brickBatchKernel(G.strainDamping > 0.f, G.codesAvailable), m, fc, cp, G.bricks.buffers.t,
+                              (const BrickShape*)G.bricks.shapes, (const int*)G.bricks.order, (const int*)G.bricks.start,
+                              G.codesAvailable ? (const float2*)G.instAlpha.p : (const float2*)nullptr, G.state.p + 2));
+    } else if (G.mode == 0) {
         CutParams cu{};
         ToolPose none{};
         ContactParams cp = G.cp;
@@ -311,6 +331,8 @@ int prepareAlphas(float h) {
         if (G.codesAvailable) {   // the same operation on each instance's six Kuhn types
             tetAlphaKernel<<<(6 * G.count + 255) / 256, 256, 0, G.stream>>>(6 * G.count, 1.f / (h * h), G.instStiff.p, G.instAlpha.p);
             CK(cudaGetLastError());
+        } else if (G.bricks.ready()) {
+            CK(G.bricks.buffers.compliances(1.f / (h * h), G.tetStiff.p, G.stream));
         }
         G.lastH = h;
     }
@@ -364,6 +386,52 @@ int stepFrames(float dt, int steps, const ToolPose* tools, bool useGraph) {
     return G.hostStatus[0] != 0u ? LCS_ERR_DEVICE_TIMEOUT : 0;
 }
 
+
+// The batch's bricks.  The topology of a batch never changes, so the liveness that the other shapes
+// derive at their first frame (links and nodes present; with the tet-support fallback, edges no live
+// tet carries) is settled here.
+int planBricks(const std::vector<HostMesh>& meshes, const GbtInstanceDesc* inst, const std::vector<int2>& iEdge, const std::vector<int2>& iTet) {
+    int optin = 0, perSm = 0, reserved = 0;
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, G.device));
+    CK(cudaDeviceGetAttribute(&perSm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, G.device));
+    CK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, G.device));
+    const int fixed = 1024;   // the kernel's static shared memory, rounded up
+    const int one = optin - fixed, two = std::min(one, perSm / 2 - reserved - fixed);
+    CK(cudaFuncSetAttribute((const void*)brickBatchKernel(G.strainDamping > 0.f, G.codesAvailable), cudaFuncAttributeMaxDynamicSharedMemorySize, one));
+    const int count = G.count;
+    const bool fallback = G.T > 0 && G.youngE > 0.f && G.ks <= 0.f;
+    std::vector<std::vector<int>> edgeSlot(count), tetSlot(count);
+    std::vector<std::vector<unsigned char>> edgeDead(count), tetDead(count);
+    std::vector<BatchBrickInstance> in(count);
+    for (int i = 0; i < count; i++) {
+        const HostMesh& hm = meshes[i];
+        const GbtInstanceDesc& d = inst[i];
+        const int eC = (int)hm.edgeColorOff.size() - 1, tC = (int)hm.tetColorOff.size() - 1;
+        edgeSlot[i].resize(hm.E); tetSlot[i].resize(hm.T); edgeDead[i].assign(hm.E, 0); tetDead[i].assign(hm.T, 0);
+        for (int c = 0; c < eC; c++)
+            for (int k = hm.edgeColorOff[c]; k < hm.edgeColorOff[c + 1]; k++) edgeSlot[i][k] = iEdge[(size_t)i * G.nEdgeColors + c].x + k - hm.edgeColorOff[c];
+        for (int c = 0; c < tC; c++)
+            for (int k = hm.tetColorOff[c]; k < hm.tetColorOff[c + 1]; k++) tetSlot[i][k] = iTet[(size_t)i * G.nTetColors + c].x + k - hm.tetColorOff[c];
+        std::vector<unsigned char> carried(fallback ? (size_t)6 * hm.N : 0, 0);
+        for (int k = 0; k < hm.T; k++) {
+            const int4 t = hm.tetIds[k];
+            bool live = d.active[t.x] && d.active[t.y] && d.active[t.z] && d.active[t.w];
+            for (int o = 0; o < 3; o++) live = live && d.nbrIdx[hm.tetOwner[3 * k + o]] >= 0;
+            tetDead[i][k] = !live;
+            for (int o = 0; fallback && live && o < 3; o++) carried[hm.tetOwner[3 * k + o]] = 1;
+        }
+        for (int k = 0; k < hm.E; k++) {
+            const int2 e = hm.edgeEnds[k];
+            edgeDead[i][k] = !(d.nbrIdx[hm.edgeOwner[k]] >= 0 && d.active[e.x] && d.active[e.y]) || (fallback && carried[hm.edgeOwner[k]]);
+        }
+        in[i] = {{hm.N, d.dimsX + 1, d.dimsY + 1, d.dimsZ + 1, d.active, eC, tC, hm.edgeColorOff.data(), hm.edgeEnds.data(), hm.edgeRest.data(),
+                  hm.tetColorOff.data(), hm.tetIds.data(), hm.tetMeta.data()},
+                 G.nodeBase[i], edgeSlot[i].data(), tetSlot[i].data(), edgeDead[i].data(), tetDead[i].data()};
+    }
+    CK(G.bricks.plan(in, G.N, G.smCount, one, two, G.strainDamping > 0.f, G.stream));
+    return 0;
+}
+
 }  // namespace
 
 // =============================================================================================
@@ -388,12 +456,19 @@ LCS_API int GBT_BatchInit(int count, const GbtInstanceDesc* inst, const GbtBatch
         const GbtInstanceDesc& d = inst[i];
         if (d.dimsX <= 0 || d.dimsY <= 0 || d.dimsZ <= 0 || !d.cornerPos || !d.mass || !d.pinned || !d.active || !d.nbrIdx ||
             !d.restNbr || d.bendPairCount < 0 || (d.bendPairCount > 0 && !d.bendPairs)) return XPBD_ERR_BAD_ARG;
-        int n = (d.dimsX + 1) * (d.dimsY + 1) * (d.dimsZ + 1);
+    }
+    std::vector<int> built(count, 0);
+    parallelFor(count, [&](int i) {
+        const GbtInstanceDesc& d = inst[i];
+        const int n = (d.dimsX + 1) * (d.dimsY + 1) * (d.dimsZ + 1);
         std::vector<float> zeros(3 * (size_t)n, 0.f);
         MeshInput in{d.dimsX, d.dimsY, d.dimsZ, d.cornerPos, d.mass, d.pinned, d.active, zeros.data(), d.nbrIdx, d.restNbr,
                      d.bendPairs, d.bendPairCount, G.youngE, G.poisson};
-        rc = buildHostMesh(in, meshes[i]);
-        if (rc) return rc;
+        built[i] = buildHostMesh(in, meshes[i]);
+    });
+    for (int i = 0; i < count; i++) {
+        if (built[i]) return built[i];
+        const GbtInstanceDesc& d = inst[i];
         HostMesh& hm = meshes[i];
         if (d.tetMuV && d.tetKappaV)   // per-tet material in storage order, placed through the colour order
             for (int k = 0; k < hm.T; k++) {
@@ -577,6 +652,10 @@ LCS_API int GBT_BatchInit(int count, const GbtInstanceDesc* inst, const GbtBatch
     CK(G.derived.upload(derived.data(), count, G.stream)); CK(G.state.upload(state.data(), 4, G.stream));
     rc = packInstances(G.smCount * 2);
     if (rc) return rc;
+    if (!(G.kb > 0.f && G.B > 0) && !(G.betaS > 0.f)) {   // what runs on bricks
+        rc = planBricks(meshes, inst, iEdge, iTet);
+        if (rc) return rc;
+    }
     G.tool.assign(count, ToolPose{}); G.toolFrom = G.tool;
 #ifdef GBT_DEBUG_BOUNDS
     CK(G.bounds.alloc(3));

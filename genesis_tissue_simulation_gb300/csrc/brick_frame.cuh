@@ -23,13 +23,14 @@ constexpr int kBrickThreads = 512;
 constexpr int kBrickFrames = 32;   // instrument frames held in shared memory at a time
 
 struct BrickTables {
-    int bricks, stages, nEdgeColors, nTetColors, maxLocal, maxOwned, nIdle, N;
-    unsigned long long exchangeBefore[2];
+    int bricks, maxLocal, maxOwned, nIdle, N;
+    BrickShape shape;                                          // a batch keeps one per instance elsewhere
     const BrickDesc* desc; const int* head; const int* localNode; const int* idle;
     const int2* importList; const int2* exportList;            // (local index, node)
-    int maxImport, maxExport;                                  // of one brick; kept in shared memory when listsShared
+    int maxList;                                               // exchange records of one brick, kept in shared memory when listsShared
     int listsShared;
-    const unsigned long long* tetWord; const float2* tetAlpha; const unsigned* edgeWord; const float* edgeRest;
+    const unsigned long long* tetWord; const float2* tetAlpha;
+    const unsigned* edgeWord; const float* edgeRest;
     const int* tetSrc; const int* edgeSrc;                     // colour slots of the mesh's tables
     float4* mail;                                              // [2 x N] published values
     float4* mailStart;                                         // [2 x N] published substep-start positions (damped sweeps)
@@ -101,6 +102,7 @@ struct BrickEdge { unsigned word; float rest; };
 
 struct Brick {
     const BrickTables& bt;
+    const BrickShape& s;   // in the kernel's parameters or in shared memory
     BrickDesc d;
     float4* P;        // [maxLocal] positions (w = inverse mass)
     float4* Q;        // [maxLocal] damped sweeps, else [maxOwned]: substep-start positions
@@ -108,6 +110,7 @@ struct Brick {
     float4* A;        // [maxOwned] accelerations
     ContactFrame* frames;   // [kBrickFrames]
     float* typeB;     // [6 x 9] rest inverses
+    const float2* typeAlpha;   // [6] compliances per Kuhn type (sweeps without one per tet)
     int* head;        // offsets of this brick (brick_plan.h)
     const int *edgeOff, *tetOff, *impOff, *expOff;
     int2 *imports, *exports;   // this brick's lists in shared memory (listsShared)
@@ -115,38 +118,41 @@ struct Brick {
     unsigned* status; // barrier status word: kSyncTimeout once a wait ran out
     long long budget; unsigned lag;   // lag: epochs awaited beyond the published one (timeout test)
 
+    // Shared memory of a resident brick of the tables' largest sizes (the lists of the widest brick).
     static __host__ __device__ size_t bytes(const BrickTables& t, bool damped) {
-        const size_t head = (size_t)t.nEdgeColors + t.nTetColors + 2 * t.stages + 4;
+        const size_t head = (size_t)t.shape.nE + t.shape.nT + 2 * t.shape.stages + 6;
         const size_t all = sizeof(float4) * ((size_t)t.maxLocal + (damped ? t.maxLocal : t.maxOwned) + 2 * (size_t)t.maxOwned) +
-               kBrickFrames * sizeof(ContactFrame) + 54 * sizeof(float) + head * sizeof(int) +
-               (t.listsShared ? sizeof(int2) * ((size_t)t.maxImport + t.maxExport) : 0);
+                           kBrickFrames * sizeof(ContactFrame) + 54 * sizeof(float) + head * sizeof(int) +
+                           (t.listsShared ? sizeof(int2) * (size_t)t.maxList : 0);
         return (all + 15) & ~(size_t)15;
     }
     // Shared-memory layout, offsets and exchange lists.  Closed by a barrier.
-    __device__ __forceinline__ Brick(const BrickTables& t, const DeviceMesh& m, int b, float4* shared, bool damped, int exchanges, unsigned* statusWord,
-                     long long spinBudget, unsigned lagEpochs)
-        : bt(t), d(t.desc[b]), status(statusWord), budget(spinBudget), lag(lagEpochs) {
+    // resident: velocities, accelerations and substep-start positions live here too; else the caller keeps
+    // them in device memory (damped sweeps still read Q).
+    __device__ __forceinline__ Brick(const BrickTables& t, const BrickShape& shape, const float (&rest)[6][9], int b, float4* shared, bool damped,
+                                     bool resident, int exchanges, unsigned* statusWord, long long spinBudget, unsigned lagEpochs)
+        : bt(t), s(shape), d(t.desc[b]), status(statusWord), budget(spinBudget), lag(lagEpochs) {
         P = shared;
-        Q = P + t.maxLocal;
-        V = Q + (damped ? t.maxLocal : t.maxOwned);
-        A = V + t.maxOwned;
-        frames = (ContactFrame*)(A + t.maxOwned);
-        imports = (int2*)(frames + kBrickFrames);
-        exports = imports + (t.listsShared ? t.maxImport : 0);
-        typeB = (float*)(exports + (t.listsShared ? t.maxExport : 0));
+        Q = P + d.nLocal;
+        V = Q + (damped ? d.nLocal : resident ? d.nOwned : 0);
+        A = V + (resident ? d.nOwned : 0);
+        frames = (ContactFrame*)(A + (resident ? d.nOwned : 0));
+        typeB = (float*)(frames + (resident ? kBrickFrames : 0));
         head = (int*)(typeB + 54);
-        edgeOff = head; tetOff = edgeOff + t.nEdgeColors + 1; impOff = tetOff + t.nTetColors + 1; expOff = impOff + t.stages + 1;
-        const int words = t.nEdgeColors + t.nTetColors + 2 * t.stages + 4;
+        edgeOff = head; tetOff = edgeOff + s.nE + 1; impOff = tetOff + s.nT + 1; expOff = impOff + s.stages + 1;
+        const int words = s.nE + s.nT + 2 * s.stages + 4;
+        imports = (int2*)(head + (words + 1) / 2 * 2);
         for (int i = threadIdx.x; i < words; i += blockDim.x) head[i] = t.head[d.head + i];
-        for (int i = threadIdx.x; i < 54; i += blockDim.x) typeB[i] = m.typeB[i / 9][i % 9];
-        epoch = t.bricks > 1 ? t.epoch[b] : 0u;
+        for (int i = threadIdx.x; i < 54; i += blockDim.x) typeB[i] = rest[i / 9][i % 9];
+        epoch = s.bricks > 1 ? t.epoch[b] : 0u;
         __syncthreads();
+        exports = imports + (impOff[s.stages] - impOff[0]);
         if (t.listsShared) {
-            for (int i = threadIdx.x; i < impOff[t.stages] - impOff[0]; i += blockDim.x) imports[i] = t.importList[impOff[0] + i];
-            for (int i = threadIdx.x; i < expOff[t.stages] - expOff[0]; i += blockDim.x) exports[i] = t.exportList[expOff[0] + i];
+            for (int i = threadIdx.x; i < impOff[s.stages] - impOff[0]; i += blockDim.x) imports[i] = t.importList[impOff[0] + i];
+            for (int i = threadIdx.x; i < expOff[s.stages] - expOff[0]; i += blockDim.x) exports[i] = t.exportList[expOff[0] + i];
             __syncthreads();
         }
-        if (t.bricks > 1 && threadIdx.x == 0) t.epoch[b] = epoch + (unsigned)exchanges;   // also when a wait runs out
+        if (s.bricks > 1 && threadIdx.x == 0) t.epoch[b] = epoch + (unsigned)exchanges;   // also when a wait runs out
     }
 
     // The positions of owned and halo nodes, and the owned nodes' accelerations and velocities.
@@ -172,8 +178,14 @@ struct Brick {
                                bt.listsShared ? imports + (oi - impOff[0]) : bt.importList + oi, ni, epoch, lag, status, budget);
     }
 
-    __device__ __forceinline__ bool exchangeAt(int p) const { return (bt.exchangeBefore[p >> 6] >> (p & 63)) & 1ull; }
-    __device__ __forceinline__ BrickTet tetAt(int k) const { return {bt.tetWord[k], bt.tetAlpha[k]}; }
+    __device__ __forceinline__ bool exchangeAt(int p) const { return (s.before[p >> 6] >> (p & 63)) & 1ull; }
+    template <bool PerType>
+    __device__ __forceinline__ BrickTet tetAt(int k) const {
+        BrickTet t;
+        t.word = bt.tetWord[k];
+        if (!PerType) t.alpha = bt.tetAlpha[k];
+        return t;
+    }
     __device__ __forceinline__ BrickEdge edgeAt(int e) const { return {bt.edgeWord[e], bt.edgeRest[e]}; }
 
     template <bool Damped, bool Record>
@@ -191,7 +203,7 @@ struct Brick {
         }
         if (solveEdge(r, fc, pa, pb, oa, ob)) { P[a] = oa; P[b] = ob; }
     }
-    template <bool Damped, bool Record>
+    template <bool Damped, bool Record, bool PerType>
     __device__ __forceinline__ void tet(const BrickTet& w, const FrameCoeffs& fc, int k, const BrickTape& tape) {
         if (!(w.word & kBrickTetLive)) return;
         const unsigned lo = (unsigned)w.word, hi = (unsigned)(w.word >> 28);
@@ -205,7 +217,7 @@ struct Brick {
         f3 q[4], o[4];
 #pragma unroll
         for (int c = 0; c < 4; c++) q[c] = Damped ? xyz(Q[id[c]]) : mk(0.f, 0.f, 0.f);
-        if (!solveTet(typeB + 9 * ((hi >> 28) & 7u), p, q, w.alpha, fc, Damped && fc.dampingOverH != 0.f, false, o)) return;
+        if (!solveTet(typeB + 9 * ((hi >> 28) & 7u), p, q, PerType ? typeAlpha[(hi >> 28) & 7u] : w.alpha, fc, Damped && fc.dampingOverH != 0.f, false, o)) return;
 #pragma unroll
         for (int c = 0; c < 4; c++) P[id[c]] = make_float4(o[c].x, o[c].y, o[c].z, p[c].w);
     }
@@ -214,15 +226,15 @@ struct Brick {
     // exchange).  A thread always holds the record of its next element, loaded while it projects the one
     // before, across colours and exchanges.  Opens and closes with a barrier; false on a timeout.
     // after(edges) is called when a colour is done.
-    template <bool Damped, bool Record = false, class After>
+    template <bool Damped, bool Record = false, bool PerType = false, class After>
     __device__ __forceinline__ bool sweep(const FrameCoeffs& fc, After&& after, const BrickTape& tape = BrickTape()) {
         const int T = blockDim.x, tid = threadIdx.x;
-        const int nE = bt.nEdgeColors, nT = bt.nTetColors;
+        const int nE = s.nE, nT = s.nT;
         int st = 0;
         BrickEdge nextEdge;
         BrickTet nextTet;
         if (fc.doEdges && nE > 0 && edgeOff[0] + tid < edgeOff[1]) nextEdge = edgeAt(edgeOff[0] + tid);
-        if (fc.doStrain && nT > 0 && tetOff[0] + tid < tetOff[1]) nextTet = tetAt(tetOff[0] + tid);
+        if (fc.doStrain && nT > 0 && tetOff[0] + tid < tetOff[1]) nextTet = tetAt<PerType>(tetOff[0] + tid);
         __syncthreads();
         {   // offsets two colours ahead: none is waited for (all zero when the phase is off)
             int lo = fc.doEdges ? edgeOff[0] : 0, hi = fc.doEdges ? edgeOff[min(1, nE)] : 0, hi2 = fc.doEdges ? edgeOff[min(2, nE)] : 0;
@@ -252,8 +264,8 @@ struct Brick {
                     const bool have = k < hi, last = k + T >= hi;
                     const BrickTet cur = nextTet;
                     const int kn = last ? hi + tid : k + T;
-                    if (kn < (last ? hi2 : hi)) nextTet = tetAt(kn);
-                    if (have) tet<Damped, Record>(cur, fc, k, tape);
+                    if (kn < (last ? hi2 : hi)) nextTet = tetAt<PerType>(kn);
+                    if (have) tet<Damped, Record, PerType>(cur, fc, k, tape);
                     if (last) break;
                     k = kn;
                 }

@@ -37,8 +37,8 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
                                            const ContactParams& cp, const BrickTables& bt, unsigned* state) {
     extern __shared__ float4 shared[];
     const int tid = threadIdx.x, T = blockDim.x;
-    const int exchanges = bt.bricks > 1 ? fc.substeps * bt.stages : 0;
-    Brick b(bt, m, blockIdx.x, shared, Damped, exchanges, state + 2, fc.spinBudget, fc.syncTestExtra > 0 ? 1u << 30 : 0u);
+    const int exchanges = bt.bricks > 1 ? fc.substeps * bt.shape.stages : 0;
+    Brick b(bt, bt.shape, m.typeB, blockIdx.x, shared, Damped, true, exchanges, state + 2, fc.spinBudget, fc.syncTestExtra > 0 ? 1u << 30 : 0u);
     const bool stamp = fc.phaseClock != nullptr && blockIdx.x == 0 && tid == 0;
     int s = 0, slot = 0;
     auto mark = [&](unsigned tag) {
@@ -157,9 +157,8 @@ cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int 
     asked = plan.asked;
     threads = plan.threads < kBrickThreads ? plan.threads : kBrickThreads;
     BrickTables q{};
-    q.stages = plan.stages; q.nEdgeColors = plan.nEdgeColors; q.nTetColors = plan.nTetColors;
+    q.shape = plan.shape();
     q.maxLocal = plan.maxLocal; q.maxOwned = plan.maxOwned; q.nIdle = (int)plan.idle.size(); q.N = N;
-    q.exchangeBefore[0] = plan.exchangeBefore[0]; q.exchangeBefore[1] = plan.exchangeBefore[1];
     cudaError_t e = put((BrickDesc**)&q.desc, plan.desc.data(), plan.desc.size(), stream);
     if (e == cudaSuccess) e = put((int**)&q.head, plan.head.data(), plan.head.size(), stream);
     if (e == cudaSuccess) e = put((int**)&q.localNode, plan.localNode.data(), plan.localNode.size(), stream);
@@ -181,7 +180,7 @@ cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int 
     q.tetSrc = tetSrc; q.edgeSrc = edgeSrc;
     q.bricks = plan.bricks;
     // the exchange lists, next to the node state, when shared memory holds both
-    q.maxImport = plan.maxImport; q.maxExport = plan.maxExport;
+    q.maxList = plan.maxList;
     q.listsShared = 1;
     if (Brick::bytes(q, damped) > (size_t)maxBytes) q.listsShared = 0;
     t = q;

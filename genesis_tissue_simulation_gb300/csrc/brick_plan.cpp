@@ -121,7 +121,7 @@ constexpr int kOneBrick = 500;
 
 }  // namespace
 
-BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int forced, bool wholeHalo, bool reverse) {
+BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int forced, bool wholeHalo, bool reverse, int maxThreads) {
     BrickPlan none;
     maxLocal = std::min(maxLocal, kBrickMaxLocal);
     const int E = m.nEdgeColors ? m.edgeOff[m.nEdgeColors] : 0, T = m.nTetColors ? m.tetOff[m.nTetColors] : 0;
@@ -199,7 +199,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
     std::vector<std::vector<std::vector<int>>> elements(B, std::vector<std::vector<int>>(P)), imports(B, std::vector<std::vector<int>>(S));
     // body(brick, the thread's own workspace of type W)
     auto parallel = [&](auto&& workspace, auto&& body) {
-        const int threads = std::max(1, std::min({(int)std::thread::hardware_concurrency(), 16, B, 1 + served / 200}));
+        const int threads = std::max(1, std::min({(int)std::thread::hardware_concurrency(), maxThreads, B, 1 + served / 200}));
         std::atomic<int> next{0};
         auto run = [&]() {
             auto own = workspace();
@@ -272,7 +272,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
     };
     for (int b = 0; b < B; b++) {
         int* h = plan.head.data() + (size_t)b * headWords;
-        plan.desc[b] = {nNode, (int)owned[b].size(), (int)(owned[b].size() + halo[b].size()), b * headWords};
+        plan.desc[b] = {nNode, (int)owned[b].size(), (int)(owned[b].size() + halo[b].size()), b * headWords, 0};
         nNode += plan.desc[b].nLocal;
         // colours in sweep order
         for (int c = 0; c < m.nEdgeColors; c++) { *h++ = nEdge; nEdge += (int)elements[b][phaseOf(true, reverse ? m.nEdgeColors - 1 - c : c)].size(); }
@@ -324,9 +324,9 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         }
     });
     for (int b = 0; b < B; b++) {
-        int in = 0, out = 0;
-        for (int st = 0; st < S; st++) { in += (int)imports[b][st].size(); out += (int)exports[b][st].size(); }
-        plan.maxImport = std::max(plan.maxImport, in); plan.maxExport = std::max(plan.maxExport, out);
+        int records = 0;
+        for (int st = 0; st < S; st++) records += (int)(imports[b][st].size() + exports[b][st].size());
+        plan.maxList = std::max(plan.maxList, records);
     }
     for (auto& lists : elements) for (auto& list : lists) plan.threads = std::max(plan.threads, ((int)list.size() + 31) / 32 * 32);
     plan.bricks = B; plan.asked = count; plan.stages = S; plan.nEdgeColors = m.nEdgeColors; plan.nTetColors = m.nTetColors; plan.cost = cost;

@@ -13,6 +13,13 @@ namespace gbt {
 struct BrickDesc {
     int nodeBase, nOwned, nLocal;   // localNode[nodeBase + l]: node of local index l, owned nodes first
     int head;
+    int shape;                      // of a batch: the instance's plan
+};
+
+// The sweep of one plan: colours, stages, and the phases an exchange precedes (bit p: phase p).
+struct BrickShape {
+    int nE, nT, stages, bricks;
+    unsigned long long before[2];
 };
 
 // Element words.  A tet: local nodes in bits 0-13, 14-27, 28-41 and 42-55, Kuhn type 56-58, live 59.
@@ -32,7 +39,7 @@ struct BrickMesh {   // the coloured mesh a plan is made for; nodes on an nx * n
 };
 
 struct BrickPlan {
-    int bricks = 0, stages = 1, nEdgeColors = 0, nTetColors = 0, maxLocal = 0, maxOwned = 0, maxImport = 0, maxExport = 0;
+    int bricks = 0, stages = 1, nEdgeColors = 0, nTetColors = 0, maxLocal = 0, maxOwned = 0, maxList = 0;
     int asked = 0;                         // the brick count the split was chosen for
     int threads = 32;                      // of a CTA: the widest phase, in whole warps
     uint64_t exchangeBefore[2] = {0, 0};   // bit p: neighbours' values are taken before phase p (edge colours, then tet colours)
@@ -43,12 +50,15 @@ struct BrickPlan {
     std::vector<uint64_t> tetWord; std::vector<int> tetSrc;
     std::vector<unsigned> edgeWord; std::vector<float> edgeRest; std::vector<int> edgeSrc;
     bool ok() const { return bricks > 0; }
+    BrickShape shape() const { return {nEdgeColors, nTetColors, stages, bricks, {exchangeBefore[0], exchangeBefore[1]}}; }
 };
 
 // The plan of `mesh` on at most `maxBricks` CTAs that keep at most `maxLocal` nodes each; forced > 0
 // asks for about that many bricks instead of the cheapest count.  wholeHalo: the first exchange takes
 // every halo node (damped sweeps read all of them at the substep's start).  reverse: the sweep runs tet
 // colours and then edge colours from last to first.  Returns a plan without bricks when none fits.
-BrickPlan buildBrickPlan(const BrickMesh& mesh, int maxBricks, int maxLocal, int forced, bool wholeHalo, bool reverse = false);
+// At most `maxThreads` host threads.
+BrickPlan buildBrickPlan(const BrickMesh& mesh, int maxBricks, int maxLocal, int forced, bool wholeHalo, bool reverse = false,
+                         int maxThreads = 16);
 
 }  // namespace gbt

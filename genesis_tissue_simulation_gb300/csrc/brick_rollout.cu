@@ -66,7 +66,7 @@ __device__ __forceinline__ void forwardBricks(const DeviceMesh& m, const DiffCoe
     extern __shared__ float4 shared[];
     const int N = db.total / db.frames, tid = threadIdx.x, step = blockDim.x;
     const FrameCoeffs fc = rollCoeffs(dc);
-    Brick b(bt, m, blockIdx.x, shared, Damped, bt.bricks > 1 ? db.total * bt.stages : 0, barrier + 1, budget, 0u);
+    Brick b(bt, bt.shape, m.typeB, blockIdx.x, shared, Damped, true, bt.bricks > 1 ? db.total * bt.shape.stages : 0, barrier + 1, budget, 0u);
     b.loadState(m.pos, m.vel, m.ext);
     for (int g = 0; g < db.total; g++) {
         if (g % db.every == 0) {
@@ -98,7 +98,7 @@ __device__ __forceinline__ void forwardBricks(const DeviceMesh& m, const DiffCoe
 template <bool Damped>
 __device__ __forceinline__ bool reverseSweep(Brick& b, const DeviceMesh& m, const DiffCoeffs& dc, const DiffBuffers& db, int j, int E, int T) {
     const int tid = threadIdx.x, step = blockDim.x;
-    const int nE = b.bt.nEdgeColors, nT = b.bt.nTetColors;
+    const int nE = b.s.nE, nT = b.s.nT;
     int st = 0;
     __syncthreads();
     if (dc.doStrain) {
@@ -110,7 +110,7 @@ __device__ __forceinline__ bool reverseSweep(Brick& b, const DeviceMesh& m, cons
         auto fetch = [&]() {
             Slot s;
             s.valid = fc < nT && fk < b.tetOff[fc + 1];
-            if (s.valid) { s.t = b.tetAt(fk); s.src = b.bt.tetSrc[fk]; }
+            if (s.valid) { s.t = b.tetAt<false>(fk); s.src = b.bt.tetSrc[fk]; }
             if (fc < nT) {
                 if (fk + step < b.tetOff[fc + 1]) fk += step;
                 else { fc++; if (fc < nT) fk = b.tetOff[fc] + tid; }
@@ -198,9 +198,9 @@ __device__ __forceinline__ void backwardBricks(const DeviceMesh& m, const DiffCo
     const int E = m.nEdgeColors > 0 ? m.edgeRange[m.nEdgeColors - 1].y : 0, T = m.nTetColors > 0 ? m.tetRange[m.nTetColors - 1].y : 0;
     const FrameCoeffs fc = rollCoeffs(dc);
     GridSync grid{barrier, barrier + 1, gridDim.x, 0u, budget, 0u};
-    Brick b(bt, m, blockIdx.x, shared, Damped, bt.bricks > 1 ? db.total * bt.stages : 0, barrier + 1, budget, 0u);
-    Brick v(rt, m, blockIdx.x, shared + Brick::bytes(bt, Damped) / sizeof(float4), Damped, rt.bricks > 1 ? db.total * rt.stages : 0, barrier + 1,
-            budget, 0u);
+    Brick b(bt, bt.shape, m.typeB, blockIdx.x, shared, Damped, true, bt.bricks > 1 ? db.total * bt.shape.stages : 0, barrier + 1, budget, 0u);
+    Brick v(rt, rt.shape, m.typeB, blockIdx.x, shared + Brick::bytes(bt, Damped) / sizeof(float4), Damped, true,
+            rt.bricks > 1 ? db.total * rt.shape.stages : 0, barrier + 1, budget, 0u);
     for (int i = tid; i < v.d.nOwned; i += step) {
         v.P[i] = db.gx[rt.localNode[v.d.nodeBase + i]];
         v.V[i] = v.A[i] = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -1225,7 +1225,7 @@ LCS_API int GBT_SetBrickCount(int count) {
 // (bricks 0: no plan).
 LCS_API int GBT_BrickInfo(int* out4) {
     if (!S.physReady || !out4) return XPBD_ERR_NOT_READY;
-    out4[0] = S.bricks.t.bricks; out4[1] = S.bricks.t.bricks > 1 ? S.bricks.t.stages : 0; out4[2] = S.bricks.threads; out4[3] = S.bricks.t.maxLocal;
+    out4[0] = S.bricks.t.bricks; out4[1] = S.bricks.t.bricks > 1 ? S.bricks.t.shape.stages : 0; out4[2] = S.bricks.threads; out4[3] = S.bricks.t.maxLocal;
     return 0;
 }
 

@@ -224,3 +224,21 @@ def test_per_tet_stiffness_keeps_explicit_tables(gpu_lib):
         assert b.element_tables() == "explicit"
         with pytest.raises(RuntimeError):
             b.set_element_tables(True)
+
+
+@pytest.mark.parametrize("count,lo,hi,damping,ks", [(1, 3, 5, 0.0, 1e6), (3, 4, 9, 0.04, 1e6), (5, 4, 12, 0.04, 0.0), (200, 3, 5, 0.0, 1e6)])
+def test_bricks_match_the_instance_kernels(gpu_lib, count, lo, hi, damping, ks):
+    """Mode 0 on bricks (one brick, split instances, more instances than SMs) against one CTA per
+    instance, graph replay included."""
+    wl = BT.make_c4(count=count, seed=5, steps=3, size_range=((lo, hi), (3, max(4, hi // 2)), (lo, hi)))
+    runs = []
+    for mode, threads in ((0, 256), (1, 256)):
+        with BT.TissueBatch(wl.grids, dt=1 / 60, substeps=3, ks=ks, strain_damping_s=damping, stiffness_scale=wl.stiffness_scale(),
+                            grasp_params=GraspParams(**GRASP), dll_path=gpu_lib) as b:
+            b.set_launch(mode, threads)
+            b.set_gravity(0.0, -981.0, 0.0)
+            b.set_capsules(wl.capsules_at(0))
+            for k in range(3):
+                b.step_many([wl.capsules_at(k + 1)], use_graph=k > 0)
+            runs.append(b.positions())
+    assert np.array_equal(runs[0], runs[1])
