@@ -1,12 +1,15 @@
 // One frame of a single mesh on spatial bricks (brick_frame.cuh), and the upkeep of a plan's tables.
 #include "brick_kernels.h"
 #include "contact_point.cuh"
+#include "particle_frame.cuh"
+#include "ribbon_tick.cuh"
 
 namespace gbt {
 namespace {
 
-// A node no element touches through its substeps, as the brick's node phases treat its own.
-__device__ void idleNode(const DeviceMesh& m, int n, const FrameCoeffs& fc, const ToolPose& from, const ToolPose& to, const ContactParams& cp) {
+// A node no element touches through substeps [s0, s1), as the brick's node phases treat its own.
+__device__ void idleNode(const DeviceMesh& m, int n, const FrameCoeffs& fc, const ToolPose& from, const ToolPose& to, const ContactParams& cp,
+                         int s0, int s1) {
     float4 P = m.pos[n], Q = P;
     f3 V = xyz(m.vel[n]);
     if (!(P.w > 0.f)) {
@@ -16,7 +19,7 @@ __device__ void idleNode(const DeviceMesh& m, int n, const FrameCoeffs& fc, cons
     }
     const float4 F = m.ext[n];
     const f3 a = mk(F.x, F.y, F.z) * P.w;
-    for (int s = 0; s < fc.substeps; s++) {
+    for (int s = s0; s < s1; s++) {
         Q = P;
         V = V + a * fc.h;
         f3 x = xyz(P) + V * fc.h;
@@ -32,9 +35,69 @@ __device__ void idleNode(const DeviceMesh& m, int n, const FrameCoeffs& fc, cons
     m.vel[n] = make_float4(V.x, V.y, V.z, 0.f);
 }
 
-template <bool Damped>
+// The ribbon tick after a substep of a blade frame: the crossing test of the edges near the blade over
+// the whole grid, then the live bits of this brick's elements where links were severed, then fresh
+// particle frames where cut points were emitted (not after the frame's last substep).  Positions and
+// substep-start positions are in device memory.  Out of line: a tick is a few microseconds of the
+// substep, and its registers stay out of the sweep's.  False when a barrier timed out.
+struct TickState { unsigned derivedAt; int rotParity; unsigned target; bool ok; };
+__device__ __noinline__ TickState ribbonTick(const DeviceMesh& m, const CutParams& cu, const BrickTables& bt, int e0, int e1, int t0, int t1,
+                                             bool lastSubstep, bool rotations, unsigned* barrier, long long budget, TickState ts) {
+    GridSync grid{barrier, barrier + 1, gridDim.x, ts.target, budget, 0u};
+    ts.ok = false;
+    const int r = grid.spreadRank(), R = grid.size();
+    const unsigned pointsBefore = *(volatile unsigned*)(cu.counters + 1);
+    if (!grid.sync()) return ts;
+    const float* rot = rotations ? m.particleRot[ts.rotParity] : nullptr;
+    if (cu.brickList && cu.tearLen2 <= 0.f) {
+        const int nb = ((m.dx + kBrick - 1) / kBrick) * ((m.dy + kBrick - 1) / kBrick) * ((m.dz + kBrick - 1) / kBrick);
+        for (int k = r >> 5; k < nb; k += R >> 5) brickBounds(m, cu, k, r & 31);
+        if (!grid.sync()) return ts;
+        const int listed = min((int)*(volatile unsigned*)cu.brickCount, nb);
+        for (int j = r; j < listed * kBrickEdges; j += R) {
+            int4 g;
+            if (brickEdge(m, *(volatile int*)(cu.brickList + j / kBrickEdges), j % kBrickEdges, g)) tickEdgeAt(m, cu, g, true, rot);
+        }
+    } else {
+        for (int e = r; e < cu.nGridEdges; e += R) tickEdge(m, cu, e, true, rot);
+    }
+    if (!grid.sync()) return ts;
+    if (grid.leader() && cu.brickCount) *cu.brickCount = 0u;   // every reader has passed the barrier above
+    const unsigned revision = *(volatile unsigned*)cu.counters;
+    if (revision != ts.derivedAt) {
+        ts.derivedAt = revision;
+        unsigned* edgeWord = (unsigned*)bt.edgeWord;
+        unsigned long long* tetWord = (unsigned long long*)bt.tetWord;
+        for (int k = e0 + threadIdx.x; k < e1; k += blockDim.x) {
+            const int e = bt.edgeSrc[k];
+            const int2 ij = m.edgeEnds[e];
+            const bool live = m.nbr[m.edgeOwner[e]] >= 0 && m.active[ij.x] != 0 && m.active[ij.y] != 0;
+            edgeWord[k] = (edgeWord[k] & ~kBrickEdgeLive) | (live ? kBrickEdgeLive : 0u);
+        }
+        for (int k = t0 + threadIdx.x; k < t1; k += blockDim.x) {
+            const int t = bt.tetSrc[k];
+            const int4 d = m.tetIds[t];
+            const int* o = m.tetOwner + 3 * t;
+            const bool live = m.nbr[o[0]] >= 0 && m.nbr[o[1]] >= 0 && m.nbr[o[2]] >= 0 && m.active[d.x] != 0 && m.active[d.y] != 0 &&
+                              m.active[d.z] != 0 && m.active[d.w] != 0;
+            tetWord[k] = (tetWord[k] & ~kBrickTetLive) | (live ? kBrickTetLive : 0ull);
+        }
+    }
+    if (rotations && !lastSubstep && *(volatile unsigned*)(cu.counters + 1) != pointsBefore) {
+        for (int i = m.nodeBase + r; i < m.nodeBase + m.nNodes; i += R)
+            particleFrame(i, m.pos, m.nbr, m.active, m.pinned, m.particleRot[ts.rotParity], m.particleRot[ts.rotParity ^ 1]);
+        ts.rotParity ^= 1;
+        if (!grid.sync()) return ts;
+    }
+    __syncthreads();   // the live bits before the next sweep reads them
+    ts.target = grid.target;
+    ts.ok = true;
+    return ts;
+}
+
+template <bool Damped, bool Cut>
 __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeffs& fc, const ToolPose& from, const ToolPose& to,
-                                           const ContactParams& cp, const BrickTables& bt, unsigned* state) {
+                                           const ContactParams& cp, const BrickTables& bt, const CutParams& cu, unsigned* state) {
     extern __shared__ float4 shared[];
     const int tid = threadIdx.x, T = blockDim.x;
     const int exchanges = bt.bricks > 1 ? fc.substeps * bt.shape.stages : 0;
@@ -49,6 +112,8 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
         }
     };
     b.loadState(m.pos, m.vel, m.ext);
+    TickState ts{Cut ? *(volatile unsigned*)cu.counters : 0u, fc.rotParity, 0u, true};
+    bool havePrev = cu.havePrev != 0;
     for (; s < fc.substeps; s++) {
         slot = 0;
         mark(kPhaseFrameStart);
@@ -85,6 +150,23 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
             b.V[i] = make_float4(v.x, v.y, v.z, 0.f);
         }
         mark(kPhaseVelocity);
+        if (Cut) {   // the first tick after the blade is set only takes the position snapshot
+            if (havePrev) {
+                for (int i = tid; i < b.d.nOwned; i += T) {
+                    const int n = bt.localNode[b.d.nodeBase + i];
+                    m.pos[n] = b.P[i];
+                    m.prev[n] = b.Q[i];
+                }
+                for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode(m, bt.idle[i], fc, from, to, cp, s, s + 1);
+                ts = ribbonTick(m, cu, bt, b.edgeOff[0], b.edgeOff[b.s.nE], b.tetOff[0], b.tetOff[b.s.nT],
+                                fc.firstSubstep + s + 1 >= fc.numSubsteps, fc.rotations != 0, state + 1, fc.spinBudget, ts);
+                if (!ts.ok) return;
+                mark(kPhaseTick);
+            } else {
+                for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode(m, bt.idle[i], fc, from, to, cp, s, s + 1);
+            }
+            havePrev = true;
+        }
     }
     for (int i = tid; i < b.d.nOwned; i += T) {
         const int n = bt.localNode[b.d.nodeBase + i];
@@ -92,8 +174,12 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
         m.prev[n] = b.Q[i];
         m.vel[n] = b.V[i];
     }
-    for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode(m, bt.idle[i], fc, from, to, cp);
-    if (blockIdx.x == 0 && tid == 0) { state[1] = (unsigned)exchanges; state[3] = (unsigned)fc.rotParity; }
+    if (!Cut)
+        for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode(m, bt.idle[i], fc, from, to, cp, 0, fc.substeps);
+    if (blockIdx.x == 0 && tid == 0) {
+        if (!Cut) state[1] = (unsigned)exchanges;   // with ticks it is the grid barrier's counter, which others may still read
+        state[3] = (unsigned)ts.rotParity;
+    }
 }
 
 __global__ void meshFlagsKernel(DeviceMesh m, int E, int T, int fallback) {
@@ -125,13 +211,15 @@ __global__ void brickAlphaKernel(int tets, const int* tetSrc, float invH2, const
 
 }  // namespace
 
-__global__ void __launch_bounds__(kBrickThreads, 1) brickFrameKernel(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to,
-                                                                     ContactParams cp, BrickTables bt, unsigned* state) {
-    brickFrame<false>(m, fc, from, to, cp, bt, state);
+template <bool Damped, bool Cut>
+static __global__ void __launch_bounds__(kBrickThreads, 1) brickFrameKernel(const __grid_constant__ DeviceMesh m, FrameCoeffs fc, ToolPose from,
+                                                                            ToolPose to, ContactParams cp, const __grid_constant__ BrickTables bt,
+                                                                            const __grid_constant__ CutParams cu, unsigned* state) {
+    brickFrame<Damped, Cut>(m, fc, from, to, cp, bt, cu, state);
 }
-__global__ void __launch_bounds__(kBrickThreads, 1) brickFrameKernelDamped(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to,
-                                                                           ContactParams cp, BrickTables bt, unsigned* state) {
-    brickFrame<true>(m, fc, from, to, cp, bt, state);
+BrickFrameKernel brickFrameKernelFor(bool damped, bool cut) {
+    return damped ? (cut ? brickFrameKernel<true, true> : brickFrameKernel<true, false>)
+                  : (cut ? brickFrameKernel<false, true> : brickFrameKernel<false, false>);
 }
 
 template <class T> cudaError_t BrickBuffers::put(T** to, const T* from, size_t count, cudaStream_t stream) {

@@ -4,10 +4,11 @@
 
 namespace gbt {
 
-__global__ void brickFrameKernel(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to, ContactParams cp, BrickTables bt,
-                                 unsigned* state);
-__global__ void brickFrameKernelDamped(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to, ContactParams cp, BrickTables bt,
-                                       unsigned* state);
+// The frame kernel; cut: with the blade's ribbon tick between substeps.  `state` as for the other frame
+// kernels ([1] and [2] zero; the exchanges run are left in [1] without a cut, the frame parity in [3]).
+using BrickFrameKernel = void (*)(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to, ContactParams cp, BrickTables bt, CutParams cu,
+                                  unsigned* state);
+BrickFrameKernel brickFrameKernelFor(bool damped, bool cut);
 
 // A plan's tables on the device.
 struct BrickBuffers {

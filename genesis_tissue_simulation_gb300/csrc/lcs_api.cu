@@ -196,8 +196,8 @@ int ensureStream() {
     CK(cudaFuncGetAttributes(&ca, (const void*)frameKernelSessionCluster));
     S.maxClusterBytes = optin - (int)ca.sharedSizeBytes;   // dynamic bytes left beside its static shared memory
     CK(cudaFuncSetAttribute((const void*)frameKernelSessionCluster, cudaFuncAttributeMaxDynamicSharedMemorySize, S.maxClusterBytes));
-    for (const void* k : {(const void*)brickFrameKernel, (const void*)brickFrameKernelDamped})
-        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
+    for (int k = 0; k < 4; k++)
+        CK(cudaFuncSetAttribute((const void*)brickFrameKernelFor(k & 1, k >> 1), cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
     S.maxBrickBytes = optin - 1024;
     int khz = 0;
     if (cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, S.device) == cudaSuccess && khz > 0) S.clockKHz = khz;
@@ -348,10 +348,10 @@ CutParams cutParams() {
 // (*followUp set), so the host flips the parity the kernel leaves in state[3].
 // Launch shapes of a frame: one CTA, the whole GPU, one thread-block cluster.
 constexpr int kShapeBlock = 0, kShapeGrid = 1, kShapeCluster = 2;
-// Automatic mode runs plain frames (no bends, perpendicular damping, guard, friction or blade) on bricks
-// wherever a plan fits.
+// Automatic mode runs plain and blade frames (no bends, perpendicular damping, guard or friction; a
+// blade not with the tet-support fallback, whose edge flags cross bricks) on bricks wherever a plan fits.
 bool brickFrames(const FrameCoeffs& fc) {
-    return S.launchMode == 0 && S.bricks.ready() && !fc.doBend && !fc.perpDamp && !fc.guarded && !fc.friction && !fc.cut;
+    return S.launchMode == 0 && S.bricks.ready() && !fc.doBend && !fc.perpDamp && !fc.guarded && !fc.friction && !(fc.cut && fc.fallback);
 }
 int launchBricks(const FrameCoeffs& fc, bool* followUp) {
     DeviceMesh m = deviceMesh();
@@ -364,12 +364,14 @@ int launchBricks(const FrameCoeffs& fc, bool* followUp) {
     ToolPose from = S.toolFrom, to = S.tool;
     ContactParams cp = S.cp;
     unsigned* state = S.state.p;
-    void* args[] = {&m, &f, &from, &to, &cp, &S.bricks.t, &state};
-    CK(cudaLaunchCooperativeKernel(S.bricksDamped ? (const void*)brickFrameKernelDamped : (const void*)brickFrameKernel, dim3(S.bricks.t.bricks),
-                                   dim3(S.bricks.threads), args, S.bricks.sharedBytes(S.bricksDamped), S.stream));
-    particleRotKernel<<<(S.N + 255) / 256, 256, 0, S.stream>>>(m, nullptr, fc.rotParity);
+    CutParams cu = cutParams();
+    if (fc.cut && S.brickCount.p) CK(cudaMemsetAsync(S.brickCount.p, 0, sizeof(unsigned), S.stream));
+    void* args[] = {&m, &f, &from, &to, &cp, &S.bricks.t, &cu, &state};
+    CK(cudaLaunchCooperativeKernel((const void*)brickFrameKernelFor(S.bricksDamped, fc.cut != 0), dim3(S.bricks.t.bricks), dim3(S.bricks.threads),
+                                   args, S.bricks.sharedBytes(S.bricksDamped), S.stream));
+    particleRotKernel<<<(S.N + 255) / 256, 256, 0, S.stream>>>(m, fc.cut ? state + 3 : nullptr, fc.rotParity);
     CK(cudaGetLastError());
-    S.lastFrameBlocks = 1;   // the kernel leaves its exchanges in the barrier counter
+    S.lastFrameBlocks = fc.cut ? S.bricks.t.bricks : 1;   // without a cut the kernel leaves its exchanges in the barrier counter
     *followUp = true;
     return 0;
 }
@@ -942,6 +944,7 @@ LCS_API int LCS_Step(float dt) {
         fc.phaseClock = S.phaseClock.p;
     }
     bool followUp = false;
+    const bool onBricks = brickFrames(fc);
     int rc = launchFrame(fc, &followUp);
     if (rc) return rc;
     if (S.profile) { CK(cudaEventRecord(e1, S.stream)); S.events.push_back(e0); S.events.push_back(e1); }
@@ -966,7 +969,9 @@ LCS_API int LCS_Step(float dt) {
             last = ns;
         }
     }
-    if (fc.cut) S.havePrev = S.bricksStale = true;
+    if (fc.cut) S.havePrev = true;
+    if (fc.cut && !onBricks) S.bricksStale = true;   // the tick on bricks keeps their live bits itself
+    if (S.hostState[2] != 0u) S.bricksStale = true;
     if (S.toolArmed) S.toolFrom = S.tool;
     if (S.hostState[2] != 0u) return LCS_ERR_DEVICE_TIMEOUT;
     S.rotParity = (int)((S.hostState[3] & 1u) ^ (followUp ? 1u : 0u));

@@ -14,13 +14,13 @@ pytestmark = pytest.mark.gpu
 LATTICES = {(2, 2, 2): (1, 2, 8), (2, 9, 2): (1, 3, 30), (17, 3, 11): (1, 4, 61), (9, 6, 13): (1, 2, 27, 152)}
 
 
-def frames(lib, size, bricks=0, mode=0, damping=0.0, ks=1e6, capsule=True, steps=3, substeps=5, blade_at=None):
+def frames(lib, size, bricks=0, mode=0, damping=0.0, ks=1e6, capsule=True, steps=3, substeps=5, blade_at=None, crossing=False, tear=0.0):
     grid = build_grid(0.2, size=tuple(np.float64(c) * 0.2 - 0.02 for c in size), density=1000.0)
     dll = ct.CDLL(str(lib))
     gpu = hasattr(dll, "GBT_SetBrickCount")
     if gpu:
         assert dll.GBT_SetBrickCount(bricks) == 0
-    with PlainTissue(grid, dt=1 / 60, substeps=substeps, ks=ks, strain_damping_s=damping, dll_path=lib) as t:
+    with PlainTissue(grid, dt=1 / 60, substeps=substeps, ks=ks, strain_damping_s=damping, tear_ratio=tear, dll_path=lib) as t:
         info = np.zeros(4, np.int32)
         try:
             if gpu:
@@ -36,7 +36,11 @@ def frames(lib, size, bricks=0, mode=0, damping=0.0, ks=1e6, capsule=True, steps
                 if detect:
                     t.set_blade(blade_sweep((mid[0], top + 1.0, mid[2] - 0.3), (mid[0], mid[1], mid[2] - 0.3),
                                             (mid[0], top + 1.0, mid[2] + 0.3), (mid[0], mid[1], mid[2] + 0.3)))
-                t.step(detect_cut=detect)
+                if crossing:   # a blade through the block, a little further every frame
+                    z0, z1 = mid[2] - 0.5 + 0.15 * k, mid[2] - 0.35 + 0.15 * k
+                    t.set_blade(blade_sweep((mid[0] + 0.02, top + 1.0, z0), (mid[0] + 0.02, mid[1], z0),
+                                            (mid[0] + 0.02, top + 1.0, z1), (mid[0] + 0.02, mid[1], z1)))
+                t.step(detect_cut=detect or crossing)
                 if detect:   # the blade is put away: plain frames of a severed lattice follow
                     t.functions["LCS_SetPressureCutMode"](1)
             rot = np.zeros((len(grid.positions), 9), np.float32)
@@ -65,6 +69,18 @@ def test_bricks_match_the_oracle_through_a_cut(gpu_lib, oracle_libs, bricks):
     got, _ = frames(gpu_lib, (9, 6, 13), bricks, steps=6, blade_at=2)
     want, _ = frames(oracle_libs[0], (9, 6, 13), steps=6, blade_at=2)
     assert (got[2] != want[2]).sum() == 0 and (got[2] < 0).sum() > 0
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("size,bricks", [((9, 6, 13), 1), ((9, 6, 13), 27), ((17, 3, 11), 61)])
+@pytest.mark.parametrize("options", [dict(), dict(damping=0.04), dict(tear=1.05)], ids=["plain", "damped", "tear"])
+def test_blade_frames_on_bricks_match_the_whole_gpu_frame(gpu_lib, size, bricks, options):
+    """Ticks between the substeps of frames whose links the rod-phase detection severs, and the particle frames after them."""
+    got, info = frames(gpu_lib, size, bricks, steps=6, crossing=True, **options)
+    want, _ = frames(gpu_lib, size, mode=1, steps=6, crossing=True, **options)
+    start = build_grid(0.2, size=tuple(np.float64(c) * 0.2 - 0.02 for c in size), density=1000.0).neighbors
+    assert info[0] >= 1 and (want[2] != start).sum() > 0
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
 
