@@ -425,7 +425,7 @@ int planBricks(const std::vector<HostMesh>& meshes, const GbtInstanceDesc* inst,
             edgeDead[i][k] = !(d.nbrIdx[hm.edgeOwner[k]] >= 0 && d.active[e.x] && d.active[e.y]) || (fallback && carried[hm.edgeOwner[k]]);
         }
         in[i] = {{hm.N, d.dimsX + 1, d.dimsY + 1, d.dimsZ + 1, d.active, eC, tC, hm.edgeColorOff.data(), hm.edgeEnds.data(), hm.edgeRest.data(),
-                  hm.tetColorOff.data(), hm.tetIds.data(), hm.tetMeta.data()},
+                  hm.tetColorOff.data(), hm.tetIds.data(), hm.tetMeta.data(), 0},
                  G.nodeBase[i], edgeSlot[i].data(), tetSlot[i].data(), edgeDead[i].data(), tetDead[i].data()};
     }
     CK(G.bricks.plan(in, G.N, G.smCount, one, two, G.strainDamping > 0.f, G.stream));

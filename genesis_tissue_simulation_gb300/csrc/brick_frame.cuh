@@ -120,7 +120,7 @@ struct Brick {
 
     // Shared memory of a resident brick of the tables' largest sizes (the lists of the widest brick).
     static __host__ __device__ size_t bytes(const BrickTables& t, bool damped) {
-        const size_t head = (size_t)t.shape.nE + t.shape.nT + 2 * t.shape.stages + 6;
+        const size_t head = (size_t)t.shape.nE + t.shape.nT + t.shape.nTensile + 2 * t.shape.stages + 6;
         const size_t all = sizeof(float4) * ((size_t)t.maxLocal + (damped ? t.maxLocal : t.maxOwned) + 2 * (size_t)t.maxOwned) +
                            kBrickFrames * sizeof(ContactFrame) + 54 * sizeof(float) + head * sizeof(int) +
                            (t.listsShared ? sizeof(int2) * (size_t)t.maxList : 0);
@@ -139,8 +139,8 @@ struct Brick {
         frames = (ContactFrame*)(A + (resident ? d.nOwned : 0));
         typeB = (float*)(frames + (resident ? kBrickFrames : 0));
         head = (int*)(typeB + 54);
-        edgeOff = head; tetOff = edgeOff + s.nE + 1; impOff = tetOff + s.nT + 1; expOff = impOff + s.stages + 1;
-        const int words = s.nE + s.nT + 2 * s.stages + 4;
+        edgeOff = head; tetOff = edgeOff + s.nE + 1; impOff = tetOff + s.nT + s.nTensile + 1; expOff = impOff + s.stages + 1;
+        const int words = s.nE + s.nT + s.nTensile + 2 * s.stages + 4;
         imports = (int2*)(head + (words + 1) / 2 * 2);
         for (int i = threadIdx.x; i < words; i += blockDim.x) head[i] = t.head[d.head + i];
         for (int i = threadIdx.x; i < 54; i += blockDim.x) typeB[i] = rest[i / 9][i % 9];
@@ -203,7 +203,8 @@ struct Brick {
         }
         if (solveEdge(r, fc, pa, pb, oa, ob)) { P[a] = oa; P[b] = ob; }
     }
-    template <bool Damped, bool Record, bool PerType>
+    // Guarded: the tissue guard's form when `guarded` (damping then includes the bulk's).
+    template <bool Damped, bool Record, bool PerType, bool Guarded>
     __device__ __forceinline__ void tet(const BrickTet& w, const FrameCoeffs& fc, int k, const BrickTape& tape) {
         if (!(w.word & kBrickTetLive)) return;
         const unsigned lo = (unsigned)w.word, hi = (unsigned)(w.word >> 28);
@@ -217,19 +218,52 @@ struct Brick {
         f3 q[4], o[4];
 #pragma unroll
         for (int c = 0; c < 4; c++) q[c] = Damped ? xyz(Q[id[c]]) : mk(0.f, 0.f, 0.f);
-        if (!solveTet(typeB + 9 * ((hi >> 28) & 7u), p, q, PerType ? typeAlpha[(hi >> 28) & 7u] : w.alpha, fc, Damped && fc.dampingOverH != 0.f, false, o)) return;
+        if (!solveTet(typeB + 9 * ((hi >> 28) & 7u), p, q, PerType ? typeAlpha[(hi >> 28) & 7u] : w.alpha, fc, Damped && tetDamped(fc, Guarded && fc.guarded != 0), Guarded && fc.guarded != 0, o)) return;
 #pragma unroll
         for (int c = 0; c < 4; c++) P[id[c]] = make_float4(o[c].x, o[c].y, o[c].z, p[c].w);
+    }
+
+    // Tensile reinforcement of one tet (one pass: its multipliers start at zero).
+    __device__ __forceinline__ void tensile(const BrickTet& w, const FrameCoeffs& fc) {
+        if (!(w.word & kBrickTetLive) || !(fc.tensileStrength > 0.f)) return;
+        const unsigned lo = (unsigned)w.word, hi = (unsigned)(w.word >> 28);
+        const int id[4] = {(int)(lo & kBrickNodeMask), (int)((lo >> kBrickNodeBits) & kBrickNodeMask), (int)(hi & kBrickNodeMask),
+                           (int)((hi >> kBrickNodeBits) & kBrickNodeMask)};
+        const float4 q[4] = {P[id[0]], P[id[1]], P[id[2]], P[id[3]]};
+        f3 p[4] = {xyz(q[0]), xyz(q[1]), xyz(q[2]), xyz(q[3])}, b[3];
+        const float* B = typeB + 9 * ((hi >> 28) & 7u);
+        b[0] = mk(B[0], B[1], B[2]); b[1] = mk(B[3], B[4], B[5]); b[2] = mk(B[6], B[7], B[8]);
+        float lambda[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        solveTensile(b, q, w.alpha.x / fmaxf(fc.tensileStrength, 1e-10f), lambda, p);
+#pragma unroll
+        for (int c = 0; c < 4; c++) P[id[c]] = make_float4(p[c].x, p[c].y, p[c].z, q[c].w);
+    }
+    // Whether any live tet that this brick owns is below the minimum relative volume (the guard's test),
+    // by this thread.
+    __device__ __forceinline__ bool belowMinimum(float minimum) const {
+        bool below = false;
+        for (int k = tetOff[0] + threadIdx.x; k < tetOff[s.nT]; k += blockDim.x) {
+            const unsigned long long w = bt.tetWord[k];
+            if (!(w & kBrickTetLive) || !(w & kBrickTetOwner)) continue;
+            const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 28);
+            const float* B = typeB + 9 * ((hi >> 28) & 7u);
+            const f3 b0 = mk(B[0], B[1], B[2]), b1 = mk(B[3], B[4], B[5]), b2 = mk(B[6], B[7], B[8]);
+            const f3 a = xyz(P[lo & kBrickNodeMask]), u = xyz(P[(lo >> kBrickNodeBits) & kBrickNodeMask]) - a,
+                     v = xyz(P[hi & kBrickNodeMask]) - a, x = xyz(P[(hi >> kBrickNodeBits) & kBrickNodeMask]) - a;
+            const float J = dot(u, cross(v, x)) * dot(b0, cross(b1, b2));
+            below = below || !isfinite(J) || J < minimum;
+        }
+        return below;
     }
 
     // One sweep over the colours from the positions in P (owned nodes current, halo by the first
     // exchange).  A thread always holds the record of its next element, loaded while it projects the one
     // before, across colours and exchanges.  Opens and closes with a barrier; false on a timeout.
     // after(edges) is called when a colour is done.
-    template <bool Damped, bool Record = false, bool PerType = false, class After>
+    template <bool Damped, bool Record = false, bool PerType = false, bool Guarded = false, class After>
     __device__ __forceinline__ bool sweep(const FrameCoeffs& fc, After&& after, const BrickTape& tape = BrickTape()) {
         const int T = blockDim.x, tid = threadIdx.x;
-        const int nE = s.nE, nT = s.nT;
+        const int nE = s.nE, nT = s.nT + (Guarded ? s.nTensile : 0);
         int st = 0;
         BrickEdge nextEdge;
         BrickTet nextTet;
@@ -265,7 +299,8 @@ struct Brick {
                     const BrickTet cur = nextTet;
                     const int kn = last ? hi + tid : k + T;
                     if (kn < (last ? hi2 : hi)) nextTet = tetAt<PerType>(kn);
-                    if (have) tet<Damped, Record, PerType>(cur, fc, k, tape);
+                    if (Guarded && c >= s.nT) { if (have) tensile(cur, fc); }
+                    else if (have) tet<Damped, Record, PerType, Guarded>(cur, fc, k, tape);
                     if (last) break;
                     k = kn;
                 }

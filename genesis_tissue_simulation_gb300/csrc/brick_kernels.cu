@@ -1,6 +1,8 @@
 // One frame of a single mesh on spatial bricks (brick_frame.cuh), and the upkeep of a plan's tables.
 #include "brick_kernels.h"
 #include "contact_point.cuh"
+#include "friction_contact.cuh"
+#include "guard_feasible.cuh"
 #include "particle_frame.cuh"
 #include "ribbon_tick.cuh"
 
@@ -8,7 +10,8 @@ namespace gbt {
 namespace {
 
 // A node no element touches through substeps [s0, s1), as the brick's node phases treat its own.
-__device__ void idleNode(const DeviceMesh& m, int n, const FrameCoeffs& fc, const ToolPose& from, const ToolPose& to, const ContactParams& cp,
+template <bool Extended>
+__device__ __noinline__ void idleNode(const DeviceMesh& m, int n, const FrameCoeffs& fc, const ToolPose& from, const ToolPose& to, const ContactParams& cp,
                          int s0, int s1) {
     float4 P = m.pos[n], Q = P;
     f3 V = xyz(m.vel[n]);
@@ -23,8 +26,12 @@ __device__ void idleNode(const DeviceMesh& m, int n, const FrameCoeffs& fc, cons
         Q = P;
         V = V + a * fc.h;
         f3 x = xyz(P) + V * fc.h;
+        const float t = fminf(1.f, (float)(fc.firstSubstep + s + 1) / (float)fc.numSubsteps);
+        if (Extended && fc.friction) {
+            const FrictionShapes shapes = frictionShapes(from, to, t, fmaxf(0.f, t - 1.f / (float)fc.numSubsteps), fc.jawThickness, cp.jawGapClosed);
+            x = frictionPoint(x, xyz(Q), P.w, shapes, fc.contactRadius, fc.contactAlphaH2, fc.muS, fc.muD);
+        }
         if (fc.contact) {
-            const float t = fminf(1.f, (float)(fc.firstSubstep + s + 1) / (float)fc.numSubsteps);
             x = contactPoint(x, P.w, V, contactFrame(from, to, t, cp, fc.contactAlphaH2), cp);
         }
         P = make_float4(x.x, x.y, x.z, P.w);
@@ -95,12 +102,26 @@ __device__ __noinline__ TickState ribbonTick(const DeviceMesh& m, const CutParam
     return ts;
 }
 
-template <bool Damped, bool Cut>
+// The guard's slow path, when some tet is below the minimum volume: the feasibility chain on the node
+// state in device memory, over the whole grid.
+struct GuardResult { unsigned target; bool ok; };
+__device__ __noinline__ GuardResult guardChain(const DeviceMesh& m, const FrameCoeffs& fc, int substepIndex, unsigned* barrier, unsigned target) {
+    GridSync grid{barrier, barrier + 1, gridDim.x, target, fc.spinBudget, 0u};
+    GuardResult g{target, false};
+    if (grid.sync() && guardFeasible(m, fc, substepIndex, grid)) g.ok = true;
+    g.target = grid.target;
+    return g;
+}
+
+// Extended: the tissue guard and contact model 1 are compiled in.
+template <bool Damped, bool Cut, bool Extended>
 __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeffs& fc, const ToolPose& from, const ToolPose& to,
                                            const ContactParams& cp, const BrickTables& bt, const CutParams& cu, unsigned* state) {
     extern __shared__ float4 shared[];
     const int tid = threadIdx.x, T = blockDim.x;
-    const int exchanges = bt.bricks > 1 ? fc.substeps * bt.shape.stages : 0;
+    const bool guarded = Extended && fc.guarded != 0;
+    const int exchanges = bt.bricks > 1 ? fc.substeps * (bt.shape.stages + (guarded ? 1 : 0)) : 0;
+    __shared__ FrictionShapes shapes[Extended ? kBrickFrames : 1];
     Brick b(bt, bt.shape, m.typeB, blockIdx.x, shared, Damped, true, exchanges, state + 2, fc.spinBudget, fc.syncTestExtra > 0 ? 1u << 30 : 0u);
     const bool stamp = fc.phaseClock != nullptr && blockIdx.x == 0 && tid == 0;
     int s = 0, slot = 0;
@@ -124,6 +145,13 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
                 b.frames[tid] = contactFrame(from, to, t, cp, fc.contactAlphaH2);
             }
         }
+        if (Extended && fc.friction && s % kBrickFrames == 0) {
+            __syncthreads();
+            if (tid < kBrickFrames && s + tid < fc.substeps) {
+                const float t = fminf(1.f, (float)(fc.firstSubstep + s + tid + 1) / (float)fc.numSubsteps);
+                shapes[tid] = frictionShapes(from, to, t, fmaxf(0.f, t - 1.f / (float)fc.numSubsteps), fc.jawThickness, cp.jawGapClosed);
+            }
+        }
         for (int i = tid; i < b.d.nOwned; i += T) {
             float4 P = b.P[i];
             b.Q[i] = make_float4(P.x, P.y, P.z, 0.f);
@@ -135,12 +163,46 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
             }
         }
         mark(kPhasePredict);
-        if (!b.sweep<Damped>(fc, [&](bool edges) { mark(edges ? kPhaseEdges : kPhaseTets); })) return;
+        if (!b.sweep<Damped, false, false, Extended>(fc, [&](bool edges) { mark(edges ? kPhaseEdges : kPhaseTets); })) return;
+        if (Extended && (fc.friction || guarded)) {   // contact, then the guard's feasibility test
+            for (int i = tid; i < b.d.nOwned; i += T) {
+                const float4 P = b.P[i];
+                if (!(P.w > 0.f)) continue;
+                f3 p = xyz(P);
+                if (fc.friction) p = frictionPoint(p, xyz(b.Q[i]), P.w, shapes[s % kBrickFrames], fc.contactRadius, fc.contactAlphaH2, fc.muS, fc.muD);
+                if (guarded && fc.contact) p = contactPoint(p, P.w, xyz(b.V[i]), b.frames[s % kBrickFrames], cp);
+                b.P[i] = make_float4(p.x, p.y, p.z, P.w);
+            }
+            __syncthreads();
+        }
+        if (guarded) {
+            if (bt.bricks > 1 && !b.exchange(0, false)) return;   // the whole halo: every owned tet's nodes
+            // one of three words in turn: a word is cleared while every brick is between its last read and
+            // its next write
+            unsigned* flag = m.guardFlags + 2;
+            if (b.belowMinimum(fc.minVolume)) flag[s % 3] = 1u;
+            GridSync grid{state + 1, state + 2, gridDim.x, ts.target, fc.spinBudget, 0u};
+            if (!grid.sync()) return;
+            ts.target = grid.target;
+            const bool repair = *(volatile unsigned*)(flag + s % 3) != 0u;
+            if (grid.leader()) flag[(s + 2) % 3] = 0u;   // read before this barrier, written after the next
+            if (repair) {
+                for (int i = tid; i < b.d.nOwned; i += T) {
+                    const int n = bt.localNode[b.d.nodeBase + i];
+                    m.pos[n] = b.P[i];
+                    m.prev[n] = b.Q[i];
+                }
+                const GuardResult g = guardChain(m, fc, fc.firstSubstep + s + 1, state + 1, ts.target);
+                ts.target = g.target;
+                if (!g.ok) return;
+                for (int i = tid; i < b.d.nOwned; i += T) b.P[i] = m.pos[bt.localNode[b.d.nodeBase + i]];
+            }
+        }
         for (int i = tid; i < b.d.nOwned; i += T) {
             float4 P = b.P[i];
             f3 v = mk(0.f, 0.f, 0.f);
             if (P.w > 0.f) {
-                if (fc.contact) {
+                if (fc.contact && !guarded) {
                     const f3 p = contactPoint(xyz(P), P.w, xyz(b.V[i]), b.frames[s % kBrickFrames], cp);
                     P = make_float4(p.x, p.y, p.z, P.w);
                     b.P[i] = P;
@@ -157,13 +219,13 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
                     m.pos[n] = b.P[i];
                     m.prev[n] = b.Q[i];
                 }
-                for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode(m, bt.idle[i], fc, from, to, cp, s, s + 1);
+                for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode<Extended>(m, bt.idle[i], fc, from, to, cp, s, s + 1);
                 ts = ribbonTick(m, cu, bt, b.edgeOff[0], b.edgeOff[b.s.nE], b.tetOff[0], b.tetOff[b.s.nT],
                                 fc.firstSubstep + s + 1 >= fc.numSubsteps, fc.rotations != 0, state + 1, fc.spinBudget, ts);
                 if (!ts.ok) return;
                 mark(kPhaseTick);
             } else {
-                for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode(m, bt.idle[i], fc, from, to, cp, s, s + 1);
+                for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode<Extended>(m, bt.idle[i], fc, from, to, cp, s, s + 1);
             }
             havePrev = true;
         }
@@ -175,9 +237,9 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
         m.vel[n] = b.V[i];
     }
     if (!Cut)
-        for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode(m, bt.idle[i], fc, from, to, cp, 0, fc.substeps);
+        for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode<Extended>(m, bt.idle[i], fc, from, to, cp, 0, fc.substeps);
     if (blockIdx.x == 0 && tid == 0) {
-        if (!Cut) state[1] = (unsigned)exchanges;   // with ticks it is the grid barrier's counter, which others may still read
+        if (!Cut && !guarded) state[1] = (unsigned)exchanges;   // with ticks or the guard it is the grid barrier's counter, which others may still read
         state[3] = (unsigned)ts.rotParity;
     }
 }
@@ -211,15 +273,17 @@ __global__ void brickAlphaKernel(int tets, const int* tetSrc, float invH2, const
 
 }  // namespace
 
-template <bool Damped, bool Cut>
-static __global__ void __launch_bounds__(kBrickThreads, 1) brickFrameKernel(const __grid_constant__ DeviceMesh m, FrameCoeffs fc, ToolPose from,
-                                                                            ToolPose to, ContactParams cp, const __grid_constant__ BrickTables bt,
-                                                                            const __grid_constant__ CutParams cu, unsigned* state) {
-    brickFrame<Damped, Cut>(m, fc, from, to, cp, bt, cu, state);
+template <bool Damped, bool Cut, bool Extended>
+static __global__ void __launch_bounds__(kBrickThreads, 1)
+brickFrameKernel(const __grid_constant__ DeviceMesh m, const __grid_constant__ FrameCoeffs fc, const __grid_constant__ ToolPose from,
+                 const __grid_constant__ ToolPose to, const __grid_constant__ ContactParams cp, const __grid_constant__ BrickTables bt,
+                 const __grid_constant__ CutParams cu, unsigned* state) {
+    brickFrame<Damped, Cut, Extended>(m, fc, from, to, cp, bt, cu, state);
 }
-BrickFrameKernel brickFrameKernelFor(bool damped, bool cut) {
-    return damped ? (cut ? brickFrameKernel<true, true> : brickFrameKernel<true, false>)
-                  : (cut ? brickFrameKernel<false, true> : brickFrameKernel<false, false>);
+BrickFrameKernel brickFrameKernelFor(bool damped, bool cut, bool extended) {
+    if (extended) return damped ? brickFrameKernel<true, false, true> : brickFrameKernel<false, false, true>;
+    return damped ? (cut ? brickFrameKernel<true, true, false> : brickFrameKernel<true, false, false>)
+                  : (cut ? brickFrameKernel<false, true, false> : brickFrameKernel<false, false, false>);
 }
 
 template <class T> cudaError_t BrickBuffers::put(T** to, const T* from, size_t count, cudaStream_t stream) {

@@ -8,7 +8,8 @@ namespace gbt {
 // kernels ([1] and [2] zero; the exchanges run are left in [1] without a cut, the frame parity in [3]).
 using BrickFrameKernel = void (*)(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to, ContactParams cp, BrickTables bt, CutParams cu,
                                   unsigned* state);
-BrickFrameKernel brickFrameKernelFor(bool damped, bool cut);
+// extended: the tissue guard and contact model 1 (no cut).
+BrickFrameKernel brickFrameKernelFor(bool damped, bool cut, bool extended);
 
 // A plan's tables on the device.
 struct BrickBuffers {

@@ -26,9 +26,10 @@ constexpr double kExchange = 1.5, kImportEach = 0.0006;
 struct Phases {
     const BrickMesh& m;
     bool reverse;
+    int nT;                // tet colours of all passes
     int count;
     std::vector<int> at;   // [count x N] element of the phase at the node, or -1
-    Phases(const BrickMesh& mesh, bool rev) : m(mesh), reverse(rev), count(mesh.nEdgeColors + mesh.nTetColors) {
+    Phases(const BrickMesh& mesh, bool rev) : m(mesh), reverse(rev), nT(mesh.nTetColors * (1 + mesh.tensilePasses)), count(mesh.nEdgeColors + nT) {
         at.assign((size_t)count * m.N, -1);
         for (int p = 0; p < count; p++) {
             int* a = at.data() + (size_t)p * m.N;
@@ -39,11 +40,12 @@ struct Phases {
                 else { const int4 t = m.tetIds[k]; a[t.x] = k; a[t.y] = k; a[t.z] = k; a[t.w] = k; }
         }
     }
-    bool isEdge(int p) const { return reverse ? p >= m.nTetColors : p < m.nEdgeColors; }
-    int colour(int p) const {
-        if (!reverse) return p < m.nEdgeColors ? p : p - m.nEdgeColors;
-        return p < m.nTetColors ? m.nTetColors - 1 - p : m.nEdgeColors - 1 - (p - m.nTetColors);
+    bool isEdge(int p) const { return reverse ? p >= nT : p < m.nEdgeColors; }
+    int colour(int p) const {   // of the mesh (a tensile pass repeats the tet colours)
+        if (!reverse) return p < m.nEdgeColors ? p : (p - m.nEdgeColors) % m.nTetColors;
+        return p < nT ? (nT - 1 - p) % m.nTetColors : m.nEdgeColors - 1 - (p - nT);
     }
+    int pass(int p) const { return isEdge(p) ? 0 : (reverse ? nT - 1 - p : p - m.nEdgeColors) / m.nTetColors; }
     void range(int p, int& lo, int& hi) const {
         const int* off = isEdge(p) ? m.edgeOff : m.tetOff;
         lo = off[colour(p)]; hi = off[colour(p) + 1];
@@ -74,11 +76,12 @@ struct Scratch {
 void widen(const Phases& ph, int p, std::vector<int>& need, Scratch& s, std::vector<int>* elements, int& count) {
     const int* at = ph.at.data() + (size_t)p * ph.m.N;
     Marks& seen = ph.isEdge(p) ? s.edge : s.tet;
+    const int mark0 = ph.isEdge(p) ? 0 : ph.pass(p) * ph.m.tetOff[ph.m.nTetColors];   // a tet once per pass
     count = 0;
     const size_t had = need.size();
     for (size_t i = 0; i < had; i++) {
         const int k = at[need[i]];
-        if (k < 0 || !seen.add(k)) continue;
+        if (k < 0 || !seen.add(mark0 + k)) continue;
         count++;
         if (elements) elements->push_back(k);
         int nd[4];
@@ -125,7 +128,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
     BrickPlan none;
     maxLocal = std::min(maxLocal, kBrickMaxLocal);
     const int E = m.nEdgeColors ? m.edgeOff[m.nEdgeColors] : 0, T = m.nTetColors ? m.tetOff[m.nTetColors] : 0;
-    const int P = m.nEdgeColors + m.nTetColors;
+    const int nT = m.nTetColors * (1 + m.tensilePasses), P = m.nEdgeColors + nT;
     if (P == 0 || P > 128 || m.N <= 0) return none;
     // nodes the bricks serve: active ones and ends of any element; the rest never meet a constraint
     std::vector<unsigned char> used(m.N, 0);
@@ -142,7 +145,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
     if (served == 0) return none;
     const int ext[3] = {hi[0] - lo[0] + 1, hi[1] - lo[1] + 1, hi[2] - lo[2] + 1};
     Phases ph(m, reverse);
-    Scratch s(m.N, std::max(E, 1), std::max(T, 1));
+    Scratch s(m.N, std::max(E, 1), std::max(T * (1 + m.tensilePasses), 1));
     auto brickOf = [&](const Split& q, int i) {
         const int x = (i % m.nx - lo[0]) * q.a / ext[0], y = (i / m.nx % m.ny - lo[1]) * q.b / ext[1],
                   z = (i / (m.nx * m.ny) - lo[2]) * q.c / ext[2];
@@ -212,7 +215,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
     };
     // which bricks take values from which (rows: the reader)
     std::vector<unsigned char> reads((size_t)B * B, 0);
-    parallel([&]() { return Scratch(m.N, std::max(E, 1), std::max(T, 1)); }, [&](int b, Scratch& sc) {
+    parallel([&]() { return Scratch(m.N, std::max(E, 1), std::max(T * (1 + m.tensilePasses), 1)); }, [&](int b, Scratch& sc) {
         for (int st = 0; st < S; st++) {
             std::vector<int> need = owned[b];
             sc.node.clear(); sc.edge.clear(); sc.tet.clear();
@@ -262,13 +265,13 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
     }
     if (plan.maxLocal > maxLocal) return none;
     // table offsets, then the tables brick by brick
-    const int headWords = m.nEdgeColors + 1 + m.nTetColors + 1 + 2 * (S + 1);
+    const int headWords = m.nEdgeColors + 1 + nT + 1 + 2 * (S + 1);
     plan.desc.resize(B);
     plan.head.resize((size_t)B * headWords);
     int nNode = 0, nEdge = 0, nTet = 0, nImp = 0, nExp = 0;
     auto phaseOf = [&](bool edge, int colour) {
         if (!reverse) return edge ? colour : m.nEdgeColors + colour;
-        return edge ? m.nTetColors + (m.nEdgeColors - 1 - colour) : m.nTetColors - 1 - colour;
+        return edge ? nT + (m.nEdgeColors - 1 - colour) : nT - 1 - colour;
     };
     for (int b = 0; b < B; b++) {
         int* h = plan.head.data() + (size_t)b * headWords;
@@ -277,7 +280,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         // colours in sweep order
         for (int c = 0; c < m.nEdgeColors; c++) { *h++ = nEdge; nEdge += (int)elements[b][phaseOf(true, reverse ? m.nEdgeColors - 1 - c : c)].size(); }
         *h++ = nEdge;
-        for (int c = 0; c < m.nTetColors; c++) { *h++ = nTet; nTet += (int)elements[b][phaseOf(false, reverse ? m.nTetColors - 1 - c : c)].size(); }
+        for (int c = 0; c < nT; c++) { *h++ = nTet; nTet += (int)elements[b][phaseOf(false, reverse ? nT - 1 - c : c)].size(); }
         *h++ = nTet;
         for (int st = 0; st < S; st++) { *h++ = nImp; nImp += (int)imports[b][st].size(); }
         *h++ = nImp;
@@ -291,7 +294,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         const BrickDesc& d = plan.desc[b];
         const int* h = plan.head.data() + d.head;
         const int* edgeOff = h; const int* tetOff = h + m.nEdgeColors + 1;
-        const int* impOff = tetOff + m.nTetColors + 1; const int* expOff = impOff + S + 1;
+        const int* impOff = tetOff + nT + 1; const int* expOff = impOff + S + 1;
         std::copy(owned[b].begin(), owned[b].end(), plan.localNode.begin() + d.nodeBase);
         std::copy(halo[b].begin(), halo[b].end(), plan.localNode.begin() + d.nodeBase + d.nOwned);
         for (int l = 0; l < d.nLocal; l++) localOf[plan.localNode[d.nodeBase + l]] = l;
@@ -306,9 +309,9 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
                 plan.edgeSrc[at++] = k;
             }
         }
-        for (int c = 0; c < m.nTetColors; c++) {
+        for (int c = 0; c < nT; c++) {
             int at = tetOff[c];
-            for (int k : elements[b][phaseOf(false, reverse ? m.nTetColors - 1 - c : c)]) {
+            for (int k : elements[b][phaseOf(false, reverse ? nT - 1 - c : c)]) {
                 const int4 t = m.tetIds[k];
                 plan.tetWord[at] = (uint64_t)local(t.x) | (uint64_t)local(t.y) << kBrickNodeBits | (uint64_t)local(t.z) << (2 * kBrickNodeBits) |
                                    (uint64_t)local(t.w) << (3 * kBrickNodeBits) | (uint64_t)(m.tetMeta[k] & 7) << 56 | kBrickTetLive |
@@ -329,7 +332,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         plan.maxList = std::max(plan.maxList, records);
     }
     for (auto& lists : elements) for (auto& list : lists) plan.threads = std::max(plan.threads, ((int)list.size() + 31) / 32 * 32);
-    plan.bricks = B; plan.asked = count; plan.stages = S; plan.nEdgeColors = m.nEdgeColors; plan.nTetColors = m.nTetColors; plan.cost = cost;
+    plan.bricks = B; plan.asked = count; plan.stages = S; plan.nEdgeColors = m.nEdgeColors; plan.nTetColors = nT; plan.tensilePasses = m.tensilePasses; plan.cost = cost;
     for (int p = 0; p < P; p++) if (before[p] && B > 1) plan.exchangeBefore[p >> 6] |= 1ull << (p & 63);
     return plan;
 }

@@ -19,6 +19,7 @@ struct BrickDesc {
 // The sweep of one plan: colours, stages, and the phases an exchange precedes (bit p: phase p).
 struct BrickShape {
     int nE, nT, stages, bricks;
+    int nTensile;                   // colours that follow the nT tet colours: the tets once more per tensile pass
     unsigned long long before[2];
 };
 
@@ -36,10 +37,12 @@ struct BrickMesh {   // the coloured mesh a plan is made for; nodes on an nx * n
     int nEdgeColors, nTetColors;
     const int* edgeOff; const int2* edgeEnds; const float* edgeRest;   // colour order
     const int* tetOff; const int4* tetIds; const int* tetMeta;
+    int tensilePasses = 0;                                          // sweeps over the tet colours after the projection's
 };
 
 struct BrickPlan {
     int bricks = 0, stages = 1, nEdgeColors = 0, nTetColors = 0, maxLocal = 0, maxOwned = 0, maxList = 0;
+    int tensilePasses = 0;                 // nTetColors counts the tet colours of every pass
     int asked = 0;                         // the brick count the split was chosen for
     int threads = 32;                      // of a CTA: the widest phase, in whole warps
     uint64_t exchangeBefore[2] = {0, 0};   // bit p: neighbours' values are taken before phase p (edge colours, then tet colours)
@@ -50,7 +53,7 @@ struct BrickPlan {
     std::vector<uint64_t> tetWord; std::vector<int> tetSrc;
     std::vector<unsigned> edgeWord; std::vector<float> edgeRest; std::vector<int> edgeSrc;
     bool ok() const { return bricks > 0; }
-    BrickShape shape() const { return {nEdgeColors, nTetColors, stages, bricks, {exchangeBefore[0], exchangeBefore[1]}}; }
+    BrickShape shape() const { return {nEdgeColors, nTetColors / (1 + tensilePasses), stages, bricks, nTetColors / (1 + tensilePasses) * tensilePasses, {exchangeBefore[0], exchangeBefore[1]}}; }
 };
 
 // The plan of `mesh` on at most `maxBricks` CTAs that keep at most `maxLocal` nodes each; forced > 0

@@ -141,7 +141,7 @@ __device__ __forceinline__ bool cPointBoxTime(const CShape& box, float radius, f
     return false;
 }
 
-__device__ __noinline__ CRecord cTrace(const CShape& from, const CShape& to, float radius, f3 x0, f3 x1) {
+static __device__ __noinline__ CRecord cTrace(const CShape& from, const CShape& to, float radius, f3 x0, f3 x1) {
     CRecord out = {};
     f3 normal = mk(0.f, 0.f, 0.f), surface = mk(0.f, 0.f, 0.f);
     if (!to.capsule && len(to.u - from.u) + len(to.n - from.n) < 1e-7f) {
@@ -204,13 +204,9 @@ __device__ __forceinline__ FrictionShapes frictionShapes(const ToolPose& a, cons
     return f;
 }
 
-// Contact model 1 for one node (k_FindToolContacts x 3 shapes, then k_SolveFrictionContacts x 2).
-__device__ __noinline__ void frictionNode(const DeviceMesh& m, int i, const FrictionShapes& f, float radius, float alpha, float muS,
-                                          float muD) {
-    float4 P = m.pos[i];
-    float w = P.w;
-    if (!(w > 0.f)) return;
-    f3 x = xyz(P), q = xyz(m.prev[i]);
+// Contact model 1 for one mobile node (inverse mass w) at x, substep start q (k_FindToolContacts x 3
+// shapes, then k_SolveFrictionContacts x 2): its new position.
+static __device__ __noinline__ f3 frictionPoint(f3 x, f3 q, float w, const FrictionShapes& f, float radius, float alpha, float muS, float muD) {
     CRecord rec[3];
     for (int kind = 0; kind < 3; kind++) {
         const CShape& to = f.s[3 + kind];
@@ -236,7 +232,13 @@ __device__ __noinline__ void frictionNode(const DeviceMesh& m, int i, const Fric
             x = x + (nextT - oldT) * w;
             lambdaT[kind] = nextT;
         }
-    m.pos[i] = make_float4(x.x, x.y, x.z, w);
+    return x;
+}
+__device__ __forceinline__ void frictionNode(const DeviceMesh& m, int i, const FrictionShapes& f, float radius, float alpha, float muS, float muD) {
+    const float4 P = m.pos[i];
+    if (!(P.w > 0.f)) return;
+    const f3 x = frictionPoint(xyz(P), xyz(m.prev[i]), P.w, f, radius, alpha, muS, muD);
+    m.pos[i] = make_float4(x.x, x.y, x.z, P.w);
 }
 
 }  // namespace gbt

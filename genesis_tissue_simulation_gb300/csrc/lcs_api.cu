@@ -122,7 +122,8 @@ struct Session {
     // topology may have changed since the live bits were derived
     BrickBuffers bricks; std::vector<int> brickIdle; unsigned long long planId = 0;
     std::vector<int2> hostEdgeEnds; std::vector<float> hostEdgeRest; std::vector<int4> hostTetIds; std::vector<int> hostTetMeta, hostActive;
-    bool bricksStale = true, bricksDamped = false; int forcedBricks = 0, maxBrickBytes = 0;
+    bool bricksStale = true, bricksDamped = false; int forcedBricks = 0, maxBrickBytes = 0, maxGuardBytes = 0;
+    BrickBuffers guardBricks;   // with the tensile pass's phases (one pass), made when the guard is armed
     // section profiler (xpbd_profile_sections, xpbd_solver.cu:30-60): device time per phase kind
     bool sections = false; DBuf<unsigned long long> phaseClock; std::vector<unsigned long long> phaseHost;
     double sectionMs[8] = {}; long long sectionCount[8] = {};
@@ -157,7 +158,7 @@ void freePhysics() {
     S.edgeEnds.release(); S.edgeRest.release(); S.bendIJK.release(); S.bendPairs.release(); S.tetIds.release();
     S.tetAlpha.release(); S.tetStiff.release(); S.state.release(); S.bounds.release(); S.floorSync.release();
     S.uncovered0.release(); S.fuseEdge0 = false;
-    S.bricks.release(); S.bricksStale = true;
+    S.bricks.release(); S.guardBricks.release(); S.bricksStale = true;
     S.lastFrameBlocks = 0;
     S.fiberLambda.release(); S.feasTarget.release(); S.needed.release(); S.incOff.release(); S.incTet.release(); S.guardFlags.release();
     S.rotA.release(); S.rotB.release(); S.rotParity = 0;
@@ -196,9 +197,16 @@ int ensureStream() {
     CK(cudaFuncGetAttributes(&ca, (const void*)frameKernelSessionCluster));
     S.maxClusterBytes = optin - (int)ca.sharedSizeBytes;   // dynamic bytes left beside its static shared memory
     CK(cudaFuncSetAttribute((const void*)frameKernelSessionCluster, cudaFuncAttributeMaxDynamicSharedMemorySize, S.maxClusterBytes));
-    for (int k = 0; k < 4; k++)
-        CK(cudaFuncSetAttribute((const void*)brickFrameKernelFor(k & 1, k >> 1), cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
-    S.maxBrickBytes = optin - 1024;
+    S.maxBrickBytes = S.maxGuardBytes = optin - 1024;
+    for (int k = 0; k < 6; k++) {
+        const void* kernel = (const void*)brickFrameKernelFor(k & 1, k == 2 || k == 3, k >= 4);
+        cudaFuncAttributes fa{};
+        CK(cudaFuncGetAttributes(&fa, kernel));
+        const int room = optin - (int)fa.sharedSizeBytes;
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+        int& least = k >= 4 ? S.maxGuardBytes : S.maxBrickBytes;
+        least = std::min(least, room);
+    }
     int khz = 0;
     if (cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, S.device) == cudaSuccess && khz > 0) S.clockKHz = khz;
     S.gridBlocks = std::max(1, perSm) * S.smCount;
@@ -348,30 +356,38 @@ CutParams cutParams() {
 // (*followUp set), so the host flips the parity the kernel leaves in state[3].
 // Launch shapes of a frame: one CTA, the whole GPU, one thread-block cluster.
 constexpr int kShapeBlock = 0, kShapeGrid = 1, kShapeCluster = 2;
-// Automatic mode runs plain and blade frames (no bends, perpendicular damping, guard or friction; a
-// blade not with the tet-support fallback, whose edge flags cross bricks) on bricks wherever a plan fits.
-bool brickFrames(const FrameCoeffs& fc) {
-    return S.launchMode == 0 && S.bricks.ready() && !fc.doBend && !fc.perpDamp && !fc.guarded && !fc.friction && !(fc.cut && fc.fallback);
+// Automatic mode runs frames without bends or perpendicular damping on bricks wherever a plan fits: plain
+// ones, blade frames (not with the tet-support fallback, whose edge flags cross bricks), friction, and
+// the tissue guard with one tensile pass (its own plan).  Null: another shape.
+BrickBuffers* brickFrames(const FrameCoeffs& fc) {
+    if (S.launchMode != 0 || fc.doBend || fc.perpDamp) return nullptr;
+    if (fc.cut && (fc.fallback || fc.guarded || fc.friction)) return nullptr;
+    BrickBuffers* b = fc.guarded ? &S.guardBricks : &S.bricks;
+    if (!b->ready() || (fc.friction && !fc.guarded && b->sharedBytes(S.bricksDamped) > (size_t)S.maxGuardBytes)) return nullptr;
+    return b;
 }
-int launchBricks(const FrameCoeffs& fc, bool* followUp) {
+int launchBricks(BrickBuffers& bricks, const FrameCoeffs& fc, bool* followUp) {
     DeviceMesh m = deviceMesh();
     if (S.bricksStale) {
         CK(refreshMeshFlags(m, S.E, S.T, fc.fallback != 0, S.stream));
-        CK(S.bricks.refresh(m, fc.fallback != 0, S.stream));
+        for (BrickBuffers* b : {&S.bricks, &S.guardBricks}) if (b->ready()) CK(b->refresh(m, fc.fallback != 0, S.stream));
         S.bricksStale = false;
     }
+    const bool extended = fc.guarded || fc.friction, damped = fc.guarded || S.bricksDamped;
     FrameCoeffs f = fc;
     ToolPose from = S.toolFrom, to = S.tool;
     ContactParams cp = S.cp;
     unsigned* state = S.state.p;
     CutParams cu = cutParams();
     if (fc.cut && S.brickCount.p) CK(cudaMemsetAsync(S.brickCount.p, 0, sizeof(unsigned), S.stream));
-    void* args[] = {&m, &f, &from, &to, &cp, &S.bricks.t, &cu, &state};
-    CK(cudaLaunchCooperativeKernel((const void*)brickFrameKernelFor(S.bricksDamped, fc.cut != 0), dim3(S.bricks.t.bricks), dim3(S.bricks.threads),
-                                   args, S.bricks.sharedBytes(S.bricksDamped), S.stream));
+    if (fc.guarded) CK(cudaMemsetAsync(S.guardFlags.p, 0, 5 * sizeof(unsigned), S.stream));
+    void* args[] = {&m, &f, &from, &to, &cp, &bricks.t, &cu, &state};
+    CK(cudaLaunchCooperativeKernel((const void*)brickFrameKernelFor(damped, fc.cut != 0, extended), dim3(bricks.t.bricks), dim3(bricks.threads),
+                                   args, bricks.sharedBytes(damped), S.stream));
     particleRotKernel<<<(S.N + 255) / 256, 256, 0, S.stream>>>(m, fc.cut ? state + 3 : nullptr, fc.rotParity);
     CK(cudaGetLastError());
-    S.lastFrameBlocks = fc.cut ? S.bricks.t.bricks : 1;   // without a cut the kernel leaves its exchanges in the barrier counter
+    // without ticks or the guard the kernel leaves its exchanges in the barrier counter
+    S.lastFrameBlocks = fc.cut || fc.guarded ? bricks.t.bricks : 1;
     *followUp = true;
     return 0;
 }
@@ -496,7 +512,7 @@ FrameCoeffs frameCoeffs(float h, int N) {
 int launchFrame(const FrameCoeffs& fc, bool* followUp) {
     unsigned* state = S.state.p;
     CK(cudaMemsetAsync(state + 1, 0, 2 * sizeof(unsigned), S.stream));
-    if (brickFrames(fc)) return launchBricks(fc, followUp);
+    if (BrickBuffers* bricks = brickFrames(fc)) return launchBricks(*bricks, fc, followUp);
     if (S.brickCount.p) CK(cudaMemsetAsync(S.brickCount.p, 0, sizeof(unsigned), S.stream));
     const Shapes u = usableShapes(fc);
     int shape = requestedShape(u);
@@ -537,7 +553,22 @@ int launchFrame(const FrameCoeffs& fc, bool* followUp) {
 // memory.  A mesh without a plan keeps the other shapes.
 BrickMesh brickMesh() {
     return {S.N, S.dx + 1, S.dy + 1, S.dz + 1, S.hostActive.data(), (int)S.edgeColorOff.size() - 1, (int)S.tetColorOff.size() - 1,
-            S.edgeColorOff.data(), S.hostEdgeEnds.data(), S.hostEdgeRest.data(), S.tetColorOff.data(), S.hostTetIds.data(), S.hostTetMeta.data()};
+            S.edgeColorOff.data(), S.hostEdgeEnds.data(), S.hostEdgeRest.data(), S.tetColorOff.data(), S.hostTetIds.data(), S.hostTetMeta.data(), 0};
+}
+// A plan of `mesh` in CTAs of at most maxBytes shared memory; a mesh without one leaves `bricks` empty.
+int planInto(BrickBuffers& bricks, const BrickMesh& mesh, bool damped, int maxBytes, std::vector<int>* idle) {
+    bricks.release();
+    // at most four records of 16 B a node, beside the offsets and instrument frames
+    const int perNode = (damped ? 2 : 1) * 16, room = maxBytes - 8192;
+    for (int share = 70; share >= 40; share -= 10) {
+        const BrickPlan plan = buildBrickPlan(mesh, S.smCount, (int)((long long)room * share / 100) / perNode, S.forcedBricks, damped);
+        if (!plan.ok()) return 0;
+        if (idle) *idle = plan.idle;
+        CK(bricks.upload(plan, S.N, damped, maxBytes, S.stream));
+        if (bricks.sharedBytes(damped) <= (size_t)maxBytes) return 0;
+        bricks.release();
+    }
+    return 0;
 }
 int planBricks(HostMesh& hm, const int* active) {
     S.bricks.release();
@@ -547,18 +578,7 @@ int planBricks(HostMesh& hm, const int* active) {
     S.bricksDamped = S.strainDamping > 0.f;   // without perpendicular damping (betaS = 0) only the tets are damped
     S.hostEdgeEnds.swap(hm.edgeEnds); S.hostEdgeRest.swap(hm.edgeRest); S.hostTetIds.swap(hm.tetIds); S.hostTetMeta.swap(hm.tetMeta);
     S.hostActive.assign(active, active + S.N);
-    const BrickMesh bm = brickMesh();
-    // shared memory: at most four records of 16 B a node, beside the offsets and instrument frames
-    const int perNode = (S.bricksDamped ? 2 : 1) * 16, rest = 8192;
-    for (int room = S.maxBrickBytes - rest, share = 70; share >= 40; share -= 10) {
-        const BrickPlan plan = buildBrickPlan(bm, S.smCount, (int)((long long)room * share / 100) / perNode, S.forcedBricks, S.bricksDamped);
-        if (!plan.ok()) return 0;
-        S.brickIdle = plan.idle;
-        CK(S.bricks.upload(plan, S.N, S.bricksDamped, S.maxBrickBytes, S.stream));
-        if (S.bricks.sharedBytes(S.bricksDamped) <= (size_t)S.maxBrickBytes) return 0;
-        S.bricks.release();
-    }
-    return 0;
+    return planInto(S.bricks, brickMesh(), S.bricksDamped, S.maxBrickBytes, &S.brickIdle);
 }
 
 }  // namespace
@@ -787,12 +807,18 @@ LCS_API int LCS_SetTissueGuard(float minimum, int passes, int count, const int* 
     CK(S.fiberLambda.alloc((size_t)6 * std::max(S.T, 1)));
     CK(S.feasTarget.alloc(S.N));
     CK(S.needed.alloc(S.N));
-    CK(S.guardFlags.alloc(2));
+    CK(S.guardFlags.alloc(5));
     CK(cudaMemsetAsync(S.needed.p, 0, S.N * sizeof(int), S.stream));
-    CK(cudaMemsetAsync(S.guardFlags.p, 0, 2 * sizeof(unsigned), S.stream));
+    CK(cudaMemsetAsync(S.guardFlags.p, 0, 5 * sizeof(unsigned), S.stream));
     CK(cudaStreamSynchronize(S.stream));
     S.volumePasses = passes;
     S.minVolume = minimum;
+    S.guardBricks.release();
+    if (passes == 1 && S.T > 0) {   // more passes carry multipliers from one to the next
+        BrickMesh bm = brickMesh();
+        bm.tensilePasses = 1;
+        return planInto(S.guardBricks, bm, true, S.maxGuardBytes, nullptr);
+    }
     return 0;
 }
 LCS_API int LCS_SetTissueMaterial(float strength, float bulkDamping) {
@@ -929,7 +955,7 @@ LCS_API int LCS_Step(float dt) {
     if (fc.doStrain && h != S.lastH) {
         tetAlphaKernel<<<(S.T + 255) / 256, 256, 0, S.stream>>>(S.T, fc.invH2, S.tetStiff.p, S.tetAlpha.p);
         CK(cudaGetLastError());
-        if (S.bricks.ready()) CK(S.bricks.compliances(fc.invH2, S.tetStiff.p, S.stream));
+        for (BrickBuffers* b : {&S.bricks, &S.guardBricks}) if (b->ready()) CK(b->compliances(fc.invH2, S.tetStiff.p, S.stream));
         S.lastH = h;
     }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -944,7 +970,7 @@ LCS_API int LCS_Step(float dt) {
         fc.phaseClock = S.phaseClock.p;
     }
     bool followUp = false;
-    const bool onBricks = brickFrames(fc);
+    const bool onBricks = brickFrames(fc) != nullptr;
     int rc = launchFrame(fc, &followUp);
     if (rc) return rc;
     if (S.profile) { CK(cudaEventRecord(e1, S.stream)); S.events.push_back(e0); S.events.push_back(e1); }

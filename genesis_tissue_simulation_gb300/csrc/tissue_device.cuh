@@ -614,18 +614,9 @@ __device__ __forceinline__ void typeRows(const DeviceMesh& m, int type, f3 b[3])
 // corner-to-corner fibres carries mu V strength / 2 s^6, s = max(length / rest - 1, 0), projected
 // with finite compliance alphaDev / strength; the rest corners are the columns of (Dm^-1)^-1.
 // `pass` > 0 continues the fibres' multipliers of this substep.
-__device__ __forceinline__ void projectTensile(const DeviceMesh& m, int k, const FrameCoeffs& fc, int pass) {
-    int meta = m.tetMeta[k];
-    if ((meta & 8) == 0 || !(fc.tensileStrength > 0.f)) return;
-    int4 ids = m.tetIds[k];
-    int id[4] = {ids.x, ids.y, ids.z, ids.w};
-    float4 P[4] = {m.pos[id[0]], m.pos[id[1]], m.pos[id[2]], m.pos[id[3]]};
-    f3 p[4] = {xyz(P[0]), xyz(P[1]), xyz(P[2]), xyz(P[3])};
-    f3 b[3];
-    typeRows(m, meta & 7, b);
+__device__ __forceinline__ void solveTensile(const f3 (&b)[3], const float4 (&P)[4], float alpha, float (&lambda)[6], f3 (&p)[4]) {
     float detB = dot(b[0], cross(b[1], b[2]));
     f3 rest[4] = {mk(0.f, 0.f, 0.f), cross(b[1], b[2]) * (1.f / detB), cross(b[2], b[0]) * (1.f / detB), cross(b[0], b[1]) * (1.f / detB)};
-    float alpha = m.tetAlpha[k].x / fmaxf(fc.tensileStrength, 1e-10f);
     int fiber = 0;
 #pragma unroll
     for (int i = 0; i < 4; i++)
@@ -635,16 +626,31 @@ __device__ __forceinline__ void projectTensile(const DeviceMesh& m, int k, const
             float length = len(edge), restLength = len(rest[j] - rest[i]);
             float strain = fmaxf(length / restLength - 1.f, 0.f), gradient = 3.f * strain * strain / restLength;
             float wi = P[i].w, wj = P[j].w;
-            float lambda = pass == 0 ? 0.f : m.fiberLambda[6 * (size_t)k + fiber];
             if (strain > 0.f && length > 0.f) {
-                float dl = (-strain * strain * strain - alpha * lambda) / ((wi + wj) * gradient * gradient + alpha);
+                float dl = (-strain * strain * strain - alpha * lambda[fiber]) / ((wi + wj) * gradient * gradient + alpha);
                 f3 g = edge * (gradient / length);
-                lambda += dl;
+                lambda[fiber] += dl;
                 p[i] = p[i] - g * (wi * dl);
                 p[j] = p[j] + g * (wj * dl);
             }
-            if (fc.volumePasses > 1) m.fiberLambda[6 * (size_t)k + fiber] = lambda;
         }
+}
+__device__ __forceinline__ void projectTensile(const DeviceMesh& m, int k, const FrameCoeffs& fc, int pass) {
+    int meta = m.tetMeta[k];
+    if ((meta & 8) == 0 || !(fc.tensileStrength > 0.f)) return;
+    int4 ids = m.tetIds[k];
+    int id[4] = {ids.x, ids.y, ids.z, ids.w};
+    const float4 P[4] = {m.pos[id[0]], m.pos[id[1]], m.pos[id[2]], m.pos[id[3]]};
+    f3 p[4] = {xyz(P[0]), xyz(P[1]), xyz(P[2]), xyz(P[3])};
+    f3 b[3];
+    typeRows(m, meta & 7, b);
+    float lambda[6];
+#pragma unroll
+    for (int f = 0; f < 6; f++) lambda[f] = pass == 0 ? 0.f : m.fiberLambda[6 * (size_t)k + f];
+    solveTensile(b, P, m.tetAlpha[k].x / fmaxf(fc.tensileStrength, 1e-10f), lambda, p);
+    if (fc.volumePasses > 1)
+#pragma unroll
+        for (int f = 0; f < 6; f++) m.fiberLambda[6 * (size_t)k + f] = lambda[f];
 #pragma unroll
     for (int c = 0; c < 4; c++) m.pos[id[c]] = make_float4(p[c].x, p[c].y, p[c].z, P[c].w);
 }

@@ -139,3 +139,33 @@ def test_rollouts_on_bricks_match_the_whole_gpu_rollout(gpu_lib, size, damping, 
         assert np.isfinite(a).all()
         # path: 12 substeps' sums in another order; the rest differs at most by zeros that were added
         assert np.abs(a - b).max() <= (1e-5 if name == "path" else 1e-6) * max(np.abs(b).max(), 1e-30), name
+
+
+@pytest.mark.parametrize("bricks", [1, 5, 152])
+@pytest.mark.parametrize("minimum", [0.15, 0.9])
+def test_guarded_frames_on_bricks_match_the_whole_gpu_frame(gpu_lib, bricks, minimum):
+    """The guard's tet form, its tensile pass and its feasibility chain (which 0.9 sets off)."""
+    from test_guard import guarded_run
+    dll = ct.CDLL(str(gpu_lib))
+    assert dll.GBT_SetBrickCount(bricks) == 0
+    try:
+        _, got, _ = guarded_run(gpu_lib, steps=6, minimum=minimum, launch_mode=0)
+    finally:
+        dll.GBT_SetBrickCount(0)
+    _, want, _ = guarded_run(gpu_lib, steps=6, minimum=minimum, launch_mode=1)
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("bricks", [1, 5, 152])
+def test_friction_frames_on_bricks_match_the_whole_gpu_frame(gpu_lib, bricks):
+    from test_friction_contact import friction_run
+    dll = ct.CDLL(str(gpu_lib))
+    assert dll.GBT_SetBrickCount(bricks) == 0
+    try:
+        _, got = friction_run(gpu_lib, steps=6, closing=True, launch_mode=0)
+    finally:
+        dll.GBT_SetBrickCount(0)
+    _, want = friction_run(gpu_lib, steps=6, closing=True, launch_mode=1)
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
