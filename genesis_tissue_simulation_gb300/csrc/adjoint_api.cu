@@ -112,7 +112,7 @@ int planReverse(const SessionView& v) {
     BrickTables f = t, r = D.reverse.t;
     if (!backwardBytes(f, r, damped(v), v.maxBrickBytes)) { D.reverse.release(); return 0; }
     CK(D.brickAlpha.ensure(v.bricks->tets));
-    for (const void* k : {(const void*)brickForward, (const void*)brickForwardDamped, (const void*)brickBackward, (const void*)brickBackwardDamped})
+    for (const void* k : {(const void*)brickForwardFor(damped(v), v.bricks->threads), (const void*)brickBackward, (const void*)brickBackwardDamped})
         CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, v.maxBrickBytes));
     D.planId = v.planId;
     D.bricks = true;
@@ -153,7 +153,7 @@ int launchBricks(const SessionView& v, bool backward, DeviceMesh m, DiffBuffers 
         own.t.tetAlpha = D.brickAlpha.p;
         CK(prepareRollout(m, b, D.E, D.T, dc.invH2, own, D.reverse, v.stream));
         void* args[] = {&m, &dc, &cp, &b, &f, &barrier, &budget};
-        CK(cudaLaunchCooperativeKernel(d ? (const void*)brickForwardDamped : (const void*)brickForward, dim3(f.bricks), dim3(v.bricks->threads),
+        CK(cudaLaunchCooperativeKernel((const void*)brickForwardFor(d, v.bricks->threads), dim3(f.bricks), dim3(v.bricks->threads),
                                        args, Brick::bytes(f, d), v.stream));
     }
     CK(cudaGetLastError());

@@ -20,6 +20,11 @@
 namespace gbt {
 
 constexpr int kBrickThreads = 512;
+// Plans whose widest colour has at most kNarrowColour elements run in CTAs of kNarrowThreads: twice the
+// registers a thread and fewer warps at each barrier pay for the few second rounds (us a substep, 512 ->
+// 256: 23 x 13 x 19 cells, 320 wide, 34.0 -> 32.8; 32 x 16 x 32 cells, 320 wide, 39.0 -> 38.5; 64 x 32 x 48
+// cells, 896 wide, 62.1 -> 69.2).
+constexpr int kNarrowThreads = 256, kNarrowColour = 320;
 constexpr int kBrickFrames = 32;   // instrument frames held in shared memory at a time
 
 struct BrickTables {
@@ -72,15 +77,22 @@ __device__ __forceinline__ bool take(const float4* from, const int2 (&e)[kTake],
 }
 // Publishes the listed values and takes the neighbours'.  A function of values, out of line: the sweep
 // around it keeps its registers, and P and Q stay shared-memory addresses there.
+// A record can not be there sooner than about kFlight cycles after neighbours in step began to publish,
+// and polls before that only hold the stores up.  64 x 32 x 48 cells: 64.1 us a substep polling at once,
+// 62.1 after 800 cycles, 60.4 after 1200; 32 x 16 x 32 cells: 41.3, 39.0 and 38.3; 16 x 8 x 16 cells: 34.2,
+// 33.5 and 33.0; 23 x 13 x 19 cells: 34.9, 34.0 and 34.6.
+constexpr int kFlight = 1100;
 static __device__ __noinline__ bool exchangeRecords(float4* box, float4* boxStart, float4* P, float4* Q, const int2* exports, int nExports,
                                                     const int2* imports, int nImports, unsigned epoch, unsigned lag, unsigned* status,
                                                     long long budget) {
     const int T = blockDim.x, tid = threadIdx.x;
+    const long long start = clock64();
     for (int i = tid; i < nExports; i += T) {
         const int2 e = exports[i];
         publish(box + e.y, xyz(P[e.x]), epoch);
         if (boxStart) publish(boxStart + e.y, xyz(Q[e.x]), epoch);
     }
+    while (clock64() - start < kFlight) {}
     bool bad = false;
     for (int i = tid; i < nImports; i += kTake * T) {
         int2 e[kTake];

@@ -273,17 +273,20 @@ __global__ void brickAlphaKernel(int tets, const int* tetSrc, float invH2, const
 
 }  // namespace
 
-template <bool Damped, bool Cut, bool Extended>
-static __global__ void __launch_bounds__(kBrickThreads, 1)
+template <bool Damped, bool Cut, bool Extended, int Threads>
+static __global__ void __launch_bounds__(Threads, 1)
 brickFrameKernel(const __grid_constant__ DeviceMesh m, const __grid_constant__ FrameCoeffs fc, const __grid_constant__ ToolPose from,
                  const __grid_constant__ ToolPose to, const __grid_constant__ ContactParams cp, const __grid_constant__ BrickTables bt,
                  const __grid_constant__ CutParams cu, unsigned* state) {
     brickFrame<Damped, Cut, Extended>(m, fc, from, to, cp, bt, cu, state);
 }
-BrickFrameKernel brickFrameKernelFor(bool damped, bool cut, bool extended) {
-    if (extended) return damped ? brickFrameKernel<true, false, true> : brickFrameKernel<false, false, true>;
-    return damped ? (cut ? brickFrameKernel<true, true, false> : brickFrameKernel<true, false, false>)
-                  : (cut ? brickFrameKernel<false, true, false> : brickFrameKernel<false, false, false>);
+template <int Threads> static BrickFrameKernel frameKernelFor(bool damped, bool cut, bool extended) {
+    if (extended) return damped ? brickFrameKernel<true, false, true, Threads> : brickFrameKernel<false, false, true, Threads>;
+    return damped ? (cut ? brickFrameKernel<true, true, false, Threads> : brickFrameKernel<true, false, false, Threads>)
+                  : (cut ? brickFrameKernel<false, true, false, Threads> : brickFrameKernel<false, false, false, Threads>);
+}
+BrickFrameKernel brickFrameKernelFor(bool damped, bool cut, bool extended, int threads) {
+    return threads <= kNarrowThreads ? frameKernelFor<kNarrowThreads>(damped, cut, extended) : frameKernelFor<kBrickThreads>(damped, cut, extended);
 }
 
 template <class T> cudaError_t BrickBuffers::put(T** to, const T* from, size_t count, cudaStream_t stream) {
@@ -307,7 +310,8 @@ cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int 
     release();
     tets = (int)plan.tetWord.size(); edges = (int)plan.edgeWord.size();
     asked = plan.asked;
-    threads = plan.threads < kBrickThreads ? plan.threads : kBrickThreads;
+    threads = plan.threads <= kNarrowColour ? (plan.threads < kNarrowThreads ? plan.threads : kNarrowThreads)
+                                            : (plan.threads < kBrickThreads ? plan.threads : kBrickThreads);
     BrickTables q{};
     q.shape = plan.shape();
     q.maxLocal = plan.maxLocal; q.maxOwned = plan.maxOwned; q.nIdle = (int)plan.idle.size(); q.N = N;

@@ -9,7 +9,7 @@ namespace gbt {
 using BrickFrameKernel = void (*)(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to, ContactParams cp, BrickTables bt, CutParams cu,
                                   unsigned* state);
 // extended: the tissue guard and contact model 1 (no cut).
-BrickFrameKernel brickFrameKernelFor(bool damped, bool cut, bool extended);
+BrickFrameKernel brickFrameKernelFor(bool damped, bool cut, bool extended, int threads);
 
 // A plan's tables on the device.
 struct BrickBuffers {

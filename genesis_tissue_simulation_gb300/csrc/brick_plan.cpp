@@ -23,6 +23,9 @@ namespace {
 constexpr double kEdgePhase = 0.25, kEdgeEach = 0.0007, kTetPhase = 0.55, kTetEach = 0.0019;
 constexpr double kExchange = 1.5, kImportEach = 0.0006;
 
+// The reverse projection of a tet costs about three times the forward one.
+constexpr double kReverseTetPhase = 1.6, kReverseTetEach = 0.0065;
+
 struct Phases {
     const BrickMesh& m;
     bool reverse;
@@ -107,7 +110,8 @@ double chooseStages(const Phases& ph, const std::vector<int>& owned, Scratch& s,
         for (int p = end - 1; p >= std::max(0, end - kLongest); p--) {
             int count;
             widen(ph, p, need, s, nullptr, count);
-            work += ph.isEdge(p) ? kEdgePhase + kEdgeEach * count : kTetPhase + kTetEach * count;
+            work += ph.isEdge(p) ? kEdgePhase + kEdgeEach * count
+                    : ph.reverse ? kReverseTetPhase + kReverseTetEach * count : kTetPhase + kTetEach * count;
             if ((int)need.size() > maxLocal && p < end - 1) break;
             const double c = best[p] + work + kExchange + kImportEach * (double)(need.size() - owned.size());
             if (c < best[end]) { best[end] = c; from[end] = p; }

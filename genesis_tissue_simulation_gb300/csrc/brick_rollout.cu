@@ -275,13 +275,14 @@ __global__ void gatherCompliances(int n, const int* src, const float2* from, flo
 
 }  // namespace
 
-__global__ void __launch_bounds__(kBrickThreads, 1) brickForward(DeviceMesh m, DiffCoeffs dc, ContactParams cp, DiffBuffers b, BrickTables bt,
-                                                                 unsigned* barrier, long long budget) {
-    forwardBricks<false>(m, dc, cp, b, bt, barrier, budget);
+template <bool Damped, int Threads>
+static __global__ void __launch_bounds__(Threads, 1) brickForward(DeviceMesh m, DiffCoeffs dc, ContactParams cp, DiffBuffers b, BrickTables bt,
+                                                                  unsigned* barrier, long long budget) {
+    forwardBricks<Damped>(m, dc, cp, b, bt, barrier, budget);
 }
-__global__ void __launch_bounds__(kBrickThreads, 1) brickForwardDamped(DeviceMesh m, DiffCoeffs dc, ContactParams cp, DiffBuffers b,
-                                                                       BrickTables bt, unsigned* barrier, long long budget) {
-    forwardBricks<true>(m, dc, cp, b, bt, barrier, budget);
+BrickForwardKernel brickForwardFor(bool damped, int threads) {
+    return threads <= kNarrowThreads ? (damped ? brickForward<true, kNarrowThreads> : brickForward<false, kNarrowThreads>)
+                                     : (damped ? brickForward<true, kBrickThreads> : brickForward<false, kBrickThreads>);
 }
 __global__ void __launch_bounds__(kReverseThreads, 1) brickBackward(DeviceMesh m, DiffCoeffs dc, ContactParams cp, DiffBuffers b, BrickTables bt,
                                                                     BrickTables rt, unsigned* barrier, long long budget) {

@@ -8,9 +8,9 @@ namespace gbt {
 // The reverse projection holds about 250 registers a thread.
 constexpr int kReverseThreads = 256;
 
-__global__ void brickForward(DeviceMesh m, DiffCoeffs dc, ContactParams cp, DiffBuffers b, BrickTables bt, unsigned* barrier, long long budget);
-__global__ void brickForwardDamped(DeviceMesh m, DiffCoeffs dc, ContactParams cp, DiffBuffers b, BrickTables bt, unsigned* barrier,
-                                   long long budget);
+using BrickForwardKernel = void (*)(DeviceMesh m, DiffCoeffs dc, ContactParams cp, DiffBuffers b, BrickTables bt, unsigned* barrier,
+                                    long long budget);
+BrickForwardKernel brickForwardFor(bool damped, int threads);
 __global__ void brickBackward(DeviceMesh m, DiffCoeffs dc, ContactParams cp, DiffBuffers b, BrickTables bt, BrickTables rt, unsigned* barrier,
                               long long budget);
 __global__ void brickBackwardDamped(DeviceMesh m, DiffCoeffs dc, ContactParams cp, DiffBuffers b, BrickTables bt, BrickTables rt,

@@ -198,8 +198,9 @@ int ensureStream() {
     S.maxClusterBytes = optin - (int)ca.sharedSizeBytes;   // dynamic bytes left beside its static shared memory
     CK(cudaFuncSetAttribute((const void*)frameKernelSessionCluster, cudaFuncAttributeMaxDynamicSharedMemorySize, S.maxClusterBytes));
     S.maxBrickBytes = S.maxGuardBytes = optin - 1024;
-    for (int k = 0; k < 6; k++) {
-        const void* kernel = (const void*)brickFrameKernelFor(k & 1, k == 2 || k == 3, k >= 4);
+    for (int q = 0; q < 12; q++) {
+        const int k = q % 6;
+        const void* kernel = (const void*)brickFrameKernelFor(k & 1, k == 2 || k == 3, k >= 4, q < 6 ? kBrickThreads : kNarrowThreads);
         cudaFuncAttributes fa{};
         CK(cudaFuncGetAttributes(&fa, kernel));
         const int room = optin - (int)fa.sharedSizeBytes;
@@ -382,7 +383,7 @@ int launchBricks(BrickBuffers& bricks, const FrameCoeffs& fc, bool* followUp) {
     if (fc.cut && S.brickCount.p) CK(cudaMemsetAsync(S.brickCount.p, 0, sizeof(unsigned), S.stream));
     if (fc.guarded) CK(cudaMemsetAsync(S.guardFlags.p, 0, 5 * sizeof(unsigned), S.stream));
     void* args[] = {&m, &f, &from, &to, &cp, &bricks.t, &cu, &state};
-    CK(cudaLaunchCooperativeKernel((const void*)brickFrameKernelFor(damped, fc.cut != 0, extended), dim3(bricks.t.bricks), dim3(bricks.threads),
+    CK(cudaLaunchCooperativeKernel((const void*)brickFrameKernelFor(damped, fc.cut != 0, extended, bricks.threads), dim3(bricks.t.bricks), dim3(bricks.threads),
                                    args, bricks.sharedBytes(damped), S.stream));
     particleRotKernel<<<(S.N + 255) / 256, 256, 0, S.stream>>>(m, fc.cut ? state + 3 : nullptr, fc.rotParity);
     CK(cudaGetLastError());
