@@ -259,7 +259,7 @@ int launchFrame(const FrameCoeffs& fc, const ContactFrame* frames) {
         attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
         ContactParams cp = G.cp;
-        CK(cudaLaunchKernelEx(&cfg, brickBatchKernel(G.strainDamping > 0.f, G.codesAvailable), m, fc, cp, G.bricks.buffers.t,
+        CK(cudaLaunchKernelEx(&cfg, G.bricks.kernel(G.strainDamping > 0.f, G.codesAvailable), m, fc, cp, G.bricks.buffers.t,
                               (const BrickShape*)G.bricks.shapes, (const int*)G.bricks.order, (const int*)G.bricks.start,
                               G.codesAvailable ? (const float2*)G.instAlpha.p : (const float2*)nullptr, G.state.p + 2));
     } else if (G.mode == 0) {
@@ -391,13 +391,9 @@ int stepFrames(float dt, int steps, const ToolPose* tools, bool useGraph) {
 // derive at their first frame (links and nodes present; with the tet-support fallback, edges no live
 // tet carries) is settled here.
 int planBricks(const std::vector<HostMesh>& meshes, const GbtInstanceDesc* inst, const std::vector<int2>& iEdge, const std::vector<int2>& iTet) {
-    int optin = 0, perSm = 0, reserved = 0;
+    int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, G.device));
-    CK(cudaDeviceGetAttribute(&perSm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, G.device));
-    CK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, G.device));
-    const int fixed = 1024;   // the kernel's static shared memory, rounded up
-    const int one = optin - fixed, two = std::min(one, perSm / 2 - reserved - fixed);
-    CK(cudaFuncSetAttribute((const void*)brickBatchKernel(G.strainDamping > 0.f, G.codesAvailable), cudaFuncAttributeMaxDynamicSharedMemorySize, one));
+    const int one = optin - 1024;   // beside the kernel's static shared memory
     const int count = G.count;
     const bool fallback = G.T > 0 && G.youngE > 0.f && G.ks <= 0.f;
     std::vector<std::vector<int>> edgeSlot(count), tetSlot(count);
@@ -428,7 +424,9 @@ int planBricks(const std::vector<HostMesh>& meshes, const GbtInstanceDesc* inst,
                   hm.tetColorOff.data(), hm.tetIds.data(), hm.tetMeta.data(), 0},
                  G.nodeBase[i], edgeSlot[i].data(), tetSlot[i].data(), edgeDead[i].data(), tetDead[i].data()};
     }
-    CK(G.bricks.plan(in, G.N, G.smCount, one, two, G.strainDamping > 0.f, G.stream));
+    CK(G.bricks.plan(in, G.N, G.smCount, one, G.strainDamping > 0.f, G.stream));
+    if (G.bricks.ready())
+        CK(cudaFuncSetAttribute((const void*)G.bricks.kernel(G.strainDamping > 0.f, G.codesAvailable), cudaFuncAttributeMaxDynamicSharedMemorySize, one));
     return 0;
 }
 

@@ -3,8 +3,8 @@
 //
 // The lockstep grid (frame_kernels.cu) sweeps colour c of all instances together and closes it with a
 // grid barrier; its gathers go through L2 and stall most of the frame (issue slots 23 % busy).  An
-// instance is independent of the others, so here its colours are closed by its own CTA's barrier, and
-// two CTAs an SM fill each other's waits.
+// instance is independent of the others, so here its colours are closed by its own CTA's barrier and its
+// gathers are shared-memory reads.
 #include <algorithm>
 #include <numeric>
 
@@ -108,15 +108,19 @@ size_t brickBytes(const BrickPlan& p, const BrickDesc& d, bool damped) {
 
 }  // namespace
 
-template <bool Damped, bool PerType>
-static __global__ void __launch_bounds__(kBrickThreads, 1) brickBatchFrame(DeviceMesh m, FrameCoeffs fc, ContactParams cp, BrickTables bt,
+template <bool Damped, bool PerType, int Threads>
+static __global__ void __launch_bounds__(Threads, 1) brickBatchFrame(DeviceMesh m, FrameCoeffs fc, ContactParams cp, BrickTables bt,
                                                                            const BrickShape* shapes, const int* order, const int* start,
                                                                            const float2* instAlpha, unsigned* status) {
     batchFrame<Damped, PerType>(m, fc, cp, bt, shapes, order, start, instAlpha, status);
 }
-BrickBatchKernel brickBatchKernel(bool damped, bool perType) {
-    return damped ? (perType ? brickBatchFrame<true, true> : brickBatchFrame<true, false>)
-                  : (perType ? brickBatchFrame<false, true> : brickBatchFrame<false, false>);
+template <int Threads> static BrickBatchKernel batchKernelFor(bool damped, bool perType) {
+    return damped ? (perType ? brickBatchFrame<true, true, Threads> : brickBatchFrame<true, false, Threads>)
+                  : (perType ? brickBatchFrame<false, true, Threads> : brickBatchFrame<false, false, Threads>);
+}
+BrickBatchKernel BatchBricks::kernel(bool damped, bool perType) const {
+    return bound == kNarrowThreads ? batchKernelFor<kNarrowThreads>(damped, perType)
+           : bound == kSplitThreads ? batchKernelFor<kSplitThreads>(damped, perType) : batchKernelFor<kBrickThreads>(damped, perType);
 }
 
 void BatchBricks::release() {
@@ -126,7 +130,7 @@ void BatchBricks::release() {
     ctas = 0;
 }
 
-cudaError_t BatchBricks::plan(const std::vector<BatchBrickInstance>& in, int N, int smCount, int maxBytes, int maxBytesTwo, bool damped,
+cudaError_t BatchBricks::plan(const std::vector<BatchBrickInstance>& in, int N, int smCount, int maxBytes, bool damped,
                               cudaStream_t stream) {
     release();
     const int count = (int)in.size();
@@ -135,17 +139,19 @@ cudaError_t BatchBricks::plan(const std::vector<BatchBrickInstance>& in, int N, 
     for (int i = 0; i < count; i++) { tets[i] = in[i].mesh.nTetColors ? in[i].mesh.tetOff[in[i].mesh.nTetColors] : 0; all += tets[i]; }
     const int record = damped ? 32 : 16, fixed = 2048;
     std::vector<int> bricks(count, 1);
-    int slots, room;
-    if (count <= smCount && all <= (long long)kSplitTets * smCount) {
-        // few tets an SM: a colour is shorter than its latency, so every instance is spread over its share
-        // of the SMs, one CTA of up to 512 threads each
-        slots = smCount; room = maxBytes; threads = kBrickThreads;
+    // One CTA of up to 512 threads an SM (256 instances of 8..32 cells, 2 frames: 5.0 ms; two CTAs of 256
+    // threads an SM with half the shared memory each split more instances: 6.4 ms).
+    const int slots = smCount, room = maxBytes;
+    const bool spread = count <= smCount && all <= (long long)kSplitTets * smCount;
+    if (spread) {
+        // few tets an SM: a colour is shorter than its latency, so every instance is spread over its share of
+        // the SMs
         for (int i = 0; i < count; i++) bricks[i] = (int)std::max<long long>(1, all ? tets[i] * smCount / all : 1);
         int sum = std::accumulate(bricks.begin(), bricks.end(), 0);
         for (; sum > slots; sum--) (*std::max_element(bricks.begin(), bricks.end()))--;
     } else {
-        // many: two CTAs of 256 threads an SM, and only the instances well above a CTA's share are split
-        slots = 2 * smCount; room = maxBytesTwo; threads = kBrickThreads / 2;
+        // many: only the instances well above a CTA's share, and those that do not fit one, are split
+        // (splitting above 1.1, 1.25 and 1.6 shares: 5.4, 5.0 and 5.5 ms)
         const double roomNodes = (double)((room - fixed) / record);
         bool fits = false;
         double share = 1.05 * (double)all / slots;
@@ -215,23 +221,24 @@ cudaError_t BatchBricks::plan(const std::vector<BatchBrickInstance>& in, int N, 
         sum.maxLocal = std::max(sum.maxLocal, p.maxLocal);
         sum.maxOwned = std::max(sum.maxOwned, p.maxOwned);
         sum.threads = std::max(sum.threads, p.threads);
+        sum.tetWidth = std::max(sum.tetWidth, p.tetWidth);
     }
-    threads = std::min(threads, sum.threads);
-    // CTAs: exchanging bricks first, one each, then the others by longest processing time.  CTAs c and
-    // c + smCount usually share an SM, so a CTA's load counts its partner's too.
+    // narrow colours: CTAs of kNarrowThreads with the whole register file (brick_frame.cuh); spread instances
+    // with wider ones: 384 threads of 168 registers, which hold the node pass without spilling (12 instances
+    // of 8..20 cells, 4 frames: 1.56 ms, 1.73 with 512); else 512 (256 instances: 4.95 ms, 5.09 with 384)
+    bound = sum.tetWidth <= kNarrowColour ? kNarrowThreads : spread ? kSplitThreads : kBrickThreads;
+    threads = std::min(bound, sum.threads);
+    // CTAs: exchanging bricks first, one each, then the others by longest processing time
     std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.tied != b.tied ? a.tied : a.work > b.work; });
     const int used = std::min(slots, (int)items.size());
     std::vector<std::vector<int>> lists(used);
-    std::vector<double> own(used, 0.), pair(smCount, 0.);
+    std::vector<double> load(used, 0.);
     for (const Item& it : items) {
         int best = -1;
-        for (int c = 0; c < used; c++) {
-            if (it.tied && !lists[c].empty()) continue;
-            if (best < 0 || own[c] + 0.5 * pair[c % smCount] < own[best] + 0.5 * pair[best % smCount]) best = c;
-        }
+        for (int c = 0; c < used; c++)
+            if (!(it.tied && !lists[c].empty()) && (best < 0 || load[c] < load[best])) best = c;
         lists[best].push_back(it.id);
-        own[best] += it.work;
-        pair[best % smCount] += it.work;
+        load[best] += it.work;
     }
     std::vector<int> orderHost, startHost(1, 0);
     for (auto& l : lists) { orderHost.insert(orderHost.end(), l.begin(), l.end()); startHost.push_back((int)orderHost.size()); }

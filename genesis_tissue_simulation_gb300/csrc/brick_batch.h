@@ -17,29 +17,30 @@ struct BatchBrickInstance {
     const unsigned char* tetDead;
 };
 
+// The frame kernel: perType, one compliance per instance and Kuhn type (instAlpha [6 x instances]); else
+// the tables' tetAlpha.
+using BrickBatchKernel = void (*)(DeviceMesh m, FrameCoeffs fc, ContactParams cp, BrickTables bt, const BrickShape* shapes, const int* order,
+                                  const int* start, const float2* instAlpha, unsigned* status);
+
 // The bricks of a batch and their CTAs.  CTA c serves the bricks order[start[c]] .. order[start[c + 1] - 1]
 // one after another; a brick that exchanges with others is always its CTA's first, so all of them run
 // at the same time (the launch is cooperative).
 // Below this many tets an SM the instances of a batch are spread over all SMs.
 constexpr int kSplitTets = 8000;
+constexpr int kSplitThreads = 384;
 
 struct BatchBricks {
     BrickBuffers buffers;
     BrickShape* shapes = nullptr;
     int* order = nullptr; int* start = nullptr;
     int ctas = 0, threads = 0; size_t bytes = 0;
+    int bound = 0;   // threads the kernel is compiled for
+    BrickBatchKernel kernel(bool damped, bool perType) const;
     bool ready() const { return ctas > 0; }
     void release();
-    // Plans every instance; not ready when one does not fit.  maxBytes: shared memory of one CTA, of two
-    // on an SM at most maxBytesTwo each.
-    cudaError_t plan(const std::vector<BatchBrickInstance>& instances, int N, int smCount, int maxBytes, int maxBytesTwo, bool damped,
+    // Plans every instance; not ready when one does not fit.  maxBytes: shared memory of one CTA.
+    cudaError_t plan(const std::vector<BatchBrickInstance>& instances, int N, int smCount, int maxBytes, bool damped,
                      cudaStream_t stream);
 };
-
-// The frame kernel: perType, one compliance per instance and Kuhn type (instAlpha [6 x instances]); else
-// the tables' tetAlpha.
-using BrickBatchKernel = void (*)(DeviceMesh m, FrameCoeffs fc, ContactParams cp, BrickTables bt, const BrickShape* shapes, const int* order,
-                                  const int* start, const float2* instAlpha, unsigned* status);
-BrickBatchKernel brickBatchKernel(bool damped, bool perType);
 
 }  // namespace gbt

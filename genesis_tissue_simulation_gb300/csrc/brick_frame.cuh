@@ -20,7 +20,7 @@
 namespace gbt {
 
 constexpr int kBrickThreads = 512;
-// Plans whose widest colour has at most kNarrowColour elements run in CTAs of kNarrowThreads: twice the
+// Plans whose widest tet colour has at most kNarrowColour elements a brick run in CTAs of kNarrowThreads: twice the
 // registers a thread and fewer warps at each barrier pay for the few second rounds (us a substep, 512 ->
 // 256: 23 x 13 x 19 cells, 320 wide, 34.0 -> 32.8; 32 x 16 x 32 cells, 320 wide, 39.0 -> 38.5; 64 x 32 x 48
 // cells, 896 wide, 62.1 -> 69.2).

@@ -310,7 +310,7 @@ cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int 
     release();
     tets = (int)plan.tetWord.size(); edges = (int)plan.edgeWord.size();
     asked = plan.asked;
-    threads = plan.threads <= kNarrowColour ? (plan.threads < kNarrowThreads ? plan.threads : kNarrowThreads)
+    threads = plan.tetWidth <= kNarrowColour ? (plan.threads < kNarrowThreads ? plan.threads : kNarrowThreads)
                                             : (plan.threads < kBrickThreads ? plan.threads : kBrickThreads);
     BrickTables q{};
     q.shape = plan.shape();

@@ -335,7 +335,11 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         for (int st = 0; st < S; st++) records += (int)(imports[b][st].size() + exports[b][st].size());
         plan.maxList = std::max(plan.maxList, records);
     }
-    for (auto& lists : elements) for (auto& list : lists) plan.threads = std::max(plan.threads, ((int)list.size() + 31) / 32 * 32);
+    for (auto& lists : elements)
+        for (int p = 0; p < P; p++) {
+            plan.threads = std::max(plan.threads, ((int)lists[p].size() + 31) / 32 * 32);
+            if (!ph.isEdge(p)) plan.tetWidth = std::max(plan.tetWidth, (int)lists[p].size());
+        }
     plan.bricks = B; plan.asked = count; plan.stages = S; plan.nEdgeColors = m.nEdgeColors; plan.nTetColors = nT; plan.tensilePasses = m.tensilePasses; plan.cost = cost;
     for (int p = 0; p < P; p++) if (before[p] && B > 1) plan.exchangeBefore[p >> 6] |= 1ull << (p & 63);
     return plan;

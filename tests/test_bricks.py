@@ -6,7 +6,8 @@ import numpy as np
 import pytest
 
 from genesis_tissue_simulation_gb300.grid import build_grid
-from genesis_tissue_simulation_gb300.native_backend import Capsule, PlainTissue, blade_sweep
+from genesis_tissue_simulation_gb300 import workloads as W
+from genesis_tissue_simulation_gb300.native_backend import Capsule, GraspParams, PlainTissue, blade_sweep
 
 pytestmark = pytest.mark.gpu
 
@@ -20,7 +21,8 @@ def frames(lib, size, bricks=0, mode=0, damping=0.0, ks=1e6, capsule=True, steps
     gpu = hasattr(dll, "GBT_SetBrickCount")
     if gpu:
         assert dll.GBT_SetBrickCount(bricks) == 0
-    with PlainTissue(grid, dt=1 / 60, substeps=substeps, ks=ks, strain_damping_s=damping, tear_ratio=tear, dll_path=lib) as t:
+    with PlainTissue(grid, dt=1 / 60, substeps=substeps, ks=ks, strain_damping_s=damping, tear_ratio=tear, grasp_params=GraspParams(**W.DEFAULT_GRASP),
+                     dll_path=lib) as t:   # contact parameters outlive a session
         info = np.zeros(4, np.int32)
         try:
             if gpu:
