@@ -201,7 +201,7 @@ cudaError_t BatchBricks::plan(const std::vector<BatchBrickInstance>& in, int N, 
         const int node0 = (int)sum.localNode.size(), edge0 = (int)sum.edgeWord.size(), tet0 = (int)sum.tetWord.size(),
                   imp0 = (int)sum.importList.size(), exp0 = (int)sum.exportList.size();
         for (const BrickDesc& d : p.desc) {
-            sum.desc.push_back({d.nodeBase + node0, d.nOwned, d.nLocal, (int)sum.head.size(), i});
+            sum.desc.push_back({d.nodeBase + node0, d.nOwned, d.nLocal, (int)sum.head.size(), i, 0, 0});
             const int* h = p.head.data() + d.head;
             auto put = [&](int n, int base) { for (int k = 0; k < n; k++) sum.head.push_back(*h++ + base); };
             put(p.nEdgeColors + 1, edge0); put(p.nTetColors + 1, tet0); put(p.stages + 1, imp0); put(p.stages + 1, exp0);

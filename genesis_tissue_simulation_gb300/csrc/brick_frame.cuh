@@ -36,6 +36,7 @@ struct BrickTables {
     int listsShared;
     const unsigned long long* tetWord; const float2* tetAlpha;
     const unsigned* edgeWord; const float* edgeRest;
+    const int* ownTet;                                         // words of each brick's own tets (plans with a tensile pass)
     const int* tetSrc; const int* edgeSrc;                     // colour slots of the mesh's tables
     float4* mail;                                              // [2 x N] published values
     float4* mailStart;                                         // [2 x N] published substep-start positions (damped sweeps)
@@ -122,6 +123,7 @@ struct Brick {
     float4* A;        // [maxOwned] accelerations
     ContactFrame* frames;   // [kBrickFrames]
     float* typeB;     // [6 x 9] rest inverses
+    const float* fibres;       // [6 x 6] rest lengths of the tensile fibres per Kuhn type (guarded sweeps)
     const float2* typeAlpha;   // [6] compliances per Kuhn type (sweeps without one per tet)
     int* head;        // offsets of this brick (brick_plan.h)
     const int *edgeOff, *tetOff, *impOff, *expOff;
@@ -242,11 +244,11 @@ struct Brick {
         const int id[4] = {(int)(lo & kBrickNodeMask), (int)((lo >> kBrickNodeBits) & kBrickNodeMask), (int)(hi & kBrickNodeMask),
                            (int)((hi >> kBrickNodeBits) & kBrickNodeMask)};
         const float4 q[4] = {P[id[0]], P[id[1]], P[id[2]], P[id[3]]};
-        f3 p[4] = {xyz(q[0]), xyz(q[1]), xyz(q[2]), xyz(q[3])}, b[3];
-        const float* B = typeB + 9 * ((hi >> 28) & 7u);
-        b[0] = mk(B[0], B[1], B[2]); b[1] = mk(B[3], B[4], B[5]); b[2] = mk(B[6], B[7], B[8]);
-        float lambda[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        solveTensile(b, q, w.alpha.x / fmaxf(fc.tensileStrength, 1e-10f), lambda, p);
+        f3 p[4] = {xyz(q[0]), xyz(q[1]), xyz(q[2]), xyz(q[3])};
+        float rest[6], lambda[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int f = 0; f < 6; f++) rest[f] = fibres[6 * ((hi >> 28) & 7u) + f];
+        solveTensile(rest, q, w.alpha.x / fmaxf(fc.tensileStrength, 1e-10f), lambda, p);
 #pragma unroll
         for (int c = 0; c < 4; c++) P[id[c]] = make_float4(p[c].x, p[c].y, p[c].z, q[c].w);
     }
@@ -254,9 +256,9 @@ struct Brick {
     // by this thread.
     __device__ __forceinline__ bool belowMinimum(float minimum) const {
         bool below = false;
-        for (int k = tetOff[0] + threadIdx.x; k < tetOff[s.nT]; k += blockDim.x) {
-            const unsigned long long w = bt.tetWord[k];
-            if (!(w & kBrickTetLive) || !(w & kBrickTetOwner)) continue;
+        for (int k = threadIdx.x; k < d.nOwn; k += blockDim.x) {
+            const unsigned long long w = bt.tetWord[bt.ownTet[d.ownFirst + k]];
+            if (!(w & kBrickTetLive)) continue;
             const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 28);
             const float* B = typeB + 9 * ((hi >> 28) & 7u);
             const f3 b0 = mk(B[0], B[1], B[2]), b1 = mk(B[3], B[4], B[5]), b2 = mk(B[6], B[7], B[8]);

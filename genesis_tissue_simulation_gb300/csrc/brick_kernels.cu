@@ -122,6 +122,7 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
     const bool guarded = Extended && fc.guarded != 0;
     const int exchanges = bt.bricks > 1 ? fc.substeps * (bt.shape.stages + (guarded ? 1 : 0)) : 0;
     __shared__ FrictionShapes shapes[Extended ? kBrickFrames : 1];
+    __shared__ float fibres[Extended ? 36 : 1];
     Brick b(bt, bt.shape, m.typeB, blockIdx.x, shared, Damped, true, exchanges, state + 2, fc.spinBudget, fc.syncTestExtra > 0 ? 1u << 30 : 0u);
     const bool stamp = fc.phaseClock != nullptr && blockIdx.x == 0 && tid == 0;
     int s = 0, slot = 0;
@@ -135,6 +136,12 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
     b.loadState(m.pos, m.vel, m.ext);
     TickState ts{Cut ? *(volatile unsigned*)cu.counters : 0u, fc.rotParity, 0u, true};
     bool havePrev = cu.havePrev != 0;
+    if (Extended && tid < 36) {   // rest lengths of the six corner-to-corner fibres of every Kuhn type
+        f3 r[3];
+        typeRows(m, tid / 6, r);
+        fibres[tid] = fibreRest(r, tid % 6);
+    }
+    b.fibres = fibres;
     for (; s < fc.substeps; s++) {
         slot = 0;
         mark(kPhaseFrameStart);
@@ -327,6 +334,7 @@ cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int 
     if (e == cudaSuccess) e = put((float**)&q.edgeRest, plan.edgeRest.data(), plan.edgeRest.size(), stream);
     if (e == cudaSuccess) e = put(&tetSrc, plan.tetSrc.data(), plan.tetSrc.size(), stream);
     if (e == cudaSuccess) e = put(&edgeSrc, plan.edgeSrc.data(), plan.edgeSrc.size(), stream);
+    if (e == cudaSuccess) e = put((int**)&q.ownTet, plan.ownTet.data(), plan.ownTet.size(), stream);
     const size_t mail = plan.bricks > 1 ? 2 * (size_t)N : 0;
     if (e == cudaSuccess) e = put(&q.mail, (const float4*)nullptr, mail, stream);
     if (e == cudaSuccess) e = put(&q.mailStart, (const float4*)nullptr, damped ? mail : 0, stream);

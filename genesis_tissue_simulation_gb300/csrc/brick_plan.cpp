@@ -279,7 +279,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
     };
     for (int b = 0; b < B; b++) {
         int* h = plan.head.data() + (size_t)b * headWords;
-        plan.desc[b] = {nNode, (int)owned[b].size(), (int)(owned[b].size() + halo[b].size()), b * headWords, 0};
+        plan.desc[b] = {nNode, (int)owned[b].size(), (int)(owned[b].size() + halo[b].size()), b * headWords, 0, 0, 0};
         nNode += plan.desc[b].nLocal;
         // colours in sweep order
         for (int c = 0; c < m.nEdgeColors; c++) { *h++ = nEdge; nEdge += (int)elements[b][phaseOf(true, reverse ? m.nEdgeColors - 1 - c : c)].size(); }
@@ -339,6 +339,13 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         for (int p = 0; p < P; p++) {
             plan.threads = std::max(plan.threads, ((int)lists[p].size() + 31) / 32 * 32);
             if (!ph.isEdge(p)) plan.tetWidth = std::max(plan.tetWidth, (int)lists[p].size());
+        }
+    if (m.tensilePasses > 0)
+        for (int b = 0; b < B; b++) {
+            const int* tetOff = plan.head.data() + plan.desc[b].head + m.nEdgeColors + 1;
+            plan.desc[b].ownFirst = (int)plan.ownTet.size();
+            for (int k = tetOff[0]; k < tetOff[m.nTetColors]; k++) if (plan.tetWord[k] & kBrickTetOwner) plan.ownTet.push_back(k);
+            plan.desc[b].nOwn = (int)plan.ownTet.size() - plan.desc[b].ownFirst;
         }
     plan.bricks = B; plan.asked = count; plan.stages = S; plan.nEdgeColors = m.nEdgeColors; plan.nTetColors = nT; plan.tensilePasses = m.tensilePasses; plan.cost = cost;
     for (int p = 0; p < P; p++) if (before[p] && B > 1) plan.exchangeBefore[p >> 6] |= 1ull << (p & 63);

@@ -14,6 +14,7 @@ struct BrickDesc {
     int nodeBase, nOwned, nLocal;   // localNode[nodeBase + l]: node of local index l, owned nodes first
     int head;
     int shape;                      // of a batch: the instance's plan
+    int ownFirst, nOwn;             // ownTet[ownFirst .. ownFirst + nOwn): the words of the tets it owns (plans with a tensile pass)
 };
 
 // The sweep of one plan: colours, stages, and the phases an exchange precedes (bit p: phase p).
@@ -51,7 +52,7 @@ struct BrickPlan {
     std::vector<BrickDesc> desc;
     std::vector<int> head, localNode, idle;
     std::vector<int2> importList, exportList;   // (local index, node)
-    std::vector<uint64_t> tetWord; std::vector<int> tetSrc;
+    std::vector<uint64_t> tetWord; std::vector<int> tetSrc, ownTet;
     std::vector<unsigned> edgeWord; std::vector<float> edgeRest; std::vector<int> edgeSrc;
     bool ok() const { return bricks > 0; }
     BrickShape shape() const { return {nEdgeColors, nTetColors / (1 + tensilePasses), stages, bricks, nTetColors / (1 + tensilePasses) * tensilePasses, {exchangeBefore[0], exchangeBefore[1]}}; }

@@ -614,16 +614,27 @@ __device__ __forceinline__ void typeRows(const DeviceMesh& m, int type, f3 b[3])
 // corner-to-corner fibres carries mu V strength / 2 s^6, s = max(length / rest - 1, 0), projected
 // with finite compliance alphaDev / strength; the rest corners are the columns of (Dm^-1)^-1.
 // `pass` > 0 continues the fibres' multipliers of this substep.
-__device__ __forceinline__ void solveTensile(const f3 (&b)[3], const float4 (&P)[4], float alpha, float (&lambda)[6], f3 (&p)[4]) {
+// Rest length of fibre f (corner pairs 01, 02, 03, 12, 13, 23) of a tet with rest inverse rows b.
+__device__ __forceinline__ float fibreRest(const f3 (&b)[3], int f) {
     float detB = dot(b[0], cross(b[1], b[2]));
     f3 rest[4] = {mk(0.f, 0.f, 0.f), cross(b[1], b[2]) * (1.f / detB), cross(b[2], b[0]) * (1.f / detB), cross(b[0], b[1]) * (1.f / detB)};
+    int at = 0;
+    float out = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = i + 1; j < 4; j++, at++)
+            if (at == f) out = len(rest[j] - rest[i]);
+    return out;
+}
+__device__ __forceinline__ void solveTensile(const float (&restLengths)[6], const float4 (&P)[4], float alpha, float (&lambda)[6], f3 (&p)[4]) {
     int fiber = 0;
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = i + 1; j < 4; j++, fiber++) {
             f3 edge = p[j] - p[i];
-            float length = len(edge), restLength = len(rest[j] - rest[i]);
+            float length = len(edge), restLength = restLengths[fiber];
             float strain = fmaxf(length / restLength - 1.f, 0.f), gradient = 3.f * strain * strain / restLength;
             float wi = P[i].w, wj = P[j].w;
             if (strain > 0.f && length > 0.f) {
@@ -644,10 +655,13 @@ __device__ __forceinline__ void projectTensile(const DeviceMesh& m, int k, const
     f3 p[4] = {xyz(P[0]), xyz(P[1]), xyz(P[2]), xyz(P[3])};
     f3 b[3];
     typeRows(m, meta & 7, b);
-    float lambda[6];
+    float lambda[6], rest[6];
 #pragma unroll
-    for (int f = 0; f < 6; f++) lambda[f] = pass == 0 ? 0.f : m.fiberLambda[6 * (size_t)k + f];
-    solveTensile(b, P, m.tetAlpha[k].x / fmaxf(fc.tensileStrength, 1e-10f), lambda, p);
+    for (int f = 0; f < 6; f++) {
+        lambda[f] = pass == 0 ? 0.f : m.fiberLambda[6 * (size_t)k + f];
+        rest[f] = fibreRest(b, f);
+    }
+    solveTensile(rest, P, m.tetAlpha[k].x / fmaxf(fc.tensileStrength, 1e-10f), lambda, p);
     if (fc.volumePasses > 1)
 #pragma unroll
         for (int f = 0; f < 6; f++) m.fiberLambda[6 * (size_t)k + f] = lambda[f];
