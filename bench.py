@@ -793,7 +793,8 @@ def main():
         torch.cuda.synchronize()
         e2e_s = time.perf_counter() - e0
         assert np.isfinite(positions).all(), "non-finite tissue state"
-        # the phase floor: grid barriers per frame launch and one barrier's latency with no work
+        # the synchronisation floor: halo exchanges per frame launch (a brick frame) and the latency of one
+        # gpu-scope round trip with no work, which each of them costs at least
         barriers = session.frame_barriers()
         barrier_us = session.grid_barrier_floor(20000) if barriers else None
     finally:
@@ -827,16 +828,16 @@ def main():
         "wall_steps_per_s": world * args.steps / wall,
         "e2e": {"value": world * args.steps / e2e_s, "unit": "steps/s", "h2d_bytes_per_step": 92 + 4,
                 "d2h_bytes_per_step": 12 * len(w.grid.positions) + 12},
-        "gpu_launches": args.steps,
+        "gpu_launches": 2 * args.steps,   # LCS_Step: the frame and the closing particle-frame pass
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "peak_kind": peak_kind, "algorithmic_bytes_per_launch": substeps * bytes_per_substep},
         "clocks": clocks.summary(),
     }
     if barriers:
         floor_ms = barriers * barrier_us / 1e3
-        line["sync_floor"] = {"bound": "grid barrier latency", "barriers_per_launch": barriers, "us_per_barrier": barrier_us,
+        line["sync_floor"] = {"bound": "halo exchange latency", "exchanges_per_launch": barriers, "us_per_round_trip": barrier_us,
                               "floor_ms": floor_ms, "ms_per_launch": 1e3 * launch_s, "frac": floor_ms / (1e3 * launch_s),
-                              "measured": "GBT_GridBarrierFloor: 20,000 back-to-back barriers on the frame kernel's grid"}
+                              "measured": "GBT_GridBarrierFloor: 20,000 back-to-back barriers of one CTA per SM"}
     if not args.no_workloads:
         line["workloads"] = {"c1": workload_measurement(lib, "c1", 100, 5), "c3": workload_measurement(lib, "c3", 30, 3)}
         # the reference's own CUDA build on the same box and plugin call sequence, against ours

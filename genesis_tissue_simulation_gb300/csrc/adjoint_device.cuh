@@ -144,6 +144,7 @@ __device__ __forceinline__ void tetVJP(const float* Bm, const float4 P[4], const
     }
     gd[0] = (gd[1] + gd[2] + gd[3]) * -1.f;
     gh[0] = (gh[1] + gh[2] + gh[3]) * -1.f;
+    const bool damped = dampingOverH != 0.f;   // undamped: the velocity terms and their adjoints are zeros
     float dd = 0.f, dh = 0.f, vd = 0.f, vh = 0.f, w[4];
     f3 dx[4];
 #pragma unroll
@@ -151,9 +152,11 @@ __device__ __forceinline__ void tetVJP(const float* Bm, const float4 P[4], const
         w[c] = P[c].w;
         dd = fmaf(w[c], dotF(gd[c], gd[c]), dd);
         dh = fmaf(w[c], dotF(gd[c], gh[c]), dh);
-        dx[c] = p[c] - q[c];
-        vd += dotF(gd[c], dx[c]);
-        vh += dotF(gh[c], dx[c]);
+        if (damped) {
+            dx[c] = p[c] - q[c];
+            vd += dotF(gd[c], dx[c]);
+            vh += dotF(gh[c], dx[c]);
+        }
     }
     float scale = 1.f + dampingOverH, invScale = 1.f / scale;
     float eAd = ad * invScale, eAh = ah * invScale;
@@ -162,7 +165,6 @@ __device__ __forceinline__ void tetVJP(const float* Bm, const float4 P[4], const
     f3 r[4];
 #pragma unroll
     for (int c = 0; c < 4; c++) { r[c] = fmv(gd[c], -gamma, gh[c]); schur = fmaf(w[c], dotF(r[c], r[c]), schur); }
-    const bool damped = dampingOverH != 0.f;
     float rd = damped ? fmaf(-dampingOverH, vd, -CD) * invScale : -CD * invScale;
     float rh = damped ? fmaf(-(scale - 1.f), vh, -CH) * invScale : -CH * invScale;
     if (!(A > 0.f) || !(schur > 0.f)) return;
@@ -218,11 +220,15 @@ __device__ __forceinline__ void tetVJP(const float* Bm, const float4 P[4], const
     // dd, dh, vd, vh
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-        ggd[c] = ggd[c] + gd[c] * (2.f * w[c] * gdd) + gh[c] * (w[c] * gdh) + dx[c] * gvd;
-        ggh[c] = ggh[c] + gd[c] * (w[c] * gdh) + dx[c] * gvh;
-        f3 gdx = gd[c] * gvd + gh[c] * gvh;
-        out.gp[c] = out.gp[c] + gdx;
-        out.gq[c] = zero - gdx;
+        ggd[c] = ggd[c] + gd[c] * (2.f * w[c] * gdd) + gh[c] * (w[c] * gdh);
+        ggh[c] = ggh[c] + gd[c] * (w[c] * gdh);
+        if (damped) {
+            ggd[c] = ggd[c] + dx[c] * gvd;
+            ggh[c] = ggh[c] + dx[c] * gvh;
+            f3 gdx = gd[c] * gvd + gh[c] * gvh;
+            out.gp[c] = out.gp[c] + gdx;
+            out.gq[c] = zero - gdx;
+        }
     }
     // gd_0 = -(gd_1 + gd_2 + gd_3), gh_0 likewise
 #pragma unroll

@@ -582,8 +582,9 @@ __global__ void __launch_bounds__(kBlockThreads) frameKernelBlockExt(DeviceMesh 
 // One frame pass over every node, k_ComputeParticleRot (V/physics.cu:109-205): frames from
 // particleRot[p] into particleRot[p ^ 1], p = *parityWord when given (the parity a frame kernel left
 // on the device), else `parity`.
-__global__ void particleRotKernel(DeviceMesh m, const unsigned* parityWord, int parity) {
+__global__ void particleRotKernel(DeviceMesh m, const unsigned* parityWord, int parity, const unsigned* state, unsigned* hostState) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (hostState && c < 4) hostState[c] = state[c];   // pinned: the frame's words reach the host without a copy
     const int p = parityWord ? (int)(*parityWord & 1u) : parity;
     if (c < m.nNodes) particleFrame(c, m.pos, m.nbr, m.active, m.pinned, m.particleRot[p], m.particleRot[p ^ 1]);
 }

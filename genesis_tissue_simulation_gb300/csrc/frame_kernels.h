@@ -41,7 +41,8 @@ constexpr int kSessionClusterThreads = 256, kSessionClusterLogThreads = 8;
 __global__ void frameKernelSessionCluster(DeviceMesh m, FrameCoeffs fc, ToolPose from, ToolPose to, ContactParams cp,
                                           CutParams cu, unsigned* state, int logK);
 
-__global__ void particleRotKernel(DeviceMesh m, const unsigned* parityWord, int parity);
+__global__ void particleRotKernel(DeviceMesh m, const unsigned* parityWord, int parity, const unsigned* state = nullptr,
+                                  unsigned* hostState = nullptr);
 __global__ void tetAlphaKernel(int n, float invH2, const float2* stiff, float2* alpha);
 __global__ void gravityKernel(int n, float gx, float gy, float gz, float4* ext);
 // xyz of n float4 records, packed as 3n floats (the getters' host layout)

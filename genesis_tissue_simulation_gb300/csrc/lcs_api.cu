@@ -61,7 +61,7 @@ struct Session {
     // tissue guard buffers (LCS_SetTissueGuard): fibre multipliers, feasibility candidates and marks,
     // incident colour slots per node (CSR), two flags
     DBuf<float> fiberLambda; DBuf<float4> feasTarget; DBuf<int> needed, incOff, incTet; DBuf<unsigned> guardFlags;
-    float lastH = -1.f;
+    float lastH = -1.f, brickH = -1.f;   // substep length the compliances (the bricks' compliances) are for
     // topology sizes (host copies for diagnostics)
     int E = 0, B = 0, T = 0;
     std::vector<int> edgeColorOff, bendColorOff, tetColorOff;   // host copies [colors+1]
@@ -167,7 +167,7 @@ void freePhysics() {
     // xpbd_shutdown, xpbd_solver.cu:3829); a material set before the first LCS_InitPhysics stays
     if (S.physReady) { S.tissueHardening = 80.f; S.bulkDampingSeconds = 0.003125f; }
     S.autoShape = -1; S.autoTrial = 0; S.autoMs[0] = S.autoMs[1] = S.autoMs[2] = -1.f;
-    S.physReady = false; S.toolArmed = false; S.E = S.B = S.T = 0; S.lastH = -1.f;
+    S.physReady = false; S.toolArmed = false; S.E = S.B = S.T = 0; S.lastH = S.brickH = -1.f;
 }
 void freeAll() {
     freePhysics();
@@ -367,7 +367,15 @@ BrickBuffers* brickFrames(const FrameCoeffs& fc) {
     if (!b->ready() || (fc.friction && !fc.guarded && b->sharedBytes(S.bricksDamped) > (size_t)S.maxGuardBytes)) return nullptr;
     return b;
 }
-int launchBricks(BrickBuffers& bricks, const FrameCoeffs& fc, bool* followUp) {
+// The plans' compliances for the frame's substep length.
+int brickCompliances(const FrameCoeffs& fc) {
+    if (!fc.doStrain || fc.h == S.brickH) return 0;
+    for (BrickBuffers* b : {&S.bricks, &S.guardBricks}) if (b->ready()) CK(b->compliances(fc.invH2, S.tetStiff.p, S.stream));
+    S.brickH = fc.h;
+    return 0;
+}
+// `state`: the frame's words; hostState: their pinned copy, or null.
+int launchBricks(BrickBuffers& bricks, const FrameCoeffs& fc, unsigned* state, unsigned* hostState, bool* followUp) {
     DeviceMesh m = deviceMesh();
     if (S.bricksStale) {
         CK(refreshMeshFlags(m, S.E, S.T, fc.fallback != 0, S.stream));
@@ -378,14 +386,13 @@ int launchBricks(BrickBuffers& bricks, const FrameCoeffs& fc, bool* followUp) {
     FrameCoeffs f = fc;
     ToolPose from = S.toolFrom, to = S.tool;
     ContactParams cp = S.cp;
-    unsigned* state = S.state.p;
     CutParams cu = cutParams();
     if (fc.cut && S.brickCount.p) CK(cudaMemsetAsync(S.brickCount.p, 0, sizeof(unsigned), S.stream));
     if (fc.guarded) CK(cudaMemsetAsync(S.guardFlags.p, 0, 5 * sizeof(unsigned), S.stream));
     void* args[] = {&m, &f, &from, &to, &cp, &bricks.t, &cu, &state};
     CK(cudaLaunchCooperativeKernel((const void*)brickFrameKernelFor(damped, fc.cut != 0, extended, bricks.threads), dim3(bricks.t.bricks), dim3(bricks.threads),
                                    args, bricks.sharedBytes(damped), S.stream));
-    particleRotKernel<<<(S.N + 255) / 256, 256, 0, S.stream>>>(m, fc.cut ? state + 3 : nullptr, fc.rotParity);
+    particleRotKernel<<<(S.N + 255) / 256, 256, 0, S.stream>>>(m, fc.cut ? state + 3 : nullptr, fc.rotParity, state, hostState);
     CK(cudaGetLastError());
     // without ticks or the guard the kernel leaves its exchanges in the barrier counter
     S.lastFrameBlocks = fc.cut || fc.guarded ? bricks.t.bricks : 1;
@@ -513,7 +520,7 @@ FrameCoeffs frameCoeffs(float h, int N) {
 int launchFrame(const FrameCoeffs& fc, bool* followUp) {
     unsigned* state = S.state.p;
     CK(cudaMemsetAsync(state + 1, 0, 2 * sizeof(unsigned), S.stream));
-    if (BrickBuffers* bricks = brickFrames(fc)) return launchBricks(*bricks, fc, followUp);
+    if (BrickBuffers* bricks = brickFrames(fc)) return launchBricks(*bricks, fc, S.state.p, S.hostState, followUp);
     if (S.brickCount.p) CK(cudaMemsetAsync(S.brickCount.p, 0, sizeof(unsigned), S.stream));
     const Shapes u = usableShapes(fc);
     int shape = requestedShape(u);
@@ -744,7 +751,7 @@ LCS_API int LCS_SetTetStiffness(int count, const float* muV, const float* kappaV
     }
     CK(cudaMemcpyAsync(S.tetStiff.p, c.data(), count * sizeof(float2), cudaMemcpyHostToDevice, S.stream));
     CK(cudaStreamSynchronize(S.stream));
-    S.lastH = -1.f;
+    S.lastH = S.brickH = -1.f;
     return 0;
 }
 
@@ -815,6 +822,7 @@ LCS_API int LCS_SetTissueGuard(float minimum, int passes, int count, const int* 
     S.volumePasses = passes;
     S.minVolume = minimum;
     S.guardBricks.release();
+    S.brickH = -1.f;
     if (passes == 1 && S.T > 0) {   // more passes carry multipliers from one to the next
         BrickMesh bm = brickMesh();
         bm.tensilePasses = 1;
@@ -956,9 +964,10 @@ LCS_API int LCS_Step(float dt) {
     if (fc.doStrain && h != S.lastH) {
         tetAlphaKernel<<<(S.T + 255) / 256, 256, 0, S.stream>>>(S.T, fc.invH2, S.tetStiff.p, S.tetAlpha.p);
         CK(cudaGetLastError());
-        for (BrickBuffers* b : {&S.bricks, &S.guardBricks}) if (b->ready()) CK(b->compliances(fc.invH2, S.tetStiff.p, S.stream));
         S.lastH = h;
     }
+    int rc = brickCompliances(fc);
+    if (rc) return rc;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (S.profile) {
         CK(cudaEventCreate(&e0)); CK(cudaEventCreate(&e1));
@@ -972,10 +981,10 @@ LCS_API int LCS_Step(float dt) {
     }
     bool followUp = false;
     const bool onBricks = brickFrames(fc) != nullptr;
-    int rc = launchFrame(fc, &followUp);
+    rc = launchFrame(fc, &followUp);
     if (rc) return rc;
     if (S.profile) { CK(cudaEventRecord(e1, S.stream)); S.events.push_back(e0); S.events.push_back(e1); }
-    CK(cudaMemcpyAsync(S.hostState, S.state.p, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
+    if (!onBricks) CK(cudaMemcpyAsync(S.hostState, S.state.p, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
     if (S.sections) {
         S.phaseHost.resize(records);
         CK(cudaMemcpyAsync(S.phaseHost.data(), S.phaseClock.p, records * sizeof(unsigned long long), cudaMemcpyDeviceToHost, S.stream));
@@ -1322,22 +1331,29 @@ LCS_API int LCS_StepNoAlloc(float dt) {
     g_stepScratchOwner[device] = S.generation;
     CK(cudaMemsetAsync(state + 1, 0, 3 * sizeof(unsigned), S.stream));
     if (S.brickCount.p) CK(cudaMemsetAsync(S.brickCount.p, 0, sizeof(unsigned), S.stream));
-    if (fc.doStrain) {
-        tetAlphaKernel<<<(S.T + 255) / 256, 256, 0, S.stream>>>(S.T, fc.invH2, S.tetStiff.p, alpha);
-        CK(cudaGetLastError());
-    }
-    DeviceMesh m = deviceMesh();
-    m.tetAlpha = alpha;
-    const Shapes u = usableShapes(fc);
-    const int shape = requestedShape(u);   // no timed trials here: they would create events
     bool followUp = false;
-    int rc = launchShape(shape, u, fc, m, state, &followUp);
+    BrickBuffers* bricks = brickFrames(fc);
+    int rc = 0;
+    if (bricks) {   // the plan's tables and compliances belong to the session
+        rc = brickCompliances(fc);
+        if (!rc) rc = launchBricks(*bricks, fc, state, nullptr, &followUp);
+    } else {
+        if (fc.doStrain) {
+            tetAlphaKernel<<<(S.T + 255) / 256, 256, 0, S.stream>>>(S.T, fc.invH2, S.tetStiff.p, alpha);
+            CK(cudaGetLastError());
+        }
+        DeviceMesh m = deviceMesh();
+        m.tetAlpha = alpha;
+        const Shapes u = usableShapes(fc);
+        rc = launchShape(requestedShape(u), u, fc, m, state, &followUp);   // no timed trials here: they would create events
+    }
     S.lastFrameBlocks = 0;   // its barrier counter lives in the static scratch, not the session state
     if (rc) return rc;
     unsigned words[2] = {0u, 0u};   // status, current particle-frame buffer
     CK(cudaMemcpyAsync(words, state + 2, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
     CK(cudaStreamSynchronize(S.stream));
-    if (fc.cut) S.havePrev = S.bricksStale = true;
+    if (fc.cut) S.havePrev = true;
+    if ((fc.cut && !bricks) || words[0] != 0u) S.bricksStale = true;
     if (S.toolArmed) S.toolFrom = S.tool;
     if (words[0] != 0u) return LCS_ERR_DEVICE_TIMEOUT;
     S.rotParity = (int)((words[1] & 1u) ^ (followUp ? 1u : 0u));

@@ -414,8 +414,8 @@ class PlainTissue(_Session):
                     colours=int(counts[2]), sweeps=int(counts[3]))
 
     def frame_barriers(self):
-        """Grid barriers the last frame executed on the whole-GPU grid (GBT_FrameBarriers; CUDA
-        library only), or None when that frame ran in another launch shape."""
+        """Grid barriers the last frame executed on the whole-GPU grid, or the halo exchanges of a plain
+        frame on bricks (GBT_FrameBarriers; CUDA library only); None in the other launch shapes."""
         f = self.dll.GBT_FrameBarriers
         f.argtypes, f.restype = (ct.c_void_p,), ct.c_int
         out = ct.c_uint(0)

@@ -203,11 +203,12 @@ LCS_API int LCS_SetBarrierTest(int extraArrivals, float budgetSeconds);
  * closes one phase.  GBT_GridBarrierFloor: microseconds per barrier of `barriers` (1..1e6) back-to-back
  * barriers on the same grid with no work between them, the latency floor of a phase. */
 LCS_API int GBT_FrameBarriers(unsigned* barriers);
-/* Automatic mode runs plain frames (no bends, guard, friction, perpendicular damping or blade) on spatial
- * bricks, one CTA each, that exchange halo values between groups of colours; results are the same bit for
- * bit.  GBT_SetBrickCount: about `count` bricks in the next LCS_InitPhysics's plan, 0 = the cheapest.
+/* Automatic mode runs frames without bends or perpendicular damping on spatial bricks, one CTA each, that
+ * exchange halo values between groups of colours (plain frames, blade frames with ks > 0, contact model 1,
+ * the tissue guard with one pass); results are the same bit for bit.  GBT_SetBrickCount: about `count`
+ * bricks in the next LCS_InitPhysics's plan, 0 = one per SM (one in all for a few hundred nodes).
  * GBT_BrickInfo: bricks (0: no plan fits), exchanges a substep, threads a CTA, nodes of the largest brick.
- * After a brick frame GBT_FrameBarriers reports the exchanges it ran. */
+ * After a plain brick frame GBT_FrameBarriers reports the exchanges it ran. */
 LCS_API int GBT_SetBrickCount(int count);
 LCS_API int GBT_BrickInfo(int* out4);
 LCS_API int GBT_GridBarrierFloor(int barriers, float* usPerBarrier);
@@ -293,9 +294,10 @@ LCS_API int GBT_DiffInfo(int* out4);   /* grid launch (1) or one CTA (0), CTAs, 
 LCS_API void GBT_DiffEnd(void);
 
 /* LCS_StepNoAlloc has no counterpart in the reference.  It advances the session by one frame
- * exactly as LCS_Step does, in the launch shape LCS_Step would pick (automatic mode: the shape its
- * timed trials kept, or before them one CTA where the nodes fit its shared memory, else the whole
- * GPU; it runs no trials itself), for hosts that cannot let a plugin allocate GPU memory while they
+ * exactly as LCS_Step does, in the launch shape LCS_Step would pick (automatic mode: bricks where
+ * LCS_Step uses them, with the tables made by LCS_InitPhysics; else the shape its timed trials kept, or
+ * before them one CTA where the nodes fit its shared memory, else the whole GPU; it runs no trials
+ * itself), for hosts that cannot let a plugin allocate GPU memory while they
  * run (engines that own every device allocation through their own pool or budget, and real-time
  * loops where an allocation, which may synchronise the device, would stall a frame).  It calls no
  * cudaMalloc, cudaFree or other allocating routine: the frame's scratch (barrier counter, status,
