@@ -1,4 +1,6 @@
 // One frame of a single mesh on spatial bricks (brick_frame.cuh), and the upkeep of a plan's tables.
+#include <type_traits>
+
 #include "brick_kernels.h"
 #include "contact_point.cuh"
 #include "friction_contact.cuh"
@@ -296,19 +298,9 @@ BrickFrameKernel brickFrameKernelFor(bool damped, bool cut, bool extended, int t
     return threads <= kNarrowThreads ? frameKernelFor<kNarrowThreads>(damped, cut, extended) : frameKernelFor<kBrickThreads>(damped, cut, extended);
 }
 
-template <class T> cudaError_t BrickBuffers::put(T** to, const T* from, size_t count, cudaStream_t stream) {
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, (count ? count : 1) * sizeof(T));
-    if (e != cudaSuccess) return e;
-    memory_[held_++] = p;
-    *to = (T*)p;
-    if (!count) return cudaSuccess;
-    return from ? cudaMemcpyAsync(p, from, count * sizeof(T), cudaMemcpyHostToDevice, stream) : cudaMemsetAsync(p, 0, count * sizeof(T), stream);
-}
-
 void BrickBuffers::release() {
-    for (int i = 0; i < held_; i++) cudaFree(memory_[i]);
-    held_ = 0;
+    if (memory_) cudaFree(memory_);
+    memory_ = nullptr;
     t = BrickTables{};
     tets = edges = 0;
 }
@@ -322,23 +314,44 @@ cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int 
     BrickTables q{};
     q.shape = plan.shape();
     q.maxLocal = plan.maxLocal; q.maxOwned = plan.maxOwned; q.nIdle = (int)plan.idle.size(); q.N = N;
-    cudaError_t e = put((BrickDesc**)&q.desc, plan.desc.data(), plan.desc.size(), stream);
-    if (e == cudaSuccess) e = put((int**)&q.head, plan.head.data(), plan.head.size(), stream);
-    if (e == cudaSuccess) e = put((int**)&q.localNode, plan.localNode.data(), plan.localNode.size(), stream);
-    if (e == cudaSuccess) e = put((int**)&q.idle, plan.idle.data(), plan.idle.size(), stream);
-    if (e == cudaSuccess) e = put((int2**)&q.importList, plan.importList.data(), plan.importList.size(), stream);
-    if (e == cudaSuccess) e = put((int2**)&q.exportList, plan.exportList.data(), plan.exportList.size(), stream);
-    if (e == cudaSuccess) e = put((unsigned long long**)&q.tetWord, (const unsigned long long*)plan.tetWord.data(), plan.tetWord.size(), stream);
-    if (e == cudaSuccess) e = put((float2**)&q.tetAlpha, (const float2*)nullptr, plan.tetWord.size(), stream);
-    if (e == cudaSuccess) e = put((unsigned**)&q.edgeWord, plan.edgeWord.data(), plan.edgeWord.size(), stream);
-    if (e == cudaSuccess) e = put((float**)&q.edgeRest, plan.edgeRest.data(), plan.edgeRest.size(), stream);
-    if (e == cudaSuccess) e = put(&tetSrc, plan.tetSrc.data(), plan.tetSrc.size(), stream);
-    if (e == cudaSuccess) e = put(&edgeSrc, plan.edgeSrc.data(), plan.edgeSrc.size(), stream);
-    if (e == cudaSuccess) e = put((int**)&q.ownTet, plan.ownTet.data(), plan.ownTet.size(), stream);
+    // every table in one allocation, 256-byte aligned: first pass sizes, second pass copies
     const size_t mail = plan.bricks > 1 ? 2 * (size_t)N : 0;
-    if (e == cudaSuccess) e = put(&q.mail, (const float4*)nullptr, mail, stream);
-    if (e == cudaSuccess) e = put(&q.mailStart, (const float4*)nullptr, damped ? mail : 0, stream);
-    if (e == cudaSuccess) e = put(&q.epoch, (const unsigned*)nullptr, plan.bricks, stream);
+    char* base = nullptr;
+    size_t at = 0;
+    cudaError_t e = cudaSuccess;
+    auto put = [&](auto** to, const void* from, size_t count) {   // from null: zeroed
+        using T = std::remove_cv_t<std::remove_pointer_t<std::remove_pointer_t<decltype(to)>>>;
+        const size_t bytes = count * sizeof(T);
+        if (base && e == cudaSuccess) {
+            *to = (T*)(base + at);
+            if (bytes) e = from ? cudaMemcpyAsync(base + at, from, bytes, cudaMemcpyHostToDevice, stream) : cudaMemsetAsync(base + at, 0, bytes, stream);
+        }
+        at += (bytes + 255) & ~(size_t)255;
+    };
+    for (int pass = 0; pass < 2; pass++) {
+        at = 0;
+        put(&q.desc, plan.desc.data(), plan.desc.size());
+        put(&q.head, plan.head.data(), plan.head.size());
+        put(&q.localNode, plan.localNode.data(), plan.localNode.size());
+        put(&q.idle, plan.idle.data(), plan.idle.size());
+        put(&q.importList, plan.importList.data(), plan.importList.size());
+        put(&q.exportList, plan.exportList.data(), plan.exportList.size());
+        put(&q.tetWord, plan.tetWord.data(), plan.tetWord.size());
+        put(&q.edgeWord, plan.edgeWord.data(), plan.edgeWord.size());
+        put(&q.edgeRest, plan.edgeRest.data(), plan.edgeRest.size());
+        put(&tetSrc, plan.tetSrc.data(), plan.tetSrc.size());
+        put(&edgeSrc, plan.edgeSrc.data(), plan.edgeSrc.size());
+        put(&q.ownTet, plan.ownTet.data(), plan.ownTet.size());
+        put(&q.tetAlpha, nullptr, plan.tetWord.size());
+        put(&q.mail, nullptr, mail);
+        put(&q.mailStart, nullptr, damped ? mail : 0);
+        put(&q.epoch, nullptr, plan.bricks);
+        if (pass == 0) {
+            e = cudaMalloc(&memory_, at ? at : 1);
+            if (e != cudaSuccess) { memory_ = nullptr; return e; }
+            base = (char*)memory_;
+        }
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);   // the plan's host tables may go
     if (e != cudaSuccess) { release(); return e; }
     q.tetSrc = tetSrc; q.edgeSrc = edgeSrc;

@@ -28,8 +28,7 @@ struct BrickBuffers {
     // Compliances over h^2 of the bricks' tets from the per-tet stiffnesses.
     cudaError_t compliances(float invH2, const float2* tetStiff, cudaStream_t stream);
 private:
-    void* memory_[16] = {}; int held_ = 0;
-    template <class T> cudaError_t put(T** to, const T* from, size_t count, cudaStream_t stream);
+    void* memory_ = nullptr;   // one allocation for every table
 };
 
 // Liveness flags of every edge and tet, the edges a live tet carries (with fallback: edgeSupport must
