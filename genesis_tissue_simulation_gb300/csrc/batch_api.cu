@@ -6,7 +6,8 @@
 // greedy colourings), so a batched instance evolves bit for bit as it would alone.  The packed
 // table stores colour c of every instance together (colour-major, instances in table order), which
 // gives two ways to run a frame, picked by GBT_BatchAutotune:
-//   lockstep   all instances advance colour by colour in one cooperative grid (frameKernelLockstep);
+//   lockstep   all instances advance colour by colour in one cooperative grid (frameKernelLockstep); where
+//              their nodes fit, every instance instead has CTAs of its own (bricks, brick_batch.cu);
 //   instances  one CTA per instance at a time, longest-processing-time packing over the CTAs, with
 //              only __syncthreads between colours (frameKernelInstances<256|512>).
 // GBT_BatchStepMany advances several frames with one CUDA graph launch: the instrument frames of all

@@ -1,4 +1,5 @@
-// Persistent frame kernels of the XPBD tissue step.
+// Persistent frame kernels of the XPBD tissue step, for the launch modes that ask for them and for frames
+// that do not run on bricks (brick_kernels.cu).
 //
 // One launch advances one outer frame: every substep's predict, the graph-coloured Gauss-Seidel
 // sweeps (lattice edges, bends, tets), capsule contact, velocity update and the blade's ribbon
