@@ -11,9 +11,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
-#include <thread>
 
 #include "brick_plan.h"
+#include "host_parallel.h"
 
 namespace gbt {
 namespace {
@@ -147,6 +147,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         for (int a = 0; a < 3; a++) { lo[a] = std::min(lo[a], c[a]); hi[a] = std::max(hi[a], c[a]); }
     }
     if (served == 0) return none;
+    if ((served + maxBricks - 1) / maxBricks > maxLocal) return none;   // before anything is sized by the mesh
     const int ext[3] = {hi[0] - lo[0] + 1, hi[1] - lo[1] + 1, hi[2] - lo[2] + 1};
     Phases ph(m, reverse);
     Scratch s(m.N, std::max(E, 1), std::max(T * (1 + m.tensilePasses), 1));
@@ -204,19 +205,8 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         owned[b].push_back(i);
     }
     std::vector<std::vector<std::vector<int>>> elements(B, std::vector<std::vector<int>>(P)), imports(B, std::vector<std::vector<int>>(S));
-    // body(brick, the thread's own workspace of type W)
-    auto parallel = [&](auto&& workspace, auto&& body) {
-        const int threads = std::max(1, std::min({(int)std::thread::hardware_concurrency(), maxThreads, B, 1 + served / 200}));
-        std::atomic<int> next{0};
-        auto run = [&]() {
-            auto own = workspace();
-            for (int b; (b = next++) < B;) body(b, own);
-        };
-        std::vector<std::thread> pool;
-        for (int t = 1; t < threads; t++) pool.emplace_back(run);
-        run();
-        for (auto& t : pool) t.join();
-    };
+    // body(brick, the thread's own workspace)
+    auto parallel = [&](auto&& workspace, auto&& body) { parallelFor(B, std::min(maxThreads, 1 + served / 200), workspace, body); };
     // which bricks take values from which (rows: the reader)
     std::vector<unsigned char> reads((size_t)B * B, 0);
     parallel([&]() { return Scratch(m.N, std::max(E, 1), std::max(T * (1 + m.tensilePasses), 1)); }, [&](int b, Scratch& sc) {
