@@ -124,7 +124,7 @@ double chooseStages(const Phases& ph, const std::vector<int>& owned, Scratch& s,
 }
 
 struct Split { int a, b, c; };
-constexpr int kOneBrick = 500;
+constexpr int kOneBrick = 800;
 
 }  // namespace
 
@@ -169,9 +169,9 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
             }
         return best;
     };
-    // One brick, or one per SM: a mesh of up to ~500 nodes runs its colours as fast in one CTA without any
-    // exchange, and beyond that more CTAs were always faster (16 x 8 x 16 cells, us a substep: 60 on 1 brick,
-    // 40 on 8, 36 on 72, 35 on 102; 8 x 4 x 8 cells: 25.1 on 1, 25.7 on 81).
+    // One brick, or one per SM: a mesh of up to kOneBrick nodes runs its colours faster in one CTA without any
+    // exchange, beyond that more CTAs are faster (us a substep on one brick and on one per SM: 360 nodes 24.0
+    // and 27.7, 600 26.4 and 29.1, 847 30.0 and 29.5, 1176 34.7 and 29.2, 2601 60 and 33; 8 bricks lie between).
     const int count = forced > 0 ? std::min(forced, maxBricks) : served <= kOneBrick ? 1 : maxBricks;
     const Split split = boxes(count);
     std::vector<char> before(P, 0);
