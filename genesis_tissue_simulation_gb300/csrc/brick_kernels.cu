@@ -138,11 +138,12 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
     b.loadState(m.pos, m.vel, m.ext);
     TickState ts{Cut ? *(volatile unsigned*)cu.counters : 0u, fc.rotParity, 0u, true};
     bool havePrev = cu.havePrev != 0;
-    if (Extended && tid < 36) {   // rest lengths of the six corner-to-corner fibres of every Kuhn type
-        f3 r[3];
-        typeRows(m, tid / 6, r);
-        fibres[tid] = fibreRest(r, tid % 6);
-    }
+    if (Extended)   // rest lengths of the six corner-to-corner fibres of every Kuhn type (a CTA may have fewer threads)
+        for (int i = tid; i < 36; i += T) {
+            f3 r[3];
+            typeRows(m, i / 6, r);
+            fibres[i] = fibreRest(r, i % 6);
+        }
     b.fibres = fibres;
     for (; s < fc.substeps; s++) {
         slot = 0;
