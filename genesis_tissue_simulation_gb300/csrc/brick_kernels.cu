@@ -304,6 +304,7 @@ void BrickBuffers::release() {
     memory_ = nullptr;
     t = BrickTables{};
     tets = edges = 0;
+    current = false;
 }
 
 cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int maxBytes, cudaStream_t stream) {
@@ -369,7 +370,9 @@ cudaError_t BrickBuffers::refresh(const DeviceMesh& m, bool fallback, cudaStream
     const int n = tets > edges ? tets : edges;
     if (n) brickLiveKernel<<<(n + 255) / 256, 256, 0, stream>>>(m, edges, edgeSrc, (unsigned*)t.edgeWord, tets, tetSrc,
                                                                (unsigned long long*)t.tetWord, fallback ? 1 : 0);
-    return cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
+    current = e == cudaSuccess;
+    return e;
 }
 
 cudaError_t BrickBuffers::compliances(float invH2, const float2* tetStiff, cudaStream_t stream) {

@@ -16,6 +16,9 @@ struct BrickBuffers {
     BrickTables t{};
     int tets = 0, edges = 0, threads = kBrickThreads;
     int asked = 0;   // bricks the plan was asked for
+    // The live bits are those of the current topology: false from upload() to the first refresh(), and set
+    // false by whoever changes the topology without writing these tables' bits.
+    bool current = false;
     int* tetSrc = nullptr; int* edgeSrc = nullptr;
     // Uploads `plan` (of a mesh of N nodes) on `stream`, for CTAs of at most maxBytes shared memory;
     // frees what was there.

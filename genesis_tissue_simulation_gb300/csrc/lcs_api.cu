@@ -118,11 +118,10 @@ struct Session {
     DBuf<unsigned> floorSync;               // barrier-floor measurement: counter, status
     DBuf<int> uncovered0; bool fuseEdge0 = false;   // nodes ending no colour-0 edge; colour 0 is a matching
     bool profile = false; std::vector<cudaEvent_t> events; int profiledSteps = 0;
-    // automatic mode, plain frames: the mesh on spatial bricks (brick_frame.cuh).  bricksStale: the
-    // topology may have changed since the live bits were derived
+    // automatic mode, plain frames: the mesh on spatial bricks (brick_frame.cuh)
     BrickBuffers bricks; std::vector<int> brickIdle; unsigned long long planId = 0;
     std::vector<int2> hostEdgeEnds; std::vector<float> hostEdgeRest; std::vector<int4> hostTetIds; std::vector<int> hostTetMeta, hostActive;
-    bool bricksStale = true, bricksDamped = false; int forcedBricks = 0, maxBrickBytes = 0, maxGuardBytes = 0;
+    bool bricksDamped = false; int forcedBricks = 0, maxBrickBytes = 0, maxGuardBytes = 0;
     BrickBuffers guardBricks;   // with the tensile pass's phases (one pass), made when the guard is armed
     // section profiler (xpbd_profile_sections, xpbd_solver.cu:30-60): device time per phase kind
     bool sections = false; DBuf<unsigned long long> phaseClock; std::vector<unsigned long long> phaseHost;
@@ -158,7 +157,7 @@ void freePhysics() {
     S.edgeEnds.release(); S.edgeRest.release(); S.bendIJK.release(); S.bendPairs.release(); S.tetIds.release();
     S.tetAlpha.release(); S.tetStiff.release(); S.state.release(); S.bounds.release(); S.floorSync.release();
     S.uncovered0.release(); S.fuseEdge0 = false;
-    S.bricks.release(); S.guardBricks.release(); S.bricksStale = true;
+    S.bricks.release(); S.guardBricks.release();
     S.lastFrameBlocks = 0;
     S.fiberLambda.release(); S.feasTarget.release(); S.needed.release(); S.incOff.release(); S.incTet.release(); S.guardFlags.release();
     S.rotA.release(); S.rotB.release(); S.rotParity = 0;
@@ -367,6 +366,13 @@ BrickBuffers* brickFrames(const FrameCoeffs& fc) {
     if (!b->ready() || (fc.friction && !fc.guarded && b->sharedBytes(S.bricksDamped) > (size_t)S.maxGuardBytes)) return nullptr;
     return b;
 }
+// The topology may have changed: every plan's live bits are derived again before its next frame.
+void bricksStale() { S.bricks.current = S.guardBricks.current = false; }
+// After a frame: a blade's tick keeps the live bits of the plan it ran on (`ran`, null: another shape) and
+// no other's; an abandoned frame (status not zero) leaves all of them open.
+void noteFrame(const FrameCoeffs& fc, const BrickBuffers* ran, unsigned status) {
+    for (BrickBuffers* b : {&S.bricks, &S.guardBricks}) if ((fc.cut && b != ran) || status != 0u) b->current = false;
+}
 // The plans' compliances for the frame's substep length.
 int brickCompliances(const FrameCoeffs& fc) {
     if (!fc.doStrain || fc.h == S.brickH) return 0;
@@ -377,10 +383,9 @@ int brickCompliances(const FrameCoeffs& fc) {
 // `state`: the frame's words; hostState: their pinned copy, or null.
 int launchBricks(BrickBuffers& bricks, const FrameCoeffs& fc, unsigned* state, unsigned* hostState, bool* followUp) {
     DeviceMesh m = deviceMesh();
-    if (S.bricksStale) {
+    if (!bricks.current) {
         CK(refreshMeshFlags(m, S.E, S.T, fc.fallback != 0, S.stream));
-        for (BrickBuffers* b : {&S.bricks, &S.guardBricks}) if (b->ready()) CK(b->refresh(m, fc.fallback != 0, S.stream));
-        S.bricksStale = false;
+        CK(bricks.refresh(m, fc.fallback != 0, S.stream));
     }
     const bool extended = fc.guarded || fc.friction, damped = fc.guarded || S.bricksDamped;
     FrameCoeffs f = fc;
@@ -580,7 +585,6 @@ int planInto(BrickBuffers& bricks, const BrickMesh& mesh, bool damped, int maxBy
 }
 int planBricks(HostMesh& hm, const int* active) {
     S.bricks.release();
-    S.bricksStale = true;
     S.planId++;
     S.brickIdle.clear();
     S.bricksDamped = S.strainDamping > 0.f;   // without perpendicular damping (betaS = 0) only the tets are damped
@@ -946,7 +950,7 @@ LCS_API int LCS_DetectCut() {
     q.lo = v(c.aabbMin); q.hi = v(c.aabbMax); q.ncut = v(c.ncut); q.valid = c.valid;
     detectQuadKernel<<<(n + 255) / 256, 256, 0, S.stream>>>(m, cu, q, S.rotParity ? S.rotB.p : S.rotA.p);
     severKernel<<<(n + 255) / 256, 256, 0, S.stream>>>(m, cu);
-    S.bricksStale = true;
+    bricksStale();
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(S.stream));
     return 0;
@@ -980,11 +984,11 @@ LCS_API int LCS_Step(float dt) {
         fc.phaseClock = S.phaseClock.p;
     }
     bool followUp = false;
-    const bool onBricks = brickFrames(fc) != nullptr;
+    const BrickBuffers* bricks = brickFrames(fc);
     rc = launchFrame(fc, &followUp);
     if (rc) return rc;
     if (S.profile) { CK(cudaEventRecord(e1, S.stream)); S.events.push_back(e0); S.events.push_back(e1); }
-    if (!onBricks) CK(cudaMemcpyAsync(S.hostState, S.state.p, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
+    if (!bricks) CK(cudaMemcpyAsync(S.hostState, S.state.p, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
     if (S.sections) {
         S.phaseHost.resize(records);
         CK(cudaMemcpyAsync(S.phaseHost.data(), S.phaseClock.p, records * sizeof(unsigned long long), cudaMemcpyDeviceToHost, S.stream));
@@ -1006,8 +1010,7 @@ LCS_API int LCS_Step(float dt) {
         }
     }
     if (fc.cut) S.havePrev = true;
-    if (fc.cut && !onBricks) S.bricksStale = true;   // the tick on bricks keeps their live bits itself
-    if (S.hostState[2] != 0u) S.bricksStale = true;
+    noteFrame(fc, bricks, S.hostState[2]);
     if (S.toolArmed) S.toolFrom = S.tool;
     if (S.hostState[2] != 0u) return LCS_ERR_DEVICE_TIMEOUT;
     S.rotParity = (int)((S.hostState[3] & 1u) ^ (followUp ? 1u : 0u));
@@ -1199,7 +1202,7 @@ LCS_API int GBT_SetState(const float* pos3N, const float* vel3N, const int* nbr6
     const unsigned never = ~0u;   // liveness: never derived
     CK(cudaMemcpyAsync(S.state.p, &never, sizeof(unsigned), cudaMemcpyHostToDevice, S.stream));
     S.generation = ++g_sessionGeneration;
-    S.bricksStale = true;
+    bricksStale();
     return cudaStatus(cudaStreamSynchronize(S.stream));
 }
 
@@ -1353,7 +1356,7 @@ LCS_API int LCS_StepNoAlloc(float dt) {
     CK(cudaMemcpyAsync(words, state + 2, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
     CK(cudaStreamSynchronize(S.stream));
     if (fc.cut) S.havePrev = true;
-    if ((fc.cut && !bricks) || words[0] != 0u) S.bricksStale = true;
+    noteFrame(fc, bricks, words[0]);
     if (S.toolArmed) S.toolFrom = S.tool;
     if (words[0] != 0u) return LCS_ERR_DEVICE_TIMEOUT;
     S.rotParity = (int)((words[1] & 1u) ^ (followUp ? 1u : 0u));
