@@ -105,13 +105,16 @@ int planReverse(const SessionView& v) {
     if (!(v.launchMode == 0 || v.launchMode == 3) || !v.bricks->ready()) return 0;
     const BrickTables& t = v.bricks->t;
     const int perNode = (damped(v) ? 2 : 1) * 16;
-    // the same split: the plan depends on the brick count, and the count on the nodes served
-    const BrickPlan plan = buildBrickPlan(v.brickMesh, v.smCount, v.maxBrickBytes / perNode, t.bricks == 1 ? 1 : v.bricks->asked, false, true);
-    if (!plan.ok() || plan.bricks != t.bricks || plan.maxOwned != t.maxOwned) return 0;
-    CK(D.reverse.upload(plan, v.N, damped(v), v.maxBrickBytes, v.stream));
+    CK(makeBricks(D.reverse, [&]() {
+        // the same split: the plan depends on the brick count, and the count on the nodes served
+        const BrickPlan plan = buildBrickPlan(v.brickMesh, v.smCount, v.maxBrickBytes / perNode, t.bricks == 1 ? 1 : v.bricks->asked, false, true);
+        if (!plan.ok() || plan.bricks != t.bricks || plan.maxOwned != t.maxOwned) return cudaSuccess;
+        cudaError_t e = D.brickAlpha.ensure(v.bricks->tets);
+        if (e == cudaSuccess) e = D.reverse.upload(plan, v.N, damped(v), v.maxBrickBytes, v.stream);
+        return e;
+    }));
     BrickTables f = t, r = D.reverse.t;
-    if (!backwardBytes(f, r, damped(v), v.maxBrickBytes)) { D.reverse.release(); return 0; }
-    CK(D.brickAlpha.ensure(v.bricks->tets));
+    if (!D.reverse.ready() || !backwardBytes(f, r, damped(v), v.maxBrickBytes)) { D.reverse.release(); return 0; }
     for (const void* k : {(const void*)brickForwardFor(damped(v), v.bricks->threads), (const void*)brickBackward, (const void*)brickBackwardDamped})
         CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, v.maxBrickBytes));
     D.planId = v.planId;

@@ -425,7 +425,7 @@ int planBricks(const std::vector<HostMesh>& meshes, const GbtInstanceDesc* inst,
                   hm.tetColorOff.data(), hm.tetIds.data(), hm.tetMeta.data(), 0},
                  G.nodeBase[i], edgeSlot[i].data(), tetSlot[i].data(), edgeDead[i].data(), tetDead[i].data()};
     }
-    CK(G.bricks.plan(in, G.N, G.smCount, one, G.strainDamping > 0.f, G.stream));
+    CK(makeBricks(G.bricks, [&]() { return G.bricks.plan(in, G.N, G.smCount, one, G.strainDamping > 0.f, G.stream); }));
     if (G.bricks.ready())
         CK(cudaFuncSetAttribute((const void*)G.bricks.kernel(G.strainDamping > 0.f, G.codesAvailable), cudaFuncAttributeMaxDynamicSharedMemorySize, one));
     return 0;

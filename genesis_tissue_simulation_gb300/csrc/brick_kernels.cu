@@ -299,6 +299,10 @@ BrickFrameKernel brickFrameKernelFor(bool damped, bool cut, bool extended, int t
     return threads <= kNarrowThreads ? frameKernelFor<kNarrowThreads>(damped, cut, extended) : frameKernelFor<kBrickThreads>(damped, cut, extended);
 }
 
+#ifdef GBT_DEBUG_BOUNDS
+int failBrickTables = 0;
+#endif
+
 void BrickBuffers::release() {
     if (memory_) cudaFree(memory_);
     memory_ = nullptr;
@@ -349,6 +353,9 @@ cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int 
         put(&q.mailStart, nullptr, damped ? mail : 0);
         put(&q.epoch, nullptr, plan.bricks);
         if (pass == 0) {
+#ifdef GBT_DEBUG_BOUNDS
+            if (failBrickTables > 0) { failBrickTables--; return cudaErrorMemoryAllocation; }
+#endif
             e = cudaMalloc(&memory_, at ? at : 1);
             if (e != cudaSuccess) { memory_ = nullptr; return e; }
             base = (char*)memory_;

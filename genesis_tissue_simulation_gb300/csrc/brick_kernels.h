@@ -1,5 +1,7 @@
 // Brick frame of a single mesh (brick_kernels.cu) and the device side of a brick plan.
 #pragma once
+#include <new>
+
 #include "brick_frame.cuh"
 
 namespace gbt {
@@ -21,7 +23,7 @@ struct BrickBuffers {
     bool current = false;
     int* tetSrc = nullptr; int* edgeSrc = nullptr;
     // Uploads `plan` (of a mesh of N nodes) on `stream`, for CTAs of at most maxBytes shared memory;
-    // frees what was there.
+    // frees what was there, and leaves nothing ready when it fails.
     cudaError_t upload(const BrickPlan& plan, int N, bool damped, int maxBytes, cudaStream_t stream);
     void release();
     bool ready() const { return t.bricks > 0; }
@@ -33,6 +35,22 @@ struct BrickBuffers {
 private:
     void* memory_ = nullptr;   // one allocation for every table
 };
+
+// Makes a plan and its tables by `make` (a cudaError_t function of no arguments that may throw).  Bricks are
+// a faster way to run a frame, not a condition of it: when host or device memory does not suffice the
+// buffers are empty, as for a mesh without a plan, and the call goes on without them.
+template <class Buffers, class Make> cudaError_t makeBricks(Buffers& buffers, Make&& make) {
+    cudaError_t e;
+    try { e = make(); } catch (const std::bad_alloc&) { e = cudaErrorMemoryAllocation; }
+    if (e == cudaSuccess) return e;
+    buffers.release();
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();   // the failed allocation is dealt with
+    return cudaSuccess;
+}
+#ifdef GBT_DEBUG_BOUNDS
+extern int failBrickTables;   // this many table allocations to come answer that there is no memory (tests)
+#endif
 
 // Liveness flags of every edge and tet, the edges a live tet carries (with fallback: edgeSupport must
 // be zero), and the nodes' inverse masses, from the current topology.

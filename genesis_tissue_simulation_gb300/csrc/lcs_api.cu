@@ -570,17 +570,20 @@ BrickMesh brickMesh() {
 }
 // A plan of `mesh` in CTAs of at most maxBytes shared memory; a mesh without one leaves `bricks` empty.
 int planInto(BrickBuffers& bricks, const BrickMesh& mesh, bool damped, int maxBytes, std::vector<int>* idle) {
-    bricks.release();
     // at most four records of 16 B a node, beside the offsets and instrument frames
     const int perNode = (damped ? 2 : 1) * 16, room = maxBytes - 8192;
-    for (int share = 70; share >= 40; share -= 10) {
-        const BrickPlan plan = buildBrickPlan(mesh, S.smCount, (int)((long long)room * share / 100) / perNode, S.forcedBricks, damped);
-        if (!plan.ok()) return 0;
-        if (idle) *idle = plan.idle;
-        CK(bricks.upload(plan, S.N, damped, maxBytes, S.stream));
-        if (bricks.sharedBytes(damped) <= (size_t)maxBytes) return 0;
-        bricks.release();
-    }
+    bricks.release();
+    CK(makeBricks(bricks, [&]() {
+        for (int share = 70; share >= 40; share -= 10) {
+            const BrickPlan plan = buildBrickPlan(mesh, S.smCount, (int)((long long)room * share / 100) / perNode, S.forcedBricks, damped);
+            if (!plan.ok()) return cudaSuccess;
+            if (idle) *idle = plan.idle;
+            const cudaError_t e = bricks.upload(plan, S.N, damped, maxBytes, S.stream);
+            if (e != cudaSuccess || bricks.sharedBytes(damped) <= (size_t)maxBytes) return e;
+            bricks.release();
+        }
+        return cudaSuccess;
+    }));
     return 0;
 }
 int planBricks(HostMesh& hm, const int* active) {
@@ -1407,6 +1410,19 @@ LCS_API int GBT_DebugBoundsRead(unsigned* out3) {
     return cudaStatus(cudaStreamSynchronize(S.stream));
 #else
     (void)out3;
+    return LCS_ERR_UNSUPPORTED;
+#endif
+}
+
+// Debug builds: the next `count` allocations of brick tables fail for want of memory (release builds:
+// LCS_ERR_UNSUPPORTED).
+LCS_API int GBT_DebugFailBrickTables(int count) {
+#ifdef GBT_DEBUG_BOUNDS
+    if (count < 0) return XPBD_ERR_BAD_ARG;
+    failBrickTables = count;
+    return 0;
+#else
+    (void)count;
     return LCS_ERR_UNSUPPORTED;
 #endif
 }

@@ -192,6 +192,10 @@ LCS_API int GBT_SetState(const float* pos3N, const float* vel3N, const int* nbr6
  * range.  out3 = {violations, first index, first site}, cleared by the read.  Release builds:
  * LCS_ERR_UNSUPPORTED. */
 LCS_API int GBT_DebugBoundsRead(unsigned* out3);
+/* Debug builds: the next `count` allocations of brick tables answer that there is no memory; the session,
+ * guard, rollout or batch then goes on without bricks, as it does when memory runs out.  Release builds
+ * answer LCS_ERR_UNSUPPORTED. */
+LCS_API int GBT_DebugFailBrickTables(int count);
 LCS_API int GBT_BatchDebugBoundsRead(unsigned* out3);
 LCS_API int LCS_SetLaunchMode(int mode);         /* 0 automatic, 1 whole-GPU cooperative grid, 2 one CTA, 3 one thread-block cluster (plain frames) */
 /* Failure-detection test mode of the grid barrier: every barrier awaits `extraArrivals` arrivals that
