@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "brick_rollout.h"
+#include "host_parallel.h"
 #include "session_view.h"
 #include "../../include/gbtissue.h"
 
@@ -47,7 +48,7 @@ struct Diff {
     // rollouts on bricks (automatic mode, a mesh with a plan): the session's tables with compliances of
     // the rollout's own, and the reverse sweep's plan.  Made for the session plan `planId`; at session
     // generation `checked` no idle node was mobile.
-    BrickBuffers reverse; Dev<float2> brickAlpha;
+    BrickBuffers reverse; Dev<float2> brickAlpha; std::optional<Team> team;
     bool bricks = false, ranOnBricks = false; unsigned long long planId = 0, checked = ~0ull;
 };
 Diff D;
@@ -60,6 +61,7 @@ void releaseAll() {
     for (auto* b : {&D.theta, &D.path, &D.gTheta, &D.gRest, &D.gB, &D.pathPartial}) b->release();
     D.bake.release(); D.alpha.release(); D.slotStorage.release(); D.brickAlpha.release(); D.reverse.release();
     D.bricks = D.ranOnBricks = false; D.checked = ~0ull;
+    D.team.reset();
     D.ready = false; D.haveForward = false;
 }
 
@@ -105,9 +107,12 @@ int planReverse(const SessionView& v) {
     if (!(v.launchMode == 0 || v.launchMode == 3) || !v.bricks->ready()) return 0;
     const BrickTables& t = v.bricks->t;
     const int perNode = (damped(v) ? 2 : 1) * 16;
+    const int forced = t.bricks == 1 ? 1 : v.bricks->asked;
+    const BriefTeam brief(D.team, planThreads(v.N, v.brickMesh.active, forced));
     CK(makeBricks(D.reverse, [&]() {
         // the same split: the plan depends on the brick count, and the count on the nodes served
-        const BrickPlan plan = buildBrickPlan(v.brickMesh, v.smCount, v.maxBrickBytes / perNode, t.bricks == 1 ? 1 : v.bricks->asked, false, true);
+        const BrickPlan plan = buildBrickPlan(v.brickMesh, v.smCount, v.maxBrickBytes / perNode, forced, false, true, brief.team);
+        brief.team.dismiss();
         if (!plan.ok() || plan.bricks != t.bricks || plan.maxOwned != t.maxOwned) return cudaSuccess;
         cudaError_t e = D.brickAlpha.ensure(v.bricks->tets);
         if (e == cudaSuccess) e = D.reverse.upload(plan, v.N, damped(v), v.maxBrickBytes, v.stream);

@@ -457,7 +457,7 @@ LCS_API int GBT_BatchInit(int count, const GbtInstanceDesc* inst, const GbtBatch
             !d.restNbr || d.bendPairCount < 0 || (d.bendPairCount > 0 && !d.bendPairs)) return XPBD_ERR_BAD_ARG;
     }
     std::vector<int> built(count, 0);
-    parallelFor(count, [&](int i) {
+    parallelFor(count, 16, [&](int i) {
         const GbtInstanceDesc& d = inst[i];
         const int n = (d.dimsX + 1) * (d.dimsY + 1) * (d.dimsZ + 1);
         std::vector<float> zeros(3 * (size_t)n, 0.f);

@@ -154,15 +154,15 @@ cudaError_t BatchBricks::plan(const std::vector<BatchBrickInstance>& in, int N, 
         // many: only the instances well above a CTA's share, and those that do not fit one, are split
         // (splitting above 1.1, 1.25 and 1.6 shares: 5.4, 5.0 and 5.5 ms)
         const double roomNodes = (double)((room - fixed) / record);
+        std::vector<int> served(count);
+        for (int i = 0; i < count; i++) served[i] = (int)std::count_if(in[i].mesh.active, in[i].mesh.active + in[i].mesh.N, [](int a) { return a != 0; });
         bool fits = false;
         double share = 1.05 * (double)all / slots;
         for (int attempt = 0; attempt < 24 && !fits; attempt++, share *= 1.1) {
             long long split = 0;
             for (int i = 0; i < count; i++) {
-                int served = 0;
-                for (int n = 0; n < in[i].mesh.N; n++) served += in[i].mesh.active[n] != 0;
                 // a brick of a split instance keeps about a third more nodes than it owns
-                const int need = served <= roomNodes ? 1 : (int)std::ceil(1.35 * served / roomNodes);
+                const int need = served[i] <= roomNodes ? 1 : (int)std::ceil(1.35 * served[i] / roomNodes);
                 bricks[i] = std::max(need, (double)tets[i] <= 1.25 * share ? 1 : (int)std::ceil((double)tets[i] / share));
                 if (bricks[i] > 1) split += bricks[i];
             }
@@ -171,9 +171,10 @@ cudaError_t BatchBricks::plan(const std::vector<BatchBrickInstance>& in, int N, 
         if (!fits) return cudaSuccess;   // not ready: the instances' nodes do not fit side by side
     }
     std::vector<BrickPlan> plans(count);
-    parallelFor(count, [&](int i) {
+    parallelFor(count, 16, [&](int i) {
+        Team team(std::min(planThreads(in[i].mesh.N, in[i].mesh.active, bricks[i]), std::max(1, 16 / count)));   // 16 threads over all instances
         for (int more = 0; more < 3 && !plans[i].ok(); more++)   // a brick whose halo does not fit: smaller ones
-            plans[i] = buildBrickPlan(in[i].mesh, bricks[i] + more, (room - fixed) / record, bricks[i] + more, damped, false, count >= 16 ? 1 : 16);
+            plans[i] = buildBrickPlan(in[i].mesh, bricks[i] + more, (room - fixed) / record, bricks[i] + more, damped, false, team);
     });
     struct Item { int id, instance; double work; bool tied; };
     std::vector<Item> items;

@@ -311,6 +311,13 @@ void BrickBuffers::release() {
     current = false;
 }
 
+size_t BrickBuffers::leastBytes(const BrickPlan& plan, bool damped) {
+    BrickTables q{};
+    q.shape = plan.shape();
+    q.maxLocal = plan.maxLocal; q.maxOwned = plan.maxOwned;
+    return Brick::bytes(q, damped);
+}
+
 cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int maxBytes, cudaStream_t stream) {
     release();
     tets = (int)plan.tetWord.size(); edges = (int)plan.edgeWord.size();

@@ -28,6 +28,7 @@ struct BrickBuffers {
     void release();
     bool ready() const { return t.bricks > 0; }
     size_t sharedBytes(bool damped) const { return Brick::bytes(t, damped); }
+    static size_t leastBytes(const BrickPlan& plan, bool damped);   // of a CTA that reads its exchange lists from device memory
     // Live bits from the mesh's flags (`flags`: edgeLive, edgeSupport with fallback, tetMeta are current).
     cudaError_t refresh(const DeviceMesh& m, bool fallback, cudaStream_t stream);
     // Compliances over h^2 of the bricks' tets from the per-tet stiffnesses.

@@ -2,6 +2,9 @@
 // and which node values it takes from its neighbours when (brick_plan.cpp, brick_frame.cuh).
 #pragma once
 #include <cstdint>
+#include <memory>
+#include <new>
+#include <utility>
 #include <vector>
 #include <cuda_runtime.h>
 
@@ -41,6 +44,14 @@ struct BrickMesh {   // the coloured mesh a plan is made for; nodes on an nx * n
     int tensilePasses = 0;                                          // sweeps over the tet colours after the projection's
 };
 
+// A table that is sized without being filled first (its makers write every entry, each thread its own pages).
+template <class T> struct Unfilled : std::allocator<T> {
+    template <class U> struct rebind { using other = Unfilled<U>; };
+    template <class U> void construct(U* p) { ::new ((void*)p) U; }
+    template <class U, class A, class... Rest> void construct(U* p, A&& a, Rest&&... rest) { ::new ((void*)p) U(std::forward<A>(a), std::forward<Rest>(rest)...); }
+};
+template <class T> using PlanTable = std::vector<T, Unfilled<T>>;
+
 struct BrickPlan {
     int bricks = 0, stages = 1, nEdgeColors = 0, nTetColors = 0, maxLocal = 0, maxOwned = 0, maxList = 0;
     int tensilePasses = 0;                 // nTetColors counts the tet colours of every pass
@@ -50,20 +61,22 @@ struct BrickPlan {
     uint64_t exchangeBefore[2] = {0, 0};   // bit p: neighbours' values are taken before phase p (edge colours, then tet colours)
     double cost = 0.;                      // model time of one substep, microseconds
     std::vector<BrickDesc> desc;
-    std::vector<int> head, localNode, idle;
-    std::vector<int2> importList, exportList;   // (local index, node)
-    std::vector<uint64_t> tetWord; std::vector<int> tetSrc, ownTet;
-    std::vector<unsigned> edgeWord; std::vector<float> edgeRest; std::vector<int> edgeSrc;
+    std::vector<int> head, idle, ownTet;
+    PlanTable<int> localNode;
+    PlanTable<int2> importList, exportList;   // (local index, node)
+    PlanTable<uint64_t> tetWord; PlanTable<int> tetSrc;
+    PlanTable<unsigned> edgeWord; PlanTable<float> edgeRest; PlanTable<int> edgeSrc;
     bool ok() const { return bricks > 0; }
     BrickShape shape() const { return {nEdgeColors, nTetColors / (1 + tensilePasses), stages, bricks, nTetColors / (1 + tensilePasses) * tensilePasses, {exchangeBefore[0], exchangeBefore[1]}}; }
 };
 
+class Team;
 // The plan of `mesh` on at most `maxBricks` CTAs that keep at most `maxLocal` nodes each; forced > 0
-// asks for about that many bricks instead of the cheapest count.  wholeHalo: the first exchange takes
-// every halo node (damped sweeps read all of them at the substep's start).  reverse: the sweep runs tet
-// colours and then edge colours from last to first.  Returns a plan without bricks when none fits.
-// At most `maxThreads` host threads.
-BrickPlan buildBrickPlan(const BrickMesh& mesh, int maxBricks, int maxLocal, int forced, bool wholeHalo, bool reverse = false,
-                         int maxThreads = 16);
+// asks for about that many bricks instead of one, or one per CTA, by the nodes served.  wholeHalo: the
+// first exchange takes every halo node (damped sweeps read all of them at the substep's start).  reverse:
+// the sweep runs tet colours and then edge colours from last to first.  Returns a plan without bricks when
+// none fits.  The loops run on `team` (planThreads: the threads worth starting for it).
+BrickPlan buildBrickPlan(const BrickMesh& mesh, int maxBricks, int maxLocal, int forced, bool wholeHalo, bool reverse, Team& team);
+int planThreads(int N, const int* active, int forced);
 
 }  // namespace gbt

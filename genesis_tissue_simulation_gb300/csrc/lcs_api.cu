@@ -18,6 +18,7 @@
 
 #include "brick_kernels.h"
 #include "frame_kernels.h"
+#include "host_parallel.h"
 #include "mesh_build.h"
 #include "session_view.h"
 #include "surface.h"
@@ -122,6 +123,7 @@ struct Session {
     BrickBuffers bricks; std::vector<int> brickIdle; unsigned long long planId = 0;
     std::vector<int2> hostEdgeEnds; std::vector<float> hostEdgeRest; std::vector<int4> hostTetIds; std::vector<int> hostTetMeta, hostActive;
     bool bricksDamped = false; int forcedBricks = 0, maxBrickBytes = 0, maxGuardBytes = 0;
+    std::optional<Team> team;   // of the last plan (dismissed)
     BrickBuffers guardBricks;   // with the tensile pass's phases (one pass), made when the guard is armed
     // section profiler (xpbd_profile_sections, xpbd_solver.cu:30-60): device time per phase kind
     bool sections = false; DBuf<unsigned long long> phaseClock; std::vector<unsigned long long> phaseHost;
@@ -149,6 +151,7 @@ void freeCut() {
     S.cutReady = false; S.toolSet = false; S.havePrev = false;
 }
 void freePhysics() {
+    S.team.reset();
     freeCut();
     releaseCutTopology();
     for (auto* b : {&S.prev, &S.vel, &S.ext}) b->release();
@@ -158,6 +161,7 @@ void freePhysics() {
     S.tetAlpha.release(); S.tetStiff.release(); S.state.release(); S.bounds.release(); S.floorSync.release();
     S.uncovered0.release(); S.fuseEdge0 = false;
     S.bricks.release(); S.guardBricks.release();
+    S.hostEdgeEnds.clear(); S.hostEdgeRest.clear(); S.hostTetIds.clear(); S.hostTetMeta.clear(); S.hostActive.clear();
     S.lastFrameBlocks = 0;
     S.fiberLambda.release(); S.feasTarget.release(); S.needed.release(); S.incOff.release(); S.incTet.release(); S.guardFlags.release();
     S.rotA.release(); S.rotB.release(); S.rotParity = 0;
@@ -569,31 +573,35 @@ BrickMesh brickMesh() {
             S.edgeColorOff.data(), S.hostEdgeEnds.data(), S.hostEdgeRest.data(), S.tetColorOff.data(), S.hostTetIds.data(), S.hostTetMeta.data(), 0};
 }
 // A plan of `mesh` in CTAs of at most maxBytes shared memory; a mesh without one leaves `bricks` empty.
-int planInto(BrickBuffers& bricks, const BrickMesh& mesh, bool damped, int maxBytes, std::vector<int>* idle) {
+int planInto(BrickBuffers& bricks, const BrickMesh& mesh, bool damped, int maxBytes, std::vector<int>* idle, Team& team) {
     // at most four records of 16 B a node, beside the offsets and instrument frames
     const int perNode = (damped ? 2 : 1) * 16, room = maxBytes - 8192;
     bricks.release();
     CK(makeBricks(bricks, [&]() {
         for (int share = 70; share >= 40; share -= 10) {
-            const BrickPlan plan = buildBrickPlan(mesh, S.smCount, (int)((long long)room * share / 100) / perNode, S.forcedBricks, damped);
+            const BrickPlan plan = buildBrickPlan(mesh, S.smCount, (int)((long long)room * share / 100) / perNode, S.forcedBricks, damped, false, team);
             if (!plan.ok()) return cudaSuccess;
+            if (BrickBuffers::leastBytes(plan, damped) > (size_t)maxBytes) continue;
+            team.dismiss();
             if (idle) *idle = plan.idle;
-            const cudaError_t e = bricks.upload(plan, S.N, damped, maxBytes, S.stream);
-            if (e != cudaSuccess || bricks.sharedBytes(damped) <= (size_t)maxBytes) return e;
-            bricks.release();
+            return bricks.upload(plan, S.N, damped, maxBytes, S.stream);
         }
         return cudaSuccess;
     }));
     return 0;
 }
-int planBricks(HostMesh& hm, const int* active) {
+// Whether any frame of the session could run on bricks (brickFrames): bends and perpendicular damping are
+// the session's for good, and a session that has them does not wait for a plan when it opens.
+bool bricksServe() { return !(S.B > 0 && S.kb > 0.f) && !(S.betaS > 0.f); }
+int planBricks(HostMesh& hm, const int* active, Team& team) {
     S.bricks.release();
     S.planId++;
     S.brickIdle.clear();
+    if (!bricksServe()) return 0;
     S.bricksDamped = S.strainDamping > 0.f;   // without perpendicular damping (betaS = 0) only the tets are damped
     S.hostEdgeEnds.swap(hm.edgeEnds); S.hostEdgeRest.swap(hm.edgeRest); S.hostTetIds.swap(hm.tetIds); S.hostTetMeta.swap(hm.tetMeta);
     S.hostActive.assign(active, active + S.N);
-    return planInto(S.bricks, brickMesh(), S.bricksDamped, S.maxBrickBytes, &S.brickIdle);
+    return planInto(S.bricks, brickMesh(), S.bricksDamped, S.maxBrickBytes, &S.brickIdle, team);
 }
 
 }  // namespace
@@ -659,6 +667,8 @@ LCS_API int LCS_InitPhysics(const PhysicsInitDesc* desc, const float* mass, cons
     MeshInput in{S.dx, S.dy, S.dz, S.hostRest.data(), mass, pinned, active, extForce, nbrIdx, restNbr, bendPairs, bpc,
                  S.youngE, S.poisson};
     HostMesh hm;
+    const bool mayServe = !(S.betaS > 0.f) && !(S.kb > 0.f && bpc > 0);
+    const BriefTeam brief(S.team, mayServe ? planThreads(cc, active, S.forcedBricks) : 1);   // its threads start while the mesh is built
     int rc = buildHostMesh(in, hm);
     if (rc) return rc;
     const int E = hm.E, B = hm.B, T = hm.T;
@@ -731,7 +741,7 @@ LCS_API int LCS_InitPhysics(const PhysicsInitDesc* desc, const float* mass, cons
     CK(cudaMemsetAsync(S.bounds.p, 0, 3 * sizeof(unsigned), S.stream));
 #endif
     CK(cudaStreamSynchronize(S.stream));
-    rc = planBricks(hm, active);
+    rc = planBricks(hm, active, brief.team);
     if (rc) return rc;
     S.generation = ++g_sessionGeneration;
     S.physReady = true;
@@ -809,6 +819,8 @@ LCS_API int LCS_SetTissueGuard(float minimum, int passes, int count, const int* 
     (void)capture;
     if (!S.physReady || S.lastH > 0 || !std::isfinite(minimum) || minimum < 0 || minimum > .95f || passes < 0 || passes > 4 ||
         count != S.N || !inside) return XPBD_ERR_BAD_ARG;
+    const bool plans = passes == 1 && S.T > 0 && bricksServe();   // more passes carry multipliers from one to the next
+    const BriefTeam brief(S.team, plans ? planThreads(S.N, S.hostActive.data(), S.forcedBricks) : 1);
     // incident colour slots of every node (the feasibility line search reads each vertex's tets)
     std::vector<int> off(S.N + 1, 0), inc((size_t)4 * S.T);
     for (int k = 0; k < S.T; k++)
@@ -830,12 +842,10 @@ LCS_API int LCS_SetTissueGuard(float minimum, int passes, int count, const int* 
     S.minVolume = minimum;
     S.guardBricks.release();
     S.brickH = -1.f;
-    if (passes == 1 && S.T > 0) {   // more passes carry multipliers from one to the next
-        BrickMesh bm = brickMesh();
-        bm.tensilePasses = 1;
-        return planInto(S.guardBricks, bm, true, S.maxGuardBytes, nullptr);
-    }
-    return 0;
+    if (!plans) return 0;
+    BrickMesh bm = brickMesh();
+    bm.tensilePasses = 1;
+    return planInto(S.guardBricks, bm, true, S.maxGuardBytes, nullptr, brief.team);
 }
 LCS_API int LCS_SetTissueMaterial(float strength, float bulkDamping) {
     if (!S.physReady || S.lastH > 0 || !std::isfinite(strength) || strength < 0 || strength > 1000 || !std::isfinite(bulkDamping) ||
