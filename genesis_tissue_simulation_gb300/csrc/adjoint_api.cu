@@ -144,6 +144,7 @@ int useBricks(const SessionView& v, bool* yes) {
 int launchBricks(const SessionView& v, bool backward, DeviceMesh m, DiffBuffers b) {
     BrickTables f = v.bricks->t, r = D.reverse.t;
     f.tetAlpha = D.brickAlpha.p;
+    f.bounds = r.bounds = m.bounds;
     ContactParams cp = v.cp;
     DiffCoeffs dc = D.dc;
     unsigned* barrier = v.state + 1;

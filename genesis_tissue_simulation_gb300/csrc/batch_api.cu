@@ -260,6 +260,7 @@ int launchFrame(const FrameCoeffs& fc, const ContactFrame* frames) {
         attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
         ContactParams cp = G.cp;
+        G.bricks.buffers.t.bounds = m.bounds;
         CK(cudaLaunchKernelEx(&cfg, G.bricks.kernel(G.strainDamping > 0.f, G.codesAvailable), m, fc, cp, G.bricks.buffers.t,
                               (const BrickShape*)G.bricks.shapes, (const int*)G.bricks.order, (const int*)G.bricks.start,
                               G.codesAvailable ? (const float2*)G.instAlpha.p : (const float2*)nullptr, G.state.p + 2));
@@ -657,8 +658,8 @@ LCS_API int GBT_BatchInit(int count, const GbtInstanceDesc* inst, const GbtBatch
     }
     G.tool.assign(count, ToolPose{}); G.toolFrom = G.tool;
 #ifdef GBT_DEBUG_BOUNDS
-    CK(G.bounds.alloc(3));
-    CK(cudaMemsetAsync(G.bounds.p, 0, 3 * sizeof(unsigned), G.stream));
+    CK(G.bounds.alloc(kBoundsWords));
+    CK(cudaMemsetAsync(G.bounds.p, 0, kBoundsWords * sizeof(unsigned), G.stream));
 #endif
     CK(cudaStreamSynchronize(G.stream));
     G.ready = true;
@@ -875,6 +876,20 @@ LCS_API int GBT_BatchDebugBoundsRead(unsigned* out3) {
     return 0;
 #else
     (void)out3;
+    return LCS_ERR_UNSUPPORTED;
+#endif
+}
+
+// Debug builds: elements whose indices the batch's bricks have checked since the last read.
+LCS_API int GBT_BatchDebugBrickChecks(unsigned* out) {
+#ifdef GBT_DEBUG_BOUNDS
+    if (!G.ready || !out || !G.bounds.p) return XPBD_ERR_BAD_ARG;
+    CK(cudaMemcpyAsync(out, G.bounds.p + 3, sizeof(unsigned), cudaMemcpyDeviceToHost, G.stream));
+    CK(cudaMemsetAsync(G.bounds.p + 3, 0, sizeof(unsigned), G.stream));
+    CK(cudaStreamSynchronize(G.stream));
+    return 0;
+#else
+    (void)out;
     return LCS_ERR_UNSUPPORTED;
 #endif
 }

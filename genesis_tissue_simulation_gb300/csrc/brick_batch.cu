@@ -36,14 +36,13 @@ __device__ __forceinline__ void batchFrame(const DeviceMesh& m, const FrameCoeff
         if (PerType && tid < 6) typeAlpha[tid] = instAlpha[6 * instance + tid];
         Brick b(bt, shape, m.typeB, id, shared, Damped, false, shape.bricks > 1 ? fc.substeps * shape.stages : 0, status, fc.spinBudget, 0u);
         b.typeAlpha = typeAlpha;
-        const int* node = bt.localNode + b.d.nodeBase;
-        for (int i = tid; i < b.d.nLocal; i += T) b.P[i] = m.pos[node[i]];
+        for (int i = tid; i < b.d.nLocal; i += T) b.P[i] = m.pos[b.node(i)];
         // owned nodes are predicted by the thread that loaded them; immobile ones never change
         for (int i = tid; i < b.d.nOwned; i += T) {
             const float4 P = b.P[i];
             if (Damped) b.Q[i] = P;
             if (!(P.w > 0.f)) continue;
-            const int n = node[i];
+            const int n = b.node(i);
             const float4 F = m.ext[n];
             m.prev[n] = make_float4(P.x, P.y, P.z, 0.f);
             const f3 v = xyz(m.vel[n]) + (mk(F.x, F.y, F.z) * P.w) * fc.h;
@@ -65,7 +64,7 @@ __device__ __forceinline__ void batchFrame(const DeviceMesh& m, const FrameCoeff
                     n[u] = -1;
                     if (i >= b.d.nOwned) continue;
                     P[u] = b.P[i];
-                    if (P[u].w > 0.f) n[u] = node[i];
+                    if (P[u].w > 0.f) n[u] = b.node(i);
                 }
 #pragma unroll
                 for (int u = 0; u < kNodes; u++)
@@ -95,7 +94,7 @@ __device__ __forceinline__ void batchFrame(const DeviceMesh& m, const FrameCoeff
         }
         for (int i = tid; i < b.d.nOwned; i += T) {
             const float4 P = b.P[i];
-            if (P.w > 0.f) m.pos[node[i]] = P;
+            if (P.w > 0.f) m.pos[b.node(i)] = P;
         }
         __syncthreads();   // shared memory passes to the next brick
     }
@@ -224,6 +223,7 @@ cudaError_t BatchBricks::plan(const std::vector<BatchBrickInstance>& in, int N, 
         sum.maxOwned = std::max(sum.maxOwned, p.maxOwned);
         sum.threads = std::max(sum.threads, p.threads);
         sum.tetWidth = std::max(sum.tetWidth, p.tetWidth);
+        sum.meshEdges += p.meshEdges; sum.meshTets += p.meshTets;
     }
     // narrow colours: CTAs of kNarrowThreads with the whole register file (brick_frame.cuh); spread instances
     // with wider ones: 384 threads of 168 registers, which hold the node pass without spilling (12 instances

@@ -44,6 +44,7 @@ struct BrickTables {
     float4* mail;                                              // [2 x N] published values
     float4* mailStart;                                         // [2 x N] published substep-start positions (damped sweeps)
     unsigned* epoch;                                           // [bricks] exchanges so far, the same in every brick
+    unsigned* bounds; int meshEdges, meshTets;                 // debug build: the gather record; colour slots of the mesh
 };
 
 __device__ __forceinline__ void publish(float4* to, f3 v, unsigned epoch) {
@@ -54,6 +55,20 @@ __device__ __forceinline__ void publish(float4* to, f3 v, unsigned epoch) {
 __device__ __forceinline__ void peek(const float4* from, unsigned long long& lo, unsigned long long& hi) {
     asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}" : "=l"(lo), "=l"(hi) : "l"(from) : "memory");
 }
+
+// Checks of one brick's exchange records in the debug build; nothing otherwise.
+#ifdef GBT_DEBUG_BOUNDS
+struct ListCheck {
+    unsigned* rec; int nOwned, nLocal, N;
+    __device__ int2 given(int2 e) const { return make_int2(checkRange(rec, e.x, 0, nOwned, kSiteBrickList), checkRange(rec, e.y, 0, N, kSiteBrickList)); }
+    __device__ int2 taken(int2 e) const { return make_int2(checkRange(rec, e.x, nOwned, nLocal - nOwned, kSiteBrickList), checkRange(rec, e.y, 0, N, kSiteBrickList)); }
+};
+#else
+struct ListCheck {
+    __device__ __forceinline__ int2 given(int2 e) const { return e; }
+    __device__ __forceinline__ int2 taken(int2 e) const { return e; }
+};
+#endif
 
 // One thread's records e[0 .. count) of an exchange, all polled together until each has its epoch.
 constexpr int kTake = 4;
@@ -88,11 +103,11 @@ __device__ __forceinline__ bool take(const float4* from, const int2 (&e)[kTake],
 constexpr int kFlight = 1100;
 static __device__ __noinline__ bool exchangeRecords(float4* box, float4* boxStart, float4* P, float4* Q, const int2* exports, int nExports,
                                                     const int2* imports, int nImports, unsigned epoch, unsigned lag, unsigned* status,
-                                                    long long budget) {
+                                                    long long budget, ListCheck check) {
     const int T = blockDim.x, tid = threadIdx.x;
     const long long start = clock64();
     for (int i = tid; i < nExports; i += T) {
-        const int2 e = exports[i];
+        const int2 e = check.given(exports[i]);
         publish(box + e.y, xyz(P[e.x]), epoch);
         if (boxStart) publish(boxStart + e.y, xyz(Q[e.x]), epoch);
     }
@@ -102,7 +117,7 @@ static __device__ __noinline__ bool exchangeRecords(float4* box, float4* boxStar
         int2 e[kTake];
         unsigned mine = 0u;
 #pragma unroll
-        for (int u = 0; u < kTake; u++) if (i + u * T < nImports) { e[u] = imports[i + u * T]; mine |= 1u << u; }
+        for (int u = 0; u < kTake; u++) if (i + u * T < nImports) { e[u] = check.taken(imports[i + u * T]); mine |= 1u << u; }
         bad = !take(box, e, mine, epoch + lag, status, budget, [&](int at, f3 v) { float4& p = P[at]; p.x = v.x; p.y = v.y; p.z = v.z; }) || bad;
         if (boxStart) bad = !take(boxStart, e, mine, epoch + lag, status, budget, [&](int at, f3 v) { Q[at] = make_float4(v.x, v.y, v.z, 0.f); }) || bad;
     }
@@ -172,11 +187,29 @@ struct Brick {
         if (s.bricks > 1 && threadIdx.x == 0) t.epoch[b] = epoch + (unsigned)exchanges;   // also when a wait runs out
     }
 
+    // Node of a local index, and the local nodes of an element's word.
+    __device__ __forceinline__ int node(int l) const { return checkRange(bt.bounds, bt.localNode[d.nodeBase + l], 0, bt.N, kSiteBrickNode); }
+    __device__ __forceinline__ int local(unsigned bits) const { return checkRange(bt.bounds, (int)(bits & kBrickNodeMask), 0, d.nLocal, kSiteBrickLocal); }
+    __device__ __forceinline__ void tetNodes(unsigned long long word, int (&id)[4]) const {
+        const unsigned lo = (unsigned)word, hi = (unsigned)(word >> 28);
+        id[0] = local(lo); id[1] = local(lo >> kBrickNodeBits); id[2] = local(hi); id[3] = local(hi >> kBrickNodeBits);
+    }
+    static __device__ __forceinline__ int tetType(unsigned long long word) { return (int)((unsigned)(word >> 56) & 7u); }
+    __device__ __forceinline__ int edgeSlot(int k) const { return checkRange(bt.bounds, bt.edgeSrc[k], 0, bt.meshEdges, kSiteBrickSource); }
+    __device__ __forceinline__ int tetSlot(int k) const { return checkRange(bt.bounds, bt.tetSrc[k], 0, bt.meshTets, kSiteBrickSource); }
+    __device__ __forceinline__ ListCheck listCheck() const {
+#ifdef GBT_DEBUG_BOUNDS
+        return {bt.bounds, d.nOwned, d.nLocal, bt.N};
+#else
+        return {};
+#endif
+    }
+
     // The positions of owned and halo nodes, and the owned nodes' accelerations and velocities.
     __device__ __forceinline__ void loadState(const float4* pos, const float4* vel, const float4* ext) {
-        for (int i = threadIdx.x; i < d.nLocal; i += blockDim.x) P[i] = pos[bt.localNode[d.nodeBase + i]];
+        for (int i = threadIdx.x; i < d.nLocal; i += blockDim.x) P[i] = pos[node(i)];
         for (int i = threadIdx.x; i < d.nOwned; i += blockDim.x) {
-            const int n = bt.localNode[d.nodeBase + i];
+            const int n = node(i);
             const float4 F = ext[n];
             const f3 a = mk(F.x, F.y, F.z) * pos[n].w;
             A[i] = make_float4(a.x, a.y, a.z, 0.f);
@@ -192,7 +225,7 @@ struct Brick {
         const int oe = expOff[st], ne = expOff[st + 1] - oe, oi = impOff[st], ni = impOff[st + 1] - oi;
         return exchangeRecords(bt.mail + box, withStart ? bt.mailStart + box : nullptr, P, Q,
                                bt.listsShared ? exports + (oe - expOff[0]) : bt.exportList + oe, ne,
-                               bt.listsShared ? imports + (oi - impOff[0]) : bt.importList + oi, ni, epoch, lag, status, budget);
+                               bt.listsShared ? imports + (oi - impOff[0]) : bt.importList + oi, ni, epoch, lag, status, budget, listCheck());
     }
 
     __device__ __forceinline__ bool exchangeAt(int p) const { return (s.before[p >> 6] >> (p & 63)) & 1ull; }
@@ -208,14 +241,14 @@ struct Brick {
     template <bool Damped, bool Record>
     __device__ __forceinline__ void edge(const BrickEdge& w, const FrameCoeffs& fc, int k, const BrickTape& tape) {
         if (!(w.word & kBrickEdgeLive)) return;
-        const int a = w.word & kBrickNodeMask, b = (w.word >> kBrickNodeBits) & kBrickNodeMask;
+        const int a = local(w.word), b = local(w.word >> kBrickNodeBits);
         EdgeRecord r;
         r.live = 1; r.rest = w.rest;
         if (Damped) { r.qi = xyz(Q[a]); r.qj = xyz(Q[b]); } else r.qi = r.qj = mk(0.f, 0.f, 0.f);
         float4 oa, ob;
         const float4 pa = P[a], pb = P[b];
         if (Record && (w.word & kBrickEdgeOwner)) {
-            float4* t = tape.edge + 2 * (size_t)bt.edgeSrc[k];
+            float4* t = tape.edge + 2 * (size_t)edgeSlot(k);
             t[0] = pa; t[1] = pb;
         }
         if (solveEdge(r, fc, pa, pb, oa, ob)) { P[a] = oa; P[b] = ob; }
@@ -224,18 +257,18 @@ struct Brick {
     template <bool Damped, bool Record, bool PerType, bool Guarded>
     __device__ __forceinline__ void tet(const BrickTet& w, const FrameCoeffs& fc, int k, const BrickTape& tape) {
         if (!(w.word & kBrickTetLive)) return;
-        const unsigned lo = (unsigned)w.word, hi = (unsigned)(w.word >> 28);
-        const int id[4] = {(int)(lo & kBrickNodeMask), (int)((lo >> kBrickNodeBits) & kBrickNodeMask), (int)(hi & kBrickNodeMask),
-                           (int)((hi >> kBrickNodeBits) & kBrickNodeMask)};
+        int id[4];
+        tetNodes(w.word, id);
+        const int type = tetType(w.word);
         const float4 p[4] = {P[id[0]], P[id[1]], P[id[2]], P[id[3]]};
         if (Record && (w.word & kBrickTetOwner)) {
-            float4* t = tape.tet + 4 * (size_t)bt.tetSrc[k];
+            float4* t = tape.tet + 4 * (size_t)tetSlot(k);
             t[0] = p[0]; t[1] = p[1]; t[2] = p[2]; t[3] = p[3];
         }
         f3 q[4], o[4];
 #pragma unroll
         for (int c = 0; c < 4; c++) q[c] = Damped ? xyz(Q[id[c]]) : mk(0.f, 0.f, 0.f);
-        if (!solveTet(typeB + 9 * ((hi >> 28) & 7u), p, q, PerType ? typeAlpha[(hi >> 28) & 7u] : w.alpha, fc, Damped && tetDamped(fc, Guarded && fc.guarded != 0), Guarded && fc.guarded != 0, o)) return;
+        if (!solveTet(typeB + 9 * type, p, q, PerType ? typeAlpha[type] : w.alpha, fc, Damped && tetDamped(fc, Guarded && fc.guarded != 0), Guarded && fc.guarded != 0, o)) return;
 #pragma unroll
         for (int c = 0; c < 4; c++) P[id[c]] = make_float4(o[c].x, o[c].y, o[c].z, p[c].w);
     }
@@ -243,14 +276,14 @@ struct Brick {
     // Tensile reinforcement of one tet (one pass: its multipliers start at zero).
     __device__ __forceinline__ void tensile(const BrickTet& w, const FrameCoeffs& fc) {
         if (!(w.word & kBrickTetLive) || !(fc.tensileStrength > 0.f)) return;
-        const unsigned lo = (unsigned)w.word, hi = (unsigned)(w.word >> 28);
-        const int id[4] = {(int)(lo & kBrickNodeMask), (int)((lo >> kBrickNodeBits) & kBrickNodeMask), (int)(hi & kBrickNodeMask),
-                           (int)((hi >> kBrickNodeBits) & kBrickNodeMask)};
+        int id[4];
+        tetNodes(w.word, id);
+        const int type = tetType(w.word);
         const float4 q[4] = {P[id[0]], P[id[1]], P[id[2]], P[id[3]]};
         f3 p[4] = {xyz(q[0]), xyz(q[1]), xyz(q[2]), xyz(q[3])};
         float rest[6], lambda[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int f = 0; f < 6; f++) rest[f] = fibres[6 * ((hi >> 28) & 7u) + f];
+        for (int f = 0; f < 6; f++) rest[f] = fibres[6 * type + f];
         solveTensile(rest, q, w.alpha.x / fmaxf(fc.tensileStrength, 1e-10f), lambda, p);
 #pragma unroll
         for (int c = 0; c < 4; c++) P[id[c]] = make_float4(p[c].x, p[c].y, p[c].z, q[c].w);
@@ -260,13 +293,13 @@ struct Brick {
     __device__ __forceinline__ bool belowMinimum(float minimum) const {
         bool below = false;
         for (int k = threadIdx.x; k < d.nOwn; k += blockDim.x) {
-            const unsigned long long w = bt.tetWord[bt.ownTet[d.ownFirst + k]];
+            const unsigned long long w = bt.tetWord[checkRange(bt.bounds, bt.ownTet[d.ownFirst + k], tetOff[0], tetOff[s.nT] - tetOff[0], kSiteBrickSource)];
             if (!(w & kBrickTetLive)) continue;
-            const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 28);
-            const float* B = typeB + 9 * ((hi >> 28) & 7u);
+            int id[4];
+            tetNodes(w, id);
+            const float* B = typeB + 9 * tetType(w);
             const f3 b0 = mk(B[0], B[1], B[2]), b1 = mk(B[3], B[4], B[5]), b2 = mk(B[6], B[7], B[8]);
-            const f3 a = xyz(P[lo & kBrickNodeMask]), u = xyz(P[(lo >> kBrickNodeBits) & kBrickNodeMask]) - a,
-                     v = xyz(P[hi & kBrickNodeMask]) - a, x = xyz(P[(hi >> kBrickNodeBits) & kBrickNodeMask]) - a;
+            const f3 a = xyz(P[id[0]]), u = xyz(P[id[1]]) - a, v = xyz(P[id[2]]) - a, x = xyz(P[id[3]]) - a;
             const float J = dot(u, cross(v, x)) * dot(b0, cross(b1, b2));
             below = below || !isfinite(J) || J < minimum;
         }
@@ -282,6 +315,7 @@ struct Brick {
         const int T = blockDim.x, tid = threadIdx.x;
         const int nE = s.nE, nT = s.nT + (Guarded ? s.nTensile : 0);
         int st = 0;
+        countChecks(bt.bounds, edgeOff[nE] - edgeOff[0] + tetOff[nT] - tetOff[0]);
         BrickEdge nextEdge;
         BrickTet nextTet;
         if (fc.doEdges && nE > 0 && edgeOff[0] + tid < edgeOff[1]) nextEdge = edgeAt(edgeOff[0] + tid);

@@ -78,17 +78,17 @@ __device__ __noinline__ TickState ribbonTick(const DeviceMesh& m, const CutParam
         unsigned* edgeWord = (unsigned*)bt.edgeWord;
         unsigned long long* tetWord = (unsigned long long*)bt.tetWord;
         for (int k = e0 + threadIdx.x; k < e1; k += blockDim.x) {
-            const int e = bt.edgeSrc[k];
+            const int e = checkRange(bt.bounds, bt.edgeSrc[k], 0, bt.meshEdges, kSiteBrickSource);
             const int2 ij = m.edgeEnds[e];
-            const bool live = m.nbr[m.edgeOwner[e]] >= 0 && m.active[ij.x] != 0 && m.active[ij.y] != 0;
+            const bool live = m.nbr[checkSlot(m, m.edgeOwner[e], kSiteEdgeSlot)] >= 0 && m.active[ij.x] != 0 && m.active[ij.y] != 0;
             edgeWord[k] = (edgeWord[k] & ~kBrickEdgeLive) | (live ? kBrickEdgeLive : 0u);
         }
         for (int k = t0 + threadIdx.x; k < t1; k += blockDim.x) {
-            const int t = bt.tetSrc[k];
+            const int t = checkRange(bt.bounds, bt.tetSrc[k], 0, bt.meshTets, kSiteBrickSource);
             const int4 d = m.tetIds[t];
             const int* o = m.tetOwner + 3 * t;
-            const bool live = m.nbr[o[0]] >= 0 && m.nbr[o[1]] >= 0 && m.nbr[o[2]] >= 0 && m.active[d.x] != 0 && m.active[d.y] != 0 &&
-                              m.active[d.z] != 0 && m.active[d.w] != 0;
+            const bool live = m.nbr[checkSlot(m, o[0], kSiteTetSlot)] >= 0 && m.nbr[checkSlot(m, o[1], kSiteTetSlot)] >= 0 &&
+                              m.nbr[checkSlot(m, o[2], kSiteTetSlot)] >= 0 && m.active[d.x] != 0 && m.active[d.y] != 0 && m.active[d.z] != 0 && m.active[d.w] != 0;
             tetWord[k] = (tetWord[k] & ~kBrickTetLive) | (live ? kBrickTetLive : 0ull);
         }
     }
@@ -198,14 +198,14 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
             if (grid.leader()) flag[(s + 2) % 3] = 0u;   // read before this barrier, written after the next
             if (repair) {
                 for (int i = tid; i < b.d.nOwned; i += T) {
-                    const int n = bt.localNode[b.d.nodeBase + i];
+                    const int n = b.node(i);
                     m.pos[n] = b.P[i];
                     m.prev[n] = b.Q[i];
                 }
                 const GuardResult g = guardChain(m, fc, fc.firstSubstep + s + 1, state + 1, ts.target);
                 ts.target = g.target;
                 if (!g.ok) return;
-                for (int i = tid; i < b.d.nOwned; i += T) b.P[i] = m.pos[bt.localNode[b.d.nodeBase + i]];
+                for (int i = tid; i < b.d.nOwned; i += T) b.P[i] = m.pos[b.node(i)];
             }
         }
         for (int i = tid; i < b.d.nOwned; i += T) {
@@ -225,29 +225,29 @@ __device__ __forceinline__ void brickFrame(const DeviceMesh& m, const FrameCoeff
         if (Cut) {   // the first tick after the blade is set only takes the position snapshot
             if (havePrev) {
                 for (int i = tid; i < b.d.nOwned; i += T) {
-                    const int n = bt.localNode[b.d.nodeBase + i];
+                    const int n = b.node(i);
                     m.pos[n] = b.P[i];
                     m.prev[n] = b.Q[i];
                 }
-                for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode<Extended>(m, bt.idle[i], fc, from, to, cp, s, s + 1);
+                for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode<Extended>(m, checkNode(m, bt.idle[i], kSiteBrickNode), fc, from, to, cp, s, s + 1);
                 ts = ribbonTick(m, cu, bt, b.edgeOff[0], b.edgeOff[b.s.nE], b.tetOff[0], b.tetOff[b.s.nT],
                                 fc.firstSubstep + s + 1 >= fc.numSubsteps, fc.rotations != 0, state + 1, fc.spinBudget, ts);
                 if (!ts.ok) return;
                 mark(kPhaseTick);
             } else {
-                for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode<Extended>(m, bt.idle[i], fc, from, to, cp, s, s + 1);
+                for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode<Extended>(m, checkNode(m, bt.idle[i], kSiteBrickNode), fc, from, to, cp, s, s + 1);
             }
             havePrev = true;
         }
     }
     for (int i = tid; i < b.d.nOwned; i += T) {
-        const int n = bt.localNode[b.d.nodeBase + i];
+        const int n = b.node(i);
         m.pos[n] = b.P[i];
         m.prev[n] = b.Q[i];
         m.vel[n] = b.V[i];
     }
     if (!Cut)
-        for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode<Extended>(m, bt.idle[i], fc, from, to, cp, 0, fc.substeps);
+        for (int i = blockIdx.x * T + tid; i < bt.nIdle; i += gridDim.x * T) idleNode<Extended>(m, checkNode(m, bt.idle[i], kSiteBrickNode), fc, from, to, cp, 0, fc.substeps);
     if (blockIdx.x == 0 && tid == 0) {
         if (!Cut && !guarded) state[1] = (unsigned)exchanges;   // with ticks or the guard it is the grid barrier's counter, which others may still read
         state[3] = (unsigned)ts.rotParity;
@@ -265,15 +265,15 @@ __global__ void meshFlagsKernel(DeviceMesh m, int E, int T, int fallback) {
     if (i < m.nNodes) m.pos[i].w = nodeInvMass(m, i);
 }
 
-__global__ void brickLiveKernel(DeviceMesh m, int edges, const int* edgeSrc, unsigned* edgeWord, int tets, const int* tetSrc,
-                                unsigned long long* tetWord, int fallback) {
+__global__ void brickLiveKernel(DeviceMesh m, int meshEdges, int edges, const int* edgeSrc, unsigned* edgeWord, int meshTets, int tets,
+                                const int* tetSrc, unsigned long long* tetWord, int fallback) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < edges) {
-        const int e = edgeSrc[i];
+        const int e = checkRange(m.bounds, edgeSrc[i], 0, meshEdges, kSiteBrickSource);
         const bool live = m.edgeLive[e] != 0 && !(fallback && m.edgeSupport[checkSlot(m, m.edgeOwner[e], kSiteEdgeSlot)]);
         edgeWord[i] = (edgeWord[i] & ~kBrickEdgeLive) | (live ? kBrickEdgeLive : 0u);
     }
-    if (i < tets) tetWord[i] = (tetWord[i] & ~kBrickTetLive) | ((m.tetMeta[tetSrc[i]] & 8) ? kBrickTetLive : 0ull);
+    if (i < tets) tetWord[i] = (tetWord[i] & ~kBrickTetLive) | ((m.tetMeta[checkRange(m.bounds, tetSrc[i], 0, meshTets, kSiteBrickSource)] & 8) ? kBrickTetLive : 0ull);
 }
 
 __global__ void brickAlphaKernel(int tets, const int* tetSrc, float invH2, const float2* stiff, float2* alpha) {
@@ -371,6 +371,7 @@ cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int 
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);   // the plan's host tables may go
     if (e != cudaSuccess) { release(); return e; }
     q.tetSrc = tetSrc; q.edgeSrc = edgeSrc;
+    q.meshEdges = plan.meshEdges; q.meshTets = plan.meshTets;
     q.bricks = plan.bricks;
     // the exchange lists, next to the node state, when shared memory holds both
     q.maxList = plan.maxList;
@@ -382,8 +383,8 @@ cudaError_t BrickBuffers::upload(const BrickPlan& plan, int N, bool damped, int 
 
 cudaError_t BrickBuffers::refresh(const DeviceMesh& m, bool fallback, cudaStream_t stream) {
     const int n = tets > edges ? tets : edges;
-    if (n) brickLiveKernel<<<(n + 255) / 256, 256, 0, stream>>>(m, edges, edgeSrc, (unsigned*)t.edgeWord, tets, tetSrc,
-                                                               (unsigned long long*)t.tetWord, fallback ? 1 : 0);
+    if (n) brickLiveKernel<<<(n + 255) / 256, 256, 0, stream>>>(m, t.meshEdges, edges, edgeSrc, (unsigned*)t.edgeWord, t.meshTets, tets,
+                                                               tetSrc, (unsigned long long*)t.tetWord, fallback ? 1 : 0);
     const cudaError_t e = cudaGetLastError();
     current = e == cudaSuccess;
     return e;

@@ -436,6 +436,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         plan.desc[b].nOwn = (int)build[b].ownTet.size();
         plan.ownTet.insert(plan.ownTet.end(), build[b].ownTet.begin(), build[b].ownTet.end());
     }
+    plan.meshEdges = m.nEdgeColors ? m.edgeOff[m.nEdgeColors] : 0; plan.meshTets = m.nTetColors ? m.tetOff[m.nTetColors] : 0;
     plan.bricks = B; plan.asked = count; plan.stages = S; plan.nEdgeColors = m.nEdgeColors; plan.nTetColors = nT; plan.tensilePasses = m.tensilePasses; plan.cost = cost;
     for (int p = 0; p < P; p++) if (before[p] && B > 1) plan.exchangeBefore[p >> 6] |= 1ull << (p & 63);
     return plan;

@@ -57,6 +57,7 @@ struct BrickPlan {
     int tensilePasses = 0;                 // nTetColors counts the tet colours of every pass
     int asked = 0;                         // the brick count the split was chosen for
     int threads = 32;                      // of a CTA: the widest phase, in whole warps
+    int meshEdges = 0, meshTets = 0;       // colour slots the words come from
     int tetWidth = 0;                      // elements of the widest tet phase of a brick
     uint64_t exchangeBefore[2] = {0, 0};   // bit p: neighbours' values are taken before phase p (edge colours, then tet colours)
     double cost = 0.;                      // model time of one substep, microseconds

@@ -34,7 +34,7 @@ __device__ __forceinline__ bool rollSubstep(Brick& b, const FrameCoeffs& fc, con
             b.P[i] = make_float4(x.x, x.y, x.z, P.w);
         }
         if (Record) {
-            const size_t at = (size_t)j * nodes + b.bt.localNode[b.d.nodeBase + i];
+            const size_t at = (size_t)j * nodes + b.node(i);
             db.tapeQ[at] = P;
             db.tapeV[at] = V;
         }
@@ -45,7 +45,7 @@ __device__ __forceinline__ bool rollSubstep(Brick& b, const FrameCoeffs& fc, con
     if (dc.contact) cap = capsuleAt(db, dc, g, N);
     for (int i = tid; i < b.d.nOwned; i += step) {
         const float4 P = b.P[i];
-        if (Record) db.tapeX[(size_t)j * nodes + b.bt.localNode[b.d.nodeBase + i]] = P;
+        if (Record) db.tapeX[(size_t)j * nodes + b.node(i)] = P;
         f3 x = xyz(P);
         if (dc.contact) x = capsuleContact(x, P.w, xyz(b.V[i]), cap, cp);
         b.P[i] = f4(x, P.w);
@@ -74,7 +74,7 @@ __device__ __forceinline__ void forwardBricks(const DeviceMesh& m, const DiffCoe
         if (g % db.every == 0) {
             const size_t base = (size_t)(g / db.every) * m.nNodes;
             for (int i = tid; i < b.d.nOwned; i += step) {
-                const int n = bt.localNode[b.d.nodeBase + i];
+                const int n = b.node(i);
                 db.ckPos[base + n] = b.P[i];
                 db.ckVel[base + n] = b.V[i];
             }
@@ -82,13 +82,13 @@ __device__ __forceinline__ void forwardBricks(const DeviceMesh& m, const DiffCoe
         if (!rollSubstep<Damped, false>(b, fc, dc, cp, db, g, N, 0, m.nNodes, 0, 0)) return;
     }
     for (int i = tid; i < b.d.nOwned; i += step) {
-        const int n = bt.localNode[b.d.nodeBase + i];
+        const int n = b.node(i);
         m.pos[n] = b.P[i];
         m.prev[n] = make_float4(b.Q[i].x, b.Q[i].y, b.Q[i].z, 0.f);
         m.vel[n] = b.V[i];
     }
     for (int i = blockIdx.x * step + tid; i < bt.nIdle; i += gridDim.x * step) {   // idle nodes are immobile (checked by the host)
-        const int n = bt.idle[i];
+        const int n = checkNode(m, bt.idle[i], kSiteBrickNode);
         const float4 P = m.pos[n];
         m.prev[n] = make_float4(P.x, P.y, P.z, 0.f);
         m.vel[n] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -102,6 +102,7 @@ __device__ __forceinline__ bool reverseSweep(Brick& b, const DeviceMesh& m, cons
     const int tid = threadIdx.x, step = blockDim.x;
     const int nE = b.s.nE, nT = b.s.nT;
     int st = 0;
+    countChecks(b.bt.bounds, b.edgeOff[nE] - b.edgeOff[0] + b.tetOff[nT] - b.tetOff[0]);
     __syncthreads();
     if (dc.doStrain) {
         // Records two elements ahead (their tape slots), tape one ahead: neither is waited for.  Position
@@ -112,7 +113,7 @@ __device__ __forceinline__ bool reverseSweep(Brick& b, const DeviceMesh& m, cons
         auto fetch = [&]() {
             Slot s;
             s.valid = fc < nT && fk < b.tetOff[fc + 1];
-            if (s.valid) { s.t = b.tetAt<false>(fk); s.src = b.bt.tetSrc[fk]; }
+            if (s.valid) { s.t = b.tetAt<false>(fk); s.src = b.tetSlot(fk); }
             if (fc < nT) {
                 if (fk + step < b.tetOff[fc + 1]) fk += step;
                 else { fc++; if (fc < nT) fk = b.tetOff[fc] + tid; }
@@ -134,9 +135,8 @@ __device__ __forceinline__ bool reverseSweep(Brick& b, const DeviceMesh& m, cons
                 s1 = fetch();
                 if (cur.valid && (cur.t.word & kBrickTetLive)) {
                     const bool owner = (cur.t.word & kBrickTetOwner) != 0;
-                    const unsigned lo = (unsigned)cur.t.word, up = (unsigned)(cur.t.word >> 28);
-                    const int id[4] = {(int)(lo & kBrickNodeMask), (int)((lo >> kBrickNodeBits) & kBrickNodeMask), (int)(up & kBrickNodeMask),
-                                       (int)((up >> kBrickNodeBits) & kBrickNodeMask)};
+                    int id[4];
+                    b.tetNodes(cur.t.word, id);
                     int slot = 0;
                     float th0 = 0.f;
                     if (owner) { slot = db.slotStorage[cur.src]; th0 = db.gTheta[slot]; }
@@ -145,7 +145,7 @@ __device__ __forceinline__ bool reverseSweep(Brick& b, const DeviceMesh& m, cons
                     for (int n = 0; n < 4; n++) { q[n] = Damped ? xyz(b.Q[id[n]]) : xyz(P[n]); go[n] = xyz(b.P[id[n]]); }
                     TetAdjoint adj;
                     const float2 a = cur.t.alpha;
-                    tetVJP(b.typeB + 9 * ((up >> 28) & 7u), P, q, a.x, a.y, Damped ? dc.dampingOverH : 0.f, dc.omega, go, owner && db.gB != nullptr, adj);
+                    tetVJP(b.typeB + 9 * Brick::tetType(cur.t.word), P, q, a.x, a.y, Damped ? dc.dampingOverH : 0.f, dc.omega, go, owner && db.gB != nullptr, adj);
 #pragma unroll
                     for (int n = 0; n < 4; n++) {
                         b.P[id[n]] = f4(adj.gp[n], 0.f);
@@ -175,7 +175,7 @@ __device__ __forceinline__ bool reverseSweep(Brick& b, const DeviceMesh& m, cons
         for (int k = b.edgeOff[c] + tid; k < b.edgeOff[c + 1]; k += step) {
             const BrickEdge e = b.edgeAt(k);
             if (!(e.word & kBrickEdgeLive)) continue;
-            const int src = b.bt.edgeSrc[k], x = e.word & kBrickNodeMask, y = (e.word >> kBrickNodeBits) & kBrickNodeMask;
+            const int src = b.edgeSlot(k), x = b.local(e.word), y = b.local(e.word >> kBrickNodeBits);
             const float4 P0 = tape[2 * (size_t)src], P1 = tape[2 * (size_t)src + 1];
             const f3 qx = Damped ? xyz(b.Q[x]) : xyz(P0), qy = Damped ? xyz(b.Q[y]) : xyz(P1);
             const EdgeAdjoint adj = edgeVJP(P0, P1, qx, qy, e.rest, dc.alphaTilde, dc.betaGammaHS, dc.omega, xyz(b.P[x]), xyz(b.P[y]));
@@ -204,7 +204,7 @@ __device__ __forceinline__ void backwardBricks(const DeviceMesh& m, const DiffCo
     Brick v(rt, rt.shape, m.typeB, blockIdx.x, shared + Brick::bytes(bt, Damped) / sizeof(float4), Damped, true,
             rt.bricks > 1 ? db.total * rt.shape.stages : 0, barrier + 1, budget, 0u);
     for (int i = tid; i < v.d.nOwned; i += step) {
-        v.P[i] = db.gx[rt.localNode[v.d.nodeBase + i]];
+        v.P[i] = db.gx[v.node(i)];
         v.V[i] = v.A[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     const f3 zero = mk(0.f, 0.f, 0.f);
@@ -223,7 +223,7 @@ __device__ __forceinline__ void backwardBricks(const DeviceMesh& m, const DiffCo
             if (dc.contact) cap = capsuleAt(db, dc, g, N);
             float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int i = tid; i < v.d.nOwned; i += step) {   // velocity update and contact, in reverse
-                const size_t at = (size_t)j * nodes + rt.localNode[v.d.nodeBase + i];
+                const size_t at = (size_t)j * nodes + v.node(i);
                 const float w = b.P[i].w;
                 f3 gx = xyz(v.P[i]), gqv = zero;
                 if (w > 0.f) {
@@ -240,7 +240,7 @@ __device__ __forceinline__ void backwardBricks(const DeviceMesh& m, const DiffCo
                 v.A[i] = f4(gqv, 0.f);
             }
             if (Damped)
-                for (int i = tid; i < v.d.nLocal; i += step) v.Q[i] = db.tapeQ[(size_t)j * nodes + rt.localNode[v.d.nodeBase + i]];
+                for (int i = tid; i < v.d.nLocal; i += step) v.Q[i] = db.tapeQ[(size_t)j * nodes + v.node(i)];
             if (dc.contact) blockSum6(acc, db.pathPartial + ((size_t)g * gridDim.x + blockIdx.x) * 6);
             if (!reverseSweep<Damped>(v, m, dc, db, j, E, T)) return;
             for (int i = tid; i < v.d.nOwned; i += step) {   // predict: x1 = x + h v1, v1 = v + h a, prev = x
@@ -252,7 +252,7 @@ __device__ __forceinline__ void backwardBricks(const DeviceMesh& m, const DiffCo
         if (seg > 0 && !grid.sync()) return;   // every reader is done with the tape
     }
     for (int i = tid; i < v.d.nOwned; i += step) {
-        const int n = rt.localNode[v.d.nodeBase + i];
+        const int n = v.node(i);
         db.gx[n] = v.P[i];
         db.gv[n] = v.V[i];
         db.gq[n] = v.A[i];

@@ -398,6 +398,7 @@ int launchBricks(BrickBuffers& bricks, const FrameCoeffs& fc, unsigned* state, u
     CutParams cu = cutParams();
     if (fc.cut && S.brickCount.p) CK(cudaMemsetAsync(S.brickCount.p, 0, sizeof(unsigned), S.stream));
     if (fc.guarded) CK(cudaMemsetAsync(S.guardFlags.p, 0, 5 * sizeof(unsigned), S.stream));
+    bricks.t.bounds = m.bounds;
     void* args[] = {&m, &f, &from, &to, &cp, &bricks.t, &cu, &state};
     CK(cudaLaunchCooperativeKernel((const void*)brickFrameKernelFor(damped, fc.cut != 0, extended, bricks.threads), dim3(bricks.t.bricks), dim3(bricks.threads),
                                    args, bricks.sharedBytes(damped), S.stream));
@@ -737,8 +738,8 @@ LCS_API int LCS_InitPhysics(const PhysicsInitDesc* desc, const float* mass, cons
     rc = uploadFrameState();
     if (rc) return rc;
 #ifdef GBT_DEBUG_BOUNDS
-    CK(S.bounds.alloc(3));
-    CK(cudaMemsetAsync(S.bounds.p, 0, 3 * sizeof(unsigned), S.stream));
+    CK(S.bounds.alloc(kBoundsWords));
+    CK(cudaMemsetAsync(S.bounds.p, 0, kBoundsWords * sizeof(unsigned), S.stream));
 #endif
     CK(cudaStreamSynchronize(S.stream));
     rc = planBricks(hm, active, brief.team);
@@ -1424,6 +1425,18 @@ LCS_API int GBT_DebugBoundsRead(unsigned* out3) {
 #endif
 }
 
+// Debug builds: elements whose indices the session's bricks have checked since the last read.
+LCS_API int GBT_DebugBrickChecks(unsigned* out) {
+#ifdef GBT_DEBUG_BOUNDS
+    if (!S.physReady || !out || !S.bounds.p) return XPBD_ERR_BAD_ARG;
+    CK(cudaMemcpyAsync(out, S.bounds.p + 3, sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
+    CK(cudaMemsetAsync(S.bounds.p + 3, 0, sizeof(unsigned), S.stream));
+    return cudaStatus(cudaStreamSynchronize(S.stream));
+#else
+    (void)out;
+    return LCS_ERR_UNSUPPORTED;
+#endif
+}
 // Debug builds: the next `count` allocations of brick tables fail for want of memory (release builds:
 // LCS_ERR_UNSUPPORTED).
 LCS_API int GBT_DebugFailBrickTables(int count) {

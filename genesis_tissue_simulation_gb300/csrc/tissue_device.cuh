@@ -111,7 +111,10 @@ constexpr unsigned kCodeLive = 1u << 18;
 // an element's node index outside the nodes the kernel serves, or a neighbour-table slot outside
 // the table, is recorded in m.bounds and replaced by a valid index so the access stays in range.
 // Release builds compile both to the index itself.
-enum BoundsSite : unsigned { kSiteEdge = 1, kSiteBend = 2, kSiteTet = 3, kSiteEdgeSlot = 4, kSiteTetSlot = 5, kSiteNeighbour = 6 };
+// The record: violations, the first bad index, its site, elements the bricks have checked.
+enum BoundsSite : unsigned { kSiteEdge = 1, kSiteBend = 2, kSiteTet = 3, kSiteEdgeSlot = 4, kSiteTetSlot = 5, kSiteNeighbour = 6,
+                             kSiteBrickLocal = 7, kSiteBrickNode = 8, kSiteBrickList = 9, kSiteBrickSource = 10 };
+constexpr int kBoundsWords = 4;
 __device__ __forceinline__ void recordBounds(unsigned* rec, int index, unsigned site) {
     if (!rec) return;
     if (atomicAdd(rec, 1u) == 0u) { rec[1] = (unsigned)index; rec[2] = site; }
@@ -131,6 +134,23 @@ __device__ __forceinline__ int checkSlot(const DeviceMesh& m, int s, unsigned si
     (void)m; (void)site;
 #endif
     return s;
+}
+
+// The same for an index of [first, first + n) that belongs to a brick (brick_frame.cuh).
+__device__ __forceinline__ int checkRange(unsigned* rec, int i, int first, int n, unsigned site) {
+#ifdef GBT_DEBUG_BOUNDS
+    if ((unsigned)(i - first) >= (unsigned)n) { recordBounds(rec, i, site); return first; }
+#else
+    (void)rec; (void)first; (void)n; (void)site;
+#endif
+    return i;
+}
+__device__ __forceinline__ void countChecks(unsigned* rec, int n) {
+#ifdef GBT_DEBUG_BOUNDS
+    if (rec && threadIdx.x == 0) atomicAdd(rec + 3, (unsigned)n);
+#else
+    (void)rec; (void)n;
+#endif
 }
 
 // A node's position: plain device memory, or its slot in the cluster's distributed shared memory.

@@ -188,15 +188,19 @@ LCS_API int GBT_SetState(const float* pos3N, const float* vel3N, const int* nbr6
 /* Debug builds (libgbtissue_debug.so, compiled with GBT_DEBUG_BOUNDS; the stand-in for a memory
  * checker): every element gather index (edge ends, bend nodes, tet nodes, neighbour-table owner
  * slots) is checked against the nodes the kernel serves; a violation is counted, its index and site
- * (1 edge, 2 bend, 3 tet, 4 edge owner slot, 5 tet owner slot) recorded and the access redirected in
- * range.  out3 = {violations, first index, first site}, cleared by the read.  Release builds:
- * LCS_ERR_UNSUPPORTED. */
+ * (1 edge, 2 bend, 3 tet, 4 edge owner slot, 5 tet owner slot; of the bricks: 7 an element's local node,
+ * 8 a node, 9 an exchange record, 10 a colour slot) recorded and the access redirected in range.
+ * out3 = {violations, first index, first site}, cleared by the read.  Release builds: LCS_ERR_UNSUPPORTED. */
 LCS_API int GBT_DebugBoundsRead(unsigned* out3);
 /* Debug builds: the next `count` allocations of brick tables answer that there is no memory; the session,
  * guard, rollout or batch then goes on without bricks, as it does when memory runs out.  Release builds
  * answer LCS_ERR_UNSUPPORTED. */
 LCS_API int GBT_DebugFailBrickTables(int count);
 LCS_API int GBT_BatchDebugBoundsRead(unsigned* out3);
+/* Debug builds: elements whose indices the bricks of the session (its rollouts included) or the batch have
+ * checked since the last read; zero when no frame ran on bricks. */
+LCS_API int GBT_DebugBrickChecks(unsigned* out);
+LCS_API int GBT_BatchDebugBrickChecks(unsigned* out);
 LCS_API int LCS_SetLaunchMode(int mode);         /* 0 automatic, 1 whole-GPU cooperative grid, 2 one CTA, 3 one thread-block cluster (plain frames) */
 /* Failure-detection test mode of the grid barrier: every barrier awaits `extraArrivals` arrivals that
  * never come and gives up after `budgetSeconds` (normal budget 2 s); LCS_Step then returns -4002 and
