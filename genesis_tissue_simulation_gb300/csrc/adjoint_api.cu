@@ -49,7 +49,8 @@ struct Diff {
     // the rollout's own, and the reverse sweep's plan.  Made for the session plan `planId`; at session
     // generation `checked` no idle node was mobile.
     BrickBuffers reverse; Dev<float2> brickAlpha; std::optional<Team> team;
-    bool bricks = false, ranOnBricks = false; unsigned long long planId = 0, checked = ~0ull;
+    bool bricks = false, ranOnBricks = false; int ran[2] = {0, 0};   // bricks of the last forward and backward
+    unsigned long long planId = 0, checked = ~0ull;
 };
 Diff D;
 
@@ -60,7 +61,7 @@ void releaseAll() {
                     &D.tapeTet, &D.gx, &D.gv, &D.gq}) b->release();
     for (auto* b : {&D.theta, &D.path, &D.gTheta, &D.gRest, &D.gB, &D.pathPartial}) b->release();
     D.bake.release(); D.alpha.release(); D.slotStorage.release(); D.brickAlpha.release(); D.reverse.release();
-    D.bricks = D.ranOnBricks = false; D.checked = ~0ull;
+    D.bricks = D.ranOnBricks = false; D.ran[0] = D.ran[1] = 0; D.checked = ~0ull;
     D.team.reset();
     D.ready = false; D.haveForward = false;
 }
@@ -269,6 +270,7 @@ LCS_API int GBT_DiffForward(float dt, int frames, const float* logCompliance, co
     D.haveForward = false;
     rc = useBricks(v, &D.ranOnBricks);
     if (rc) return rc;
+    D.ran[0] = D.ranOnBricks ? v.bricks->t.bricks : 0;
     rc = D.ranOnBricks ? launchBricks(v, false, m, buffers()) : launch(v, false, m, buffers());
     if (rc) return rc;
     CK(cudaMemcpyAsync(D.finalPos.p, v.mesh.pos, D.N * sizeof(float4), cudaMemcpyDeviceToDevice, v.stream));
@@ -302,6 +304,7 @@ LCS_API int GBT_DiffBackward(const float* gradPos, float* gradLogCompliance, flo
     if (gradRestInverse) CK(cudaMemsetAsync(D.gB.p, 0, 9 * (size_t)std::max(D.T, 1) * sizeof(float), s)); else b.gB = nullptr;
     DeviceMesh m = v.mesh;
     m.tetAlpha = D.alpha.p;
+    D.ran[1] = bricks ? v.bricks->t.bricks : 0;
     rc = bricks ? launchBricks(v, true, m, b) : launch(v, true, m, b);
     if (rc) return rc;
     if (D.T) CK(cudaMemcpyAsync(gradLogCompliance, D.gTheta.p, D.T * sizeof(float), cudaMemcpyDeviceToDevice, s));
@@ -331,6 +334,13 @@ LCS_API int GBT_DiffInfo(int* out4) {
     if (!D.ready || !out4) return XPBD_ERR_NOT_READY;
     const int bricks = D.bricks ? D.reverse.t.bricks : 0;
     out4[0] = bricks ? (bricks > 1 ? 1 : 0) : (D.grid ? 1 : 0); out4[1] = bricks ? bricks : D.blocks; out4[2] = D.every; out4[3] = D.maxFrames;
+    return 0;
+}
+
+// Bricks the last forward and the last backward ran on (0: another shape).
+LCS_API int GBT_DiffBricks(int* out2) {
+    if (!D.ready || !out2) return XPBD_ERR_NOT_READY;
+    out2[0] = D.ran[0]; out2[1] = D.ran[1];
     return 0;
 }
 

@@ -64,6 +64,7 @@ struct Batch {
     // per-instance per-type stiffness and compliances; `useCodes` selects them over the explicit tables
     Buf<unsigned> tetCode, edgeCode; Buf<int4> instGeo; Buf<float2> instStiff, instAlpha;
     bool codesAvailable = false, useCodes = false;
+    int frameBricks = 0;                             // bricks the last frame ran on (0: another shape)
     BatchBricks bricks;                              // mode 0 on bricks (plain frames of a batch that fits)
     Buf<int> mobile;                                 // nodes of positive inverse mass (lockstep node passes)
     Buf<ContactFrame> frames;
@@ -102,6 +103,7 @@ void releaseAll() {
     G.codesAvailable = G.useCodes = false;
     G.mobile.release();
     G.bricks.release();
+    G.frameBricks = 0;
     if (G.framesHost) cudaFreeHost(G.framesHost);
     G.framesHost = nullptr; G.framesHostCap = 0;
     G.packedXyz.release();
@@ -253,7 +255,8 @@ void stageFrames(int steps, const ToolPose* tools, float h) {
 int launchFrame(const FrameCoeffs& fc, const ContactFrame* frames) {
     DeviceMesh m = batchMesh();
     m.contactFrames = frames;
-    if (G.mode == 0 && brickFrames(fc)) {
+    G.frameBricks = G.mode == 0 && brickFrames(fc) ? G.bricks.buffers.t.bricks : 0;
+    if (G.frameBricks > 0) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(G.bricks.ctas); cfg.blockDim = dim3(G.bricks.threads); cfg.dynamicSmemBytes = G.bricks.bytes; cfg.stream = G.stream;
         cudaLaunchAttribute attr[1];
@@ -717,6 +720,13 @@ LCS_API int GBT_BatchInfo(int* counts8) {
     if (!G.ready || !counts8) return XPBD_ERR_BAD_ARG;
     int v[8] = {G.count, G.N, G.E, G.T, G.nEdgeColors, G.nTetColors, G.mode, G.threads};
     std::memcpy(counts8, v, sizeof(v));
+    return 0;
+}
+
+// Bricks the last frame (or the captured frames the last replay ran) of the batch ran on, 0 for another shape.
+LCS_API int GBT_BatchFrameBricks(int* bricks) {
+    if (!G.ready || !bricks) return XPBD_ERR_BAD_ARG;
+    *bricks = G.frameBricks;
     return 0;
 }
 

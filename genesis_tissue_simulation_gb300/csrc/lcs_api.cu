@@ -124,6 +124,7 @@ struct Session {
     std::vector<int2> hostEdgeEnds; std::vector<float> hostEdgeRest; std::vector<int4> hostTetIds; std::vector<int> hostTetMeta, hostActive;
     bool bricksDamped = false; int forcedBricks = 0, maxBrickBytes = 0, maxGuardBytes = 0;
     std::optional<Team> team;   // of the last plan (dismissed)
+    int frameBricks = 0;        // bricks the last frame ran on (0: another shape)
     BrickBuffers guardBricks;   // with the tensile pass's phases (one pass), made when the guard is armed
     // section profiler (xpbd_profile_sections, xpbd_solver.cu:30-60): device time per phase kind
     bool sections = false; DBuf<unsigned long long> phaseClock; std::vector<unsigned long long> phaseHost;
@@ -162,7 +163,7 @@ void freePhysics() {
     S.uncovered0.release(); S.fuseEdge0 = false;
     S.bricks.release(); S.guardBricks.release();
     S.hostEdgeEnds.clear(); S.hostEdgeRest.clear(); S.hostTetIds.clear(); S.hostTetMeta.clear(); S.hostActive.clear();
-    S.lastFrameBlocks = 0;
+    S.lastFrameBlocks = 0; S.frameBricks = 0;
     S.fiberLambda.release(); S.feasTarget.release(); S.needed.release(); S.incOff.release(); S.incTet.release(); S.guardFlags.release();
     S.rotA.release(); S.rotB.release(); S.rotParity = 0;
     S.volumePasses = 0; S.minVolume = 0.f;
@@ -1024,6 +1025,7 @@ LCS_API int LCS_Step(float dt) {
         }
     }
     if (fc.cut) S.havePrev = true;
+    S.frameBricks = bricks ? bricks->t.bricks : 0;
     noteFrame(fc, bricks, S.hostState[2]);
     if (S.toolArmed) S.toolFrom = S.tool;
     if (S.hostState[2] != 0u) return LCS_ERR_DEVICE_TIMEOUT;
@@ -1287,6 +1289,13 @@ LCS_API int GBT_BrickInfo(int* out4) {
     return 0;
 }
 
+// Bricks the last frame ran on, the guard's plan included (0: it ran in another shape).
+LCS_API int GBT_FrameBricks(int* bricks) {
+    if (!S.physReady || !bricks) return XPBD_ERR_NOT_READY;
+    *bricks = S.frameBricks;
+    return 0;
+}
+
 LCS_API int LCS_SetLaunchMode(int mode) {
     if (mode < 0 || mode > 3) return XPBD_ERR_BAD_ARG;
     S.launchMode = mode;
@@ -1370,6 +1379,7 @@ LCS_API int LCS_StepNoAlloc(float dt) {
     CK(cudaMemcpyAsync(words, state + 2, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, S.stream));
     CK(cudaStreamSynchronize(S.stream));
     if (fc.cut) S.havePrev = true;
+    S.frameBricks = bricks ? bricks->t.bricks : 0;
     noteFrame(fc, bricks, words[0]);
     if (S.toolArmed) S.toolFrom = S.tool;
     if (words[0] != 0u) return LCS_ERR_DEVICE_TIMEOUT;

@@ -219,6 +219,8 @@ LCS_API int GBT_FrameBarriers(unsigned* barriers);
  * After a plain brick frame GBT_FrameBarriers reports the exchanges it ran. */
 LCS_API int GBT_SetBrickCount(int count);
 LCS_API int GBT_BrickInfo(int* out4);
+/* Bricks the last LCS_Step or LCS_StepNoAlloc frame ran on (the guard's plan included); 0: another shape. */
+LCS_API int GBT_FrameBricks(int* bricks);
 LCS_API int GBT_GridBarrierFloor(int barriers, float* usPerBarrier);
 
 /* ---- batched instances (no counterpart in the reference, which has one session per process) ----
@@ -243,6 +245,7 @@ LCS_API int GBT_BatchStep(float dt);                                   /* one fr
 LCS_API int GBT_BatchStepMany(float dt, int steps, const void* tools, int useGraph);
 LCS_API int GBT_BatchGetPositions(float* out3N);                      /* all nodes, instance after instance */
 LCS_API int GBT_BatchNodeRange(int instance, int* base, int* count);
+LCS_API int GBT_BatchFrameBricks(int* bricks);   /* bricks the last frame ran on, all instances; 0: another shape */
 LCS_API int GBT_BatchInfo(int* counts8);                               /* instances, nodes, edges, tets, edge colours, tet colours, mode, threads */
 /* Launch shape: mode 0 lockstep grid (threads 256), 1 one CTA per instance (threads 256 | 512),
  * 2 one thread-block cluster per instance list with positions in distributed shared memory
@@ -299,6 +302,7 @@ LCS_API int GBT_DiffForward(float dt, int frames, const float* logCompliance, co
 LCS_API int GBT_DiffBackward(const float* gradPos, float* gradLogCompliance, float* gradCapsulePath, float* gradRestLength,
                              float* gradRestInverse, float* gradOrigin);
 LCS_API int GBT_DiffInfo(int* out4);   /* grid launch (1) or one CTA (0), CTAs, checkpoint interval, max frames */
+LCS_API int GBT_DiffBricks(int* out2);   /* bricks the last forward and the last backward ran on (0: another shape) */
 LCS_API void GBT_DiffEnd(void);
 
 /* LCS_StepNoAlloc has no counterpart in the reference.  It advances the session by one frame
