@@ -378,6 +378,9 @@ __device__ void runFrame(const DeviceMesh& m, const FrameCoeffs& fc, const ToolP
                 f3 v = posRef<Dsm>(m, i).w > 0.f ? xyz(V) * fc.velScale : mk(0.f, 0.f, 0.f);
                 m.vel[i] = make_float4(v.x, v.y, v.z, 0.f);
             }
+            // the next predict takes its nodes in another order (by colour-0 edge, or off the mobile list), so
+            // another thread may read a velocity written here
+            if (s + 1 < fc.substeps && !sync.sync()) return;
         }
         mark(s, kPhaseVelocity);
         // -- blade ribbon tick between substeps --
@@ -410,6 +413,8 @@ __device__ void runFrame(const DeviceMesh& m, const FrameCoeffs& fc, const ToolP
                     framePass();
                     if (!sync.sync()) return;
                 }
+            } else if (s + 1 < fc.substeps && !sync.sync()) {   // no tick's barrier between this velocity pass and the next predict
+                return;
             }
             havePrev = true;
         }
