@@ -226,8 +226,9 @@ cudaError_t BatchBricks::plan(const std::vector<BatchBrickInstance>& in, int N, 
         sum.meshEdges += p.meshEdges; sum.meshTets += p.meshTets;
     }
     // narrow colours: CTAs of kNarrowThreads with the whole register file (brick_frame.cuh); spread instances
-    // with wider ones: 384 threads of 168 registers, which hold the node pass without spilling (12 instances
-    // of 8..20 cells, 4 frames: 1.56 ms, 1.73 with 512); else 512 (256 instances: 4.95 ms, 5.09 with 384)
+    // with wider ones: 384 threads of 168 registers, which hold the node pass without spilling (ms a frame of 10
+    // substeps with 384 and 512: 12 instances of 8..20 cells 0.40 and 0.44, 24 of them 0.49 and 0.53, 60 0.74 and 0.75,
+    // 152 of 8..16 1.20 and 1.20, 100 of 8..24 1.22 and 1.21); else 512 (256 instances, 2 frames: 4.95 ms, 5.09 with 384)
     bound = sum.tetWidth <= kNarrowColour ? kNarrowThreads : spread ? kSplitThreads : kBrickThreads;
     threads = std::min(bound, sum.threads);
     // CTAs: exchanging bricks first, one each, then the others by longest processing time

@@ -24,9 +24,10 @@ namespace gbt {
 
 constexpr int kBrickThreads = 512;
 // Plans whose widest tet colour has at most kNarrowColour elements a brick run in CTAs of kNarrowThreads: twice the
-// registers a thread and fewer warps at each barrier pay for the few second rounds (us a substep, 512 ->
-// 256: 23 x 13 x 19 cells, 320 wide, 34.0 -> 32.8; 32 x 16 x 32 cells, 320 wide, 39.0 -> 38.5; 64 x 32 x 48
-// cells, 896 wide, 62.1 -> 69.2).
+// registers a thread and fewer warps at each barrier pay for the few second rounds.  The line is by the widest
+// tet colour of a brick (edge colours may be twice as wide); us a frame of 20 substeps with 512 -> 256 threads:
+// 211 wide (24 x 14 x 20 cells) 700 -> 678, 291 (32 x 16 x 32) 768 -> 764, 322 (44 x 20 x 36) 869 -> 869, 341 (40 x 20 x 30)
+// 840 -> 832, 374 (48 x 24 x 36) 943 -> 982, 441 (64 x 16 x 48) 997 -> 1,097, 482 (64 x 32 x 48) 1,205 -> 1,366.
 constexpr int kNarrowThreads = 256, kNarrowColour = 320;
 constexpr int kBrickFrames = 32;   // instrument frames held in shared memory at a time
 

@@ -9,9 +9,9 @@
 // Elements near a brick's faces are projected by more than one brick, from the same values with the
 // same operations, so every brick's owned nodes end exactly as one sweep over the whole mesh leaves them.
 //
-// A session waits for its plan when it opens, so the plan is made by a few threads over the bricks, into flat
-// lists, and sorted lists come out of bitmaps (milliseconds for 16 x 8 x 16, 11 x 6 x 13 in reverse and 64 x 32
-// x 48 cells on 8 threads, first plan of a process: @P0@ with a vector and a sort per brick and colour, @P1@).
+// A session waits for its plan when it opens, so a few threads share the bricks, lists are flat, and sorted ones
+// come out of bitmaps (milliseconds on 16 threads: 16 x 8 x 16 cells 1.4, 11 x 6 x 13 in reverse 0.95, 64 x 32 x 48
+// 6.2; with a vector and a sort per brick and colour 3.3, 2.1 and 25).
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -137,9 +137,9 @@ void startWalk(Scratch& s, const int* owned, int n) {
 
 // The cheapest split of the phases into stages for a brick that owns `owned` (bricks > 1): for every
 // end of a stage one backward walk prices its starts, up to kLongest phases back (the longest stage of
-// any measured plan that paid was 9).  A walk ends where its stage no longer fits.
+// any measured plan that paid was 9).  A walk ends where its stage no longer fits; false when none does.
 constexpr int kLongest = 10;
-template <class Mine> double chooseStages(const Phases& ph, const std::vector<int>& owned, Team& team, Mine&& mine, int maxLocal, std::vector<char>& before) {
+template <class Mine> bool chooseStages(const Phases& ph, const std::vector<int>& owned, Team& team, Mine&& mine, int maxLocal, std::vector<char>& before) {
     const int P = ph.count;
     struct Price { double work; int imports; };
     std::vector<Price> price((size_t)(P + 1) * kLongest, Price{0., -1});   // [end][phases back - 1]
@@ -168,7 +168,7 @@ template <class Mine> double chooseStages(const Phases& ph, const std::vector<in
         }
     before.assign(P, 0);
     for (int e = P; e > 0; e = from[e]) before[from[e]] = 1;
-    return best[P];
+    return best[P] < 1e30;
 }
 
 struct Split { int a, b, c; };
@@ -280,14 +280,12 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
     }
     std::vector<char> before(P, 0);
     std::vector<int> stageStart;
-    double cost = 0.;
     const int mid = split.a / 2 + split.a * (split.b / 2 + split.b * (split.c / 2));   // the brick with the most halo
     if (B > 1) {
         // the brick at the middle of the grid stands for all
         const std::vector<int> owned(ownedNodes.begin() + ownedAt[mid], ownedNodes.begin() + ownedAt[mid + 1]);
         if (owned.empty() || (int)owned.size() > maxLocal) return none;
-        cost = chooseStages(ph, owned, team, mine, maxLocal, before);
-        if (cost >= 1e30) return none;
+        if (!chooseStages(ph, owned, team, mine, maxLocal, before)) return none;
     }
     before[0] = 1;
     for (int p = 0; p < P; p++) if (before[p]) stageStart.push_back(p);
@@ -437,7 +435,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         plan.ownTet.insert(plan.ownTet.end(), build[b].ownTet.begin(), build[b].ownTet.end());
     }
     plan.meshEdges = m.nEdgeColors ? m.edgeOff[m.nEdgeColors] : 0; plan.meshTets = m.nTetColors ? m.tetOff[m.nTetColors] : 0;
-    plan.bricks = B; plan.asked = count; plan.stages = S; plan.nEdgeColors = m.nEdgeColors; plan.nTetColors = nT; plan.tensilePasses = m.tensilePasses; plan.cost = cost;
+    plan.bricks = B; plan.asked = count; plan.stages = S; plan.nEdgeColors = m.nEdgeColors; plan.nTetColors = nT; plan.tensilePasses = m.tensilePasses;
     for (int p = 0; p < P; p++) if (before[p] && B > 1) plan.exchangeBefore[p >> 6] |= 1ull << (p & 63);
     return plan;
 }

@@ -60,7 +60,6 @@ struct BrickPlan {
     int meshEdges = 0, meshTets = 0;       // colour slots the words come from
     int tetWidth = 0;                      // elements of the widest tet phase of a brick
     uint64_t exchangeBefore[2] = {0, 0};   // bit p: neighbours' values are taken before phase p (edge colours, then tet colours)
-    double cost = 0.;                      // model time of one substep, microseconds
     std::vector<BrickDesc> desc;
     std::vector<int> head, idle, ownTet;
     PlanTable<int> localNode;

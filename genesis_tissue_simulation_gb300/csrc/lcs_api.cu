@@ -1275,7 +1275,7 @@ LCS_API int LCS_ProfileSectionsRead(char* text, int capacity) {
     return 0;
 }
 
-// Bricks of the next LCS_InitPhysics's plan: about `count`, or the cheapest by the model (0).
+// Bricks of the next LCS_InitPhysics's plan: about `count`, or (0) one per SM, one in all for a small mesh.
 LCS_API int GBT_SetBrickCount(int count) {
     if (count < 0) return XPBD_ERR_BAD_ARG;
     S.forcedBricks = count;
