@@ -40,6 +40,7 @@ def test_workloads_on_bricks(gpu_lib, debug_lib, name, scale, steps):  # noqa: F
     w = W.make(name, steps=steps, scale=scale)
     s = w.open(debug_lib)
     try:
+        s.dll.LCS_SetLaunchMode(0)
         w.run(s, steps=steps)
         sound(s)
         got = s.positions()
@@ -63,6 +64,7 @@ def test_damped_sessions_without_edge_stiffness_on_bricks(debug_lib, size, brick
     assert dll.GBT_SetBrickCount(bricks) == 0
     try:
         with PlainTissue(block(size), dt=1 / 60, substeps=4, ks=0.0, strain_damping_s=0.04, grasp_params=GraspParams(**GRASP), dll_path=debug_lib) as t:
+            t.dll.LCS_SetLaunchMode(0)
             t.set_gravity(0.0, -981.0, 0.0)
             for k in range(3):
                 press(t, k)
