@@ -467,7 +467,8 @@ LCS_API int GBT_BatchInit(int count, const GbtInstanceDesc* inst, const GbtBatch
         std::vector<float> zeros(3 * (size_t)n, 0.f);
         MeshInput in{d.dimsX, d.dimsY, d.dimsZ, d.cornerPos, d.mass, d.pinned, d.active, zeros.data(), d.nbrIdx, d.restNbr,
                      d.bendPairs, d.bendPairCount, G.youngE, G.poisson};
-        built[i] = buildHostMesh(in, meshes[i]);
+        Team alone(1);
+        built[i] = buildHostMesh(in, meshes[i], alone);
     });
     for (int i = 0; i < count; i++) {
         if (built[i]) return built[i];

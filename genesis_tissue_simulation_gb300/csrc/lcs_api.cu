@@ -669,9 +669,8 @@ LCS_API int LCS_InitPhysics(const PhysicsInitDesc* desc, const float* mass, cons
     MeshInput in{S.dx, S.dy, S.dz, S.hostRest.data(), mass, pinned, active, extForce, nbrIdx, restNbr, bendPairs, bpc,
                  S.youngE, S.poisson};
     HostMesh hm;
-    const bool mayServe = !(S.betaS > 0.f) && !(S.kb > 0.f && bpc > 0);
-    const BriefTeam brief(S.team, mayServe ? planThreads(cc, active, S.forcedBricks) : 1);   // its threads start while the mesh is built
-    int rc = buildHostMesh(in, hm);
+    const BriefTeam brief(S.team, planThreads(cc, active, S.forcedBricks));
+    int rc = buildHostMesh(in, hm, brief.team);
     if (rc) return rc;
     const int E = hm.E, B = hm.B, T = hm.T;
     S.edgeColorOff = hm.edgeColorOff; S.bendColorOff = hm.bendColorOff; S.tetColorOff = hm.tetColorOff;

@@ -31,7 +31,9 @@ struct HostMesh {
     float typeB[6][9];                     // rest Dm^-1 per Kuhn type
 };
 
-// Returns 0, or XPBD_ERR_BAD_ARG / XPBD_ERR_COLOR_OVERFLOW / XPBD_ERR_IRREGULAR_REST.
-int buildHostMesh(const MeshInput& in, HostMesh& out);
+// Returns 0, or XPBD_ERR_BAD_ARG / XPBD_ERR_COLOR_OVERFLOW / XPBD_ERR_IRREGULAR_REST.  Edges, bends and the layers
+// of tets are made by `team`.
+class Team;
+int buildHostMesh(const MeshInput& in, HostMesh& out, Team& team);
 
 }  // namespace gbt
