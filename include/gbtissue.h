@@ -214,7 +214,8 @@ LCS_API int GBT_FrameBarriers(unsigned* barriers);
 /* Automatic mode runs frames without bends or perpendicular damping on spatial bricks, one CTA each, that
  * exchange halo values between groups of colours (plain frames, blade frames with ks > 0, contact model 1,
  * the tissue guard with one pass); results are the same bit for bit.  GBT_SetBrickCount: about `count`
- * bricks in the next LCS_InitPhysics's plan, 0 = one per SM (one in all for a few hundred nodes).
+ * bricks in the next LCS_InitPhysics's plan, 0 = one per SM (one in all for a few hundred nodes); of n
+ * sessions side by side, each in its own copy of the library, ask for SMs / n, else their frames take turns.
  * GBT_BrickInfo: bricks (0: no plan fits), exchanges a substep, threads a CTA, nodes of the largest brick.
  * After a plain brick frame GBT_FrameBarriers reports the exchanges it ran. */
 LCS_API int GBT_SetBrickCount(int count);
