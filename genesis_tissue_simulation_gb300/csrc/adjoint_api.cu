@@ -48,7 +48,7 @@ struct Diff {
     // rollouts on bricks (automatic mode, a mesh with a plan): the session's tables with compliances of
     // the rollout's own, and the reverse sweep's plan.  Made for the session plan `planId`; at session
     // generation `checked` no idle node was mobile.
-    BrickBuffers reverse; Dev<float2> brickAlpha; std::optional<Team> team;
+    BrickBuffers reverse; Dev<float2> brickAlpha;
     bool bricks = false, ranOnBricks = false; int ran[2] = {0, 0};   // bricks of the last forward and backward
     unsigned long long planId = 0, checked = ~0ull;
 };
@@ -62,7 +62,6 @@ void releaseAll() {
     for (auto* b : {&D.theta, &D.path, &D.gTheta, &D.gRest, &D.gB, &D.pathPartial}) b->release();
     D.bake.release(); D.alpha.release(); D.slotStorage.release(); D.brickAlpha.release(); D.reverse.release();
     D.bricks = D.ranOnBricks = false; D.ran[0] = D.ran[1] = 0; D.checked = ~0ull;
-    D.team.reset();
     D.ready = false; D.haveForward = false;
 }
 
@@ -109,11 +108,11 @@ int planReverse(const SessionView& v) {
     const BrickTables& t = v.bricks->t;
     const int perNode = (damped(v) ? 2 : 1) * 16;
     const int forced = t.bricks == 1 ? 1 : v.bricks->asked;
-    const BriefTeam brief(D.team, planThreads(v.N, v.brickMesh.active, forced));
+    Team team(planThreads(v.N, v.brickMesh.active, forced));
     CK(makeBricks(D.reverse, [&]() {
         // the same split: the plan depends on the brick count, and the count on the nodes served
-        const BrickPlan plan = buildBrickPlan(v.brickMesh, v.smCount, v.maxBrickBytes / perNode, forced, false, true, brief.team);
-        brief.team.dismiss();
+        const BrickPlan plan = buildBrickPlan(v.brickMesh, v.smCount, v.maxBrickBytes / perNode, forced, false, true, team);
+        team.dismiss();
         if (!plan.ok() || plan.bricks != t.bricks || plan.maxOwned != t.maxOwned) return cudaSuccess;
         cudaError_t e = D.brickAlpha.ensure(v.bricks->tets);
         if (e == cudaSuccess) e = D.reverse.upload(plan, v.N, damped(v), v.maxBrickBytes, v.stream);

@@ -123,7 +123,6 @@ struct Session {
     BrickBuffers bricks; std::vector<int> brickIdle; unsigned long long planId = 0;
     std::vector<int2> hostEdgeEnds; std::vector<float> hostEdgeRest; std::vector<int4> hostTetIds; std::vector<int> hostTetMeta, hostActive;
     bool bricksDamped = false; int forcedBricks = 0, maxBrickBytes = 0, maxGuardBytes = 0;
-    std::optional<Team> team;   // of the last plan (dismissed)
     int frameBricks = 0;        // bricks the last frame ran on (0: another shape)
     BrickBuffers guardBricks;   // with the tensile pass's phases (one pass), made when the guard is armed
     // section profiler (xpbd_profile_sections, xpbd_solver.cu:30-60): device time per phase kind
@@ -152,7 +151,6 @@ void freeCut() {
     S.cutReady = false; S.toolSet = false; S.havePrev = false;
 }
 void freePhysics() {
-    S.team.reset();
     freeCut();
     releaseCutTopology();
     for (auto* b : {&S.prev, &S.vel, &S.ext}) b->release();
@@ -669,8 +667,8 @@ LCS_API int LCS_InitPhysics(const PhysicsInitDesc* desc, const float* mass, cons
     MeshInput in{S.dx, S.dy, S.dz, S.hostRest.data(), mass, pinned, active, extForce, nbrIdx, restNbr, bendPairs, bpc,
                  S.youngE, S.poisson};
     HostMesh hm;
-    const BriefTeam brief(S.team, planThreads(cc, active, S.forcedBricks));
-    int rc = buildHostMesh(in, hm, brief.team);
+    Team team(planThreads(cc, active, S.forcedBricks));
+    int rc = buildHostMesh(in, hm, team);
     if (rc) return rc;
     const int E = hm.E, B = hm.B, T = hm.T;
     S.edgeColorOff = hm.edgeColorOff; S.bendColorOff = hm.bendColorOff; S.tetColorOff = hm.tetColorOff;
@@ -742,7 +740,7 @@ LCS_API int LCS_InitPhysics(const PhysicsInitDesc* desc, const float* mass, cons
     CK(cudaMemsetAsync(S.bounds.p, 0, kBoundsWords * sizeof(unsigned), S.stream));
 #endif
     CK(cudaStreamSynchronize(S.stream));
-    rc = planBricks(hm, active, brief.team);
+    rc = planBricks(hm, active, team);
     if (rc) return rc;
     S.generation = ++g_sessionGeneration;
     S.physReady = true;
@@ -821,7 +819,7 @@ LCS_API int LCS_SetTissueGuard(float minimum, int passes, int count, const int* 
     if (!S.physReady || S.lastH > 0 || !std::isfinite(minimum) || minimum < 0 || minimum > .95f || passes < 0 || passes > 4 ||
         count != S.N || !inside) return XPBD_ERR_BAD_ARG;
     const bool plans = passes == 1 && S.T > 0 && bricksServe();   // more passes carry multipliers from one to the next
-    const BriefTeam brief(S.team, plans ? planThreads(S.N, S.hostActive.data(), S.forcedBricks) : 1);
+    Team team(plans ? planThreads(S.N, S.hostActive.data(), S.forcedBricks) : 1);
     // incident colour slots of every node (the feasibility line search reads each vertex's tets)
     std::vector<int> off(S.N + 1, 0), inc((size_t)4 * S.T);
     for (int k = 0; k < S.T; k++)
@@ -846,7 +844,7 @@ LCS_API int LCS_SetTissueGuard(float minimum, int passes, int count, const int* 
     if (!plans) return 0;
     BrickMesh bm = brickMesh();
     bm.tensilePasses = 1;
-    return planInto(S.guardBricks, bm, true, S.maxGuardBytes, nullptr, brief.team);
+    return planInto(S.guardBricks, bm, true, S.maxGuardBytes, nullptr, team);
 }
 LCS_API int LCS_SetTissueMaterial(float strength, float bulkDamping) {
     if (!S.physReady || S.lastH > 0 || !std::isfinite(strength) || strength < 0 || strength > 1000 || !std::isfinite(bulkDamping) ||
