@@ -38,17 +38,19 @@ struct Phases {
     int nT;                // tet colours of all passes
     int count;
     std::unique_ptr<int[]> at;   // [edge colours, then tet colours][N] the colour's element at the node, or -1
+    std::unique_ptr<std::atomic<unsigned char>[]> ends;   // [N] whether any element ends at the node
     Phases(const BrickMesh& mesh, bool rev, Team& team)
         : m(mesh), reverse(rev), nT(mesh.nTetColors * (1 + mesh.tensilePasses)), count(mesh.nEdgeColors + nT),
-          at(new int[(size_t)(mesh.nEdgeColors + mesh.nTetColors) * mesh.N]) {
+          at(new int[(size_t)(mesh.nEdgeColors + mesh.nTetColors) * mesh.N]), ends(new std::atomic<unsigned char>[mesh.N]()) {
         team.run(m.nEdgeColors + m.nTetColors, [&](int row, int) {
             int* a = at.get() + (size_t)row * m.N;
             std::fill(a, a + m.N, -1);
+            auto put = [&](int n, int k) { a[n] = k; ends[n].store(1, std::memory_order_relaxed); };
             if (row < m.nEdgeColors) {
-                for (int k = m.edgeOff[row]; k < m.edgeOff[row + 1]; k++) a[m.edgeEnds[k].x] = a[m.edgeEnds[k].y] = k;
+                for (int k = m.edgeOff[row]; k < m.edgeOff[row + 1]; k++) { put(m.edgeEnds[k].x, k); put(m.edgeEnds[k].y, k); }
             } else {
                 const int c = row - m.nEdgeColors;
-                for (int k = m.tetOff[c]; k < m.tetOff[c + 1]; k++) { const int4 t = m.tetIds[k]; a[t.x] = a[t.y] = a[t.z] = a[t.w] = k; }
+                for (int k = m.tetOff[c]; k < m.tetOff[c + 1]; k++) { const int4 t = m.tetIds[k]; put(t.x, k); put(t.y, k); put(t.z, k); put(t.w, k); }
             }
         });
     }
@@ -212,11 +214,7 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
     std::vector<Box> part(chunks);
     team.run(chunks, [&](int q, int) {
         const int i0 = q * chunk, i1 = std::min(m.N, i0 + chunk);
-        for (int i = i0; i < i1; i++) used[i] = m.active[i] != 0;
-        for (int row = 0; row < m.nEdgeColors + m.nTetColors; row++) {
-            const int* a = ph.at.get() + (size_t)row * m.N;
-            for (int i = i0; i < i1; i++) used[i] |= (unsigned char)(a[i] >= 0);
-        }
+        for (int i = i0; i < i1; i++) used[i] = m.active[i] != 0 || ph.ends[i].load(std::memory_order_relaxed) != 0;
         Box b{{m.nx, m.ny, m.nz}, {-1, -1, -1}, 0};
         int c[3] = {i0 % m.nx, i0 / m.nx % m.ny, i0 / (m.nx * m.ny)};
         for (int i = i0; i < i1; i++) {
@@ -295,13 +293,14 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
     // which bricks take values from which (rows: the reader)
     std::vector<unsigned char> reads((size_t)B * B, 0);
     std::atomic<bool> fits{true};
+    std::atomic<size_t> likely[2] = {{0}, {0}};   // sizes of a brick's lists, as far as seen
     auto walk = [&](int b, int worker) {
         if (!fits.load(std::memory_order_relaxed)) return;
         Scratch& s = mine(worker);
         Build& q = build[b];
         q.owned = ownedNodes.data() + ownedAt[b]; q.nOwned = ownedAt[b + 1] - ownedAt[b];
         q.phaseAt.assign(P, 0); q.phaseCount.assign(P, 0); q.importAt.assign(1, 0);
-        if (b != mid) { q.elements.reserve(build[mid].elements.size()); q.imports.reserve(build[mid].imports.size()); }
+        q.elements.reserve(likely[0].load(std::memory_order_relaxed)); q.imports.reserve(likely[1].load(std::memory_order_relaxed));
         int local = q.nOwned;
         for (int st = 0; st < S; st++) {
             startWalk(s, q.owned, q.nOwned);
@@ -318,11 +317,16 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
             q.importAt.push_back((int)q.imports.size());
         }
         s.halo.drain([](int) {});
+        likely[0].store(std::max(likely[0].load(std::memory_order_relaxed), q.elements.size()), std::memory_order_relaxed);
+        likely[1].store(std::max(likely[1].load(std::memory_order_relaxed), q.imports.size()), std::memory_order_relaxed);
         if (local > maxLocal) fits.store(false, std::memory_order_relaxed);
     };
-    walk(mid, 0);   // a mesh that does not fit is told by it
-    if (!fits) return none;
-    team.run(B, [&](int b, int worker) { if (b != mid) walk(b, worker); });
+    const bool asked = served > maxLocal;   // a mesh that does not fit is told by its middle brick
+    if (asked) {
+        walk(mid, 0);
+        if (!fits) return none;
+    }
+    team.run(B, [&](int b, int worker) { if (!asked || b != mid) walk(b, worker); });
     if (!fits) return none;
     // Neighbours take values from each other in every stage: a brick may overwrite a published value
     // two exchanges later, which is safe only once its readers have published their next ones.
@@ -428,6 +432,10 @@ BrickPlan buildBrickPlan(const BrickMesh& m, int maxBricks, int maxLocal, int fo
         }
         for (int i = 0; i < q.importAt[S]; i++) plan.importList[impOff[0] + i] = make_int2(local[q.imports[i]], q.imports[i]);
         for (int i = 0; i < q.exportAt[S]; i++) plan.exportList[expOff[0] + i] = make_int2(local[q.exports[i]], q.exports[i]);
+        std::vector<int> own;
+        own.swap(q.ownTet);
+        q = Build();   // given back by the threads that filled them
+        q.ownTet.swap(own);
     });
     for (int b = 0; b < B && m.tensilePasses > 0; b++) {
         plan.desc[b].ownFirst = (int)plan.ownTet.size();
